@@ -161,6 +161,8 @@ static Consts make_consts(const ns_params* p) {
     c.gamma = p->gamma;
     c.gm1 = p->gamma - 1.0;
     c.inv_gm1 = 1.0 / (p->gamma - 1.0);
+    c.sqrt_gamma = std::sqrt(p->gamma);
+    c.inv_sqrt_gamma = 1.0 / std::sqrt(p->gamma);
     c.mu = p->mu;
     c.lamb = (-2. / 3.) * p->mu;
     c.heat = p->gamma / (p->Pr * (p->gamma - 1.0));

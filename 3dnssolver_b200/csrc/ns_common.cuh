@@ -65,6 +65,7 @@ inline FaceBox make_facebox(int nx, int ny, int nz, int dir) {
 // Kernel-side constants derived from ns_params.
 struct Consts {
     double gamma, gm1, inv_gm1;
+    double sqrt_gamma, inv_sqrt_gamma;
     double mu, lamb, heat;      // lamb = -2/3 mu, heat = gamma/(Pr(gamma-1))
     double dx, dy, dz, inv_dx, inv_dy, inv_dz;
     double cfl;
@@ -132,21 +133,13 @@ NS_HOST_DEVICE int fold_x(int i, int nx, const Consts& c) {
 // ---------------------------------------------------------------------------
 // WENO-5 (Jiang-Shu smoothness indicators, src/convection_schemes/weno-5.cpp:222-322)
 //
-// The three nonlinear weights are formed without a division each: with
-// s_k = eps + beta_k (Shu) the weights d_k/s_k^2 normalised by their sum equal
-// d_k * prod_{j!=k} s_j^2 / sum_m d_m prod_{j!=m} s_j^2 (Borges: d_k (B_k+tau) prod_{j!=k} B_j),
-// and the left and right reconstructions of one face share one division.
-// The algebra is exact; results differ from the reference's form by rounding only.  Single precision keeps per-weight reciprocals
-// (products of squares would leave the float range) and raises eps above the
-// float rounding floor of beta: eps32 = max(eps, (8 u32 s)^2), s the largest
-// |f| of the stencil.
+// in single precision (the FP64 form is in ns_face64.cuh).  Each weight takes a
+// reciprocal of its own (products of squares would leave the float range), and
+// eps is raised above the float rounding floor of beta: eps32 = max(eps, (8 u32 s)^2),
+// s the largest |f| of the stencil.
 
 template <typename T>
 struct WenoC;
-template <>
-struct WenoC<double> {
-    static constexpr double eps_shu = 1e-6, eps_borges = 1e-14;
-};
 template <>
 struct WenoC<float> {
     static constexpr float eps_shu = 1e-6f, eps_borges = 1e-14f;
@@ -166,43 +159,26 @@ __device__ __forceinline__ void weno_betas(T a, T b, T c, T d, T e, T& b0, T& b1
 }
 
 // Weights of one reconstruction from the stencil (a..e) and linear weights
-// (d0,d1,d2): n_k proportional to the nonlinear weights, with the common
-// factor left in (exact algebra, see above).
+// (d0,d1,d2): n_k proportional to the nonlinear weights.
 template <typename T, bool BORGES>
 __device__ __forceinline__ void weno_weights(T a, T b, T c, T d, T e, T d0, T d1, T d2, T& n0, T& n1,
                                              T& n2) {
     T b0, b1, b2;
     weno_betas(a, b, c, d, e, b0, b1, b2);
-    if constexpr (sizeof(T) == 8) {
-        if constexpr (BORGES) {
-            T tau = fabs(b0 - b2);
-            T B0 = b0 + WenoC<T>::eps_borges, B1 = b1 + WenoC<T>::eps_borges,
-              B2 = b2 + WenoC<T>::eps_borges;
-            n0 = d0 * (B0 + tau) * (B1 * B2);
-            n1 = d1 * (B1 + tau) * (B0 * B2);
-            n2 = d2 * (B2 + tau) * (B0 * B1);
-        } else {
-            T s0 = WenoC<T>::eps_shu + b0, s1 = WenoC<T>::eps_shu + b1, s2 = WenoC<T>::eps_shu + b2;
-            T A0 = s0 * s0, A1 = s1 * s1, A2 = s2 * s2;
-            n0 = d0 * (A1 * A2);
-            n1 = d1 * (A0 * A2);
-            n2 = d2 * (A0 * A1);
-        }
+    static_assert(sizeof(T) == 4, "single precision");
+    if constexpr (BORGES) {
+        T tau = fabsf(b0 - b2);
+        n0 = d0 * (T(1) + __fdividef(tau, b0 + WenoC<T>::eps_borges));
+        n1 = d1 * (T(1) + __fdividef(tau, b1 + WenoC<T>::eps_borges));
+        n2 = d2 * (T(1) + __fdividef(tau, b2 + WenoC<T>::eps_borges));
     } else {
-        if constexpr (BORGES) {
-            T tau = fabsf(b0 - b2);
-            n0 = d0 * (T(1) + __fdividef(tau, b0 + WenoC<T>::eps_borges));
-            n1 = d1 * (T(1) + __fdividef(tau, b1 + WenoC<T>::eps_borges));
-            n2 = d2 * (T(1) + __fdividef(tau, b2 + WenoC<T>::eps_borges));
-        } else {
-            T s = fmaxf(fmaxf(fmaxf(fabsf(a), fabsf(b)), fmaxf(fabsf(c), fabsf(d))), fabsf(e));
-            T fl = T(8) * T(5.9604645e-8) * s;
-            T eps = fmaxf(WenoC<T>::eps_shu, fl * fl);
-            T s0 = eps + b0, s1 = eps + b1, s2 = eps + b2;
-            n0 = __fdividef(d0, s0 * s0);
-            n1 = __fdividef(d1, s1 * s1);
-            n2 = __fdividef(d2, s2 * s2);
-        }
+        T s = fmaxf(fmaxf(fmaxf(fabsf(a), fabsf(b)), fmaxf(fabsf(c), fabsf(d))), fabsf(e));
+        T fl = T(8) * T(5.9604645e-8) * s;
+        T eps = fmaxf(WenoC<T>::eps_shu, fl * fl);
+        T s0 = eps + b0, s1 = eps + b1, s2 = eps + b2;
+        n0 = __fdividef(d0, s0 * s0);
+        n1 = __fdividef(d1, s1 * s1);
+        n2 = __fdividef(d2, s2 * s2);
     }
 }
 
@@ -239,9 +215,6 @@ __device__ __forceinline__ void weno_right_nd(T a, T b, T c, T d, T e, T& num, T
 // (PTX rcp.approx.ftz.f64), then the quotient with one Markstein correction
 // (P. Markstein, IA-64 and Elementary Functions, 2000): q = x y, r = x - d q,
 // q + r y.  Within an ulp of the rounded quotient.
-#ifndef NS_WENO_NR
-#define NS_WENO_NR 1
-#endif
 __device__ __forceinline__ double div_pos_nr(double x, double d) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
@@ -257,9 +230,6 @@ __device__ __forceinline__ double div_pos_nr(double x, double d) {
 // 1 / sqrt(x) for a positive, normal x: two Newton-Raphson iterations
 // y <- y + (y / 2)(1 - x y^2) from the hardware estimate (PTX
 // rsqrt.approx.ftz.f64).  Within an ulp or two of the rounded value.
-#ifndef NS_RSQRT_NR
-#define NS_RSQRT_NR 1
-#endif
 __device__ __forceinline__ double rsqrt_pos_nr(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -269,19 +239,13 @@ __device__ __forceinline__ double rsqrt_pos_nr(double x) {
     return fma(0.5 * y, e, y);
 }
 
-// f = WENO5_left(l) + WENO5_right(r) with one division in FP64:
-// nL/dL + nR/dR = (nL dR + nR dL)/(dL dR); FP32 uses two fast reciprocals.
+// f = WENO5_left(l) + WENO5_right(r), two fast reciprocals
 template <typename T, bool BORGES>
 __device__ __forceinline__ T weno_pair(T l0, T l1, T l2, T l3, T l4, T r0, T r1, T r2, T r3, T r4) {
     T nL, dL, nR, dR;
     weno_left_nd<T, BORGES>(l0, l1, l2, l3, l4, nL, dL);
     weno_right_nd<T, BORGES>(r0, r1, r2, r3, r4, nR, dR);
-    if constexpr (sizeof(T) == 8) {
-        if constexpr (NS_WENO_NR) return div_pos_nr(nL * dR + nR * dL, dL * dR);
-        else return (nL * dR + nR * dL) / (dL * dR);
-    }
-    else
-        return __fdividef(nL, dL) + __fdividef(nR, dR);
+    return __fdividef(nL, dL) + __fdividef(nR, dR);
 }
 
 }  // namespace nsb

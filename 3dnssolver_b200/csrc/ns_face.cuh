@@ -1,4 +1,5 @@
-// ns_face.cuh -- WENO-5 face flux of one face (device functions).
+// ns_face.cuh -- WENO-5 face flux of one face in single precision (device
+// functions); the FP64 faces are in ns_face64.cuh.
 //
 // A face along axis DIR lies between cells a and a+1; its 6-cell stencil is
 // a-2..a+3.  face_stencil loads the stencil, forms half the Euler flux of each
@@ -39,15 +40,6 @@ __device__ __forceinline__ constexpr int st(int t) {
     return PHYS ? (t == 0 ? 0 : (t == 4 ? 1 : t + 1)) : t;
 }
 
-template <typename T>
-__device__ __forceinline__ T tsqrt(T x) {
-    if constexpr (sizeof(T) == 8) return sqrt(x); else return sqrtf(x);
-}
-template <typename T>
-__device__ __forceinline__ T trcp(T x) {
-    if constexpr (sizeof(T) == 8) return 1.0 / x; else return __fdividef(1.0f, x);
-}
-
 // Left/right eigenvectors of the 3D Euler Jacobian (ConvectionFlux::eigenvectors,
 // convection_flux.cpp:117-175) at the arithmetic face average, kept as the
 // scalars the sparse rows need.
@@ -55,17 +47,6 @@ template <typename T>
 struct Eig {
     T vel[3], qn, ql, qm, q2, c, c2, H, Kpc, K2pc, inv2c;
 };
-
-// 1/sqrt(x), x > 0 (sound speeds): Newton-Raphson in FP64 (rsqrt_pos_nr)
-template <typename T>
-__device__ __forceinline__ T trsqrt(T x) {
-    if constexpr (sizeof(T) == 8) {
-        if constexpr (NS_RSQRT_NR) return rsqrt_pos_nr(x);
-        else return rsqrt(x);
-    } else {
-        return rsqrtf(x);
-    }
-}
 
 // Reference semantics (c2 = gamma/(p rho), convection_flux.cpp:139): one
 // r = rsqrt(p rho) and one rg = rsqrt(gamma) give c = sqrt(gamma) r,
@@ -83,10 +64,9 @@ __device__ __forceinline__ Eig<T> make_eig(const T wa[5], T gamma, T inv_gm1) {
     T K = gamma - T(1);
     if constexpr (PHYS) {
         // c2 = gamma p / rho from one r = rsqrt(gamma p rho): c = gamma p r,
-        // 1/c = rho r, so no division or square root (each costs a Newton
-        // sequence in FP64)
+        // 1/c = rho r, so no division or square root
         const T gp = gamma * p;
-        const T r = trsqrt(gp * rho);
+        const T r = rsqrtf(gp * rho);
         const T ic = rho * r;
         e.c = gp * r;
         e.c2 = e.c * e.c;
@@ -94,10 +74,10 @@ __device__ __forceinline__ Eig<T> make_eig(const T wa[5], T gamma, T inv_gm1) {
         e.inv2c = T(0.5) * ic;
     } else {
         T pr = p * rho;
-        T r = trsqrt(pr);
+        T r = rsqrtf(pr);
         // sqrt(gamma) and 1/gamma from one rg = rsqrt(gamma): no square root or
         // division per face
-        const T rg = trsqrt(gamma);
+        const T rg = rsqrtf(gamma);
         e.c = (gamma * rg) * r;
         e.c2 = gamma * (r * r);
         e.Kpc = (K * T(0.5) * (rg * rg)) * pr;
@@ -208,7 +188,7 @@ __device__ __forceinline__ void face_stencil_from(Loader ld, const Consts& c, T 
             T w[5], u[5];
             ld(s, w, u);
             const T gp = gamma * w[1];
-            const T a = fabs(w[2 + DIR]) + gp * trsqrt(gp * w[0]);
+            const T a = fabsf(w[2 + DIR]) + gp * rsqrtf(gp * w[0]);
             amax = (s == 0) ? a : (a > amax ? a : amax);
         }
         const T halpha = half * amax;

@@ -21,6 +21,7 @@
 #include "ns_common.cuh"
 #include "ns_eos.cuh"
 #include "ns_face.cuh"
+#include "ns_face64.cuh"
 #include "ns_kernels.h"
 #include "ns_tcgen05.cuh"
 #include "ns_tma.cuh"
@@ -249,23 +250,23 @@ __device__ __forceinline__ void face_at(const double* __restrict__ W, const doub
                                         const FaceBox& fb, int aa, int bb, int kk) {
     long long step;
     long long o0 = face_origin<DIR>(b, aa, bb, kk, step);
-    T fL[5][5], fR[5][5], wa[5];
-    if constexpr (WONLY) {
-        auto ld = [&](int s, T w[5], T u[5]) {
-            const long long os = o0 + s * step;
-#pragma unroll
-            for (int q = 0; q < 5; q++) w[q] = W[q * b.fstride + os];
-            cons_from_prim(w, c.inv_gm1, u);
-        };
-        face_stencil_from<DIR, CHAR, PHYS, T>(ld, c, fL, fR, wa);
-    } else {
-        face_stencil<DIR, CHAR, PHYS, T>(W, U, b, c, o0, step, fL, fR, wa);
-    }
     T out[5];
-    if constexpr (!CHAR)
-        face_comp<T, BORGES>(fL, fR, out);
-    else
-        face_char<DIR, PHYS, T, BORGES>(fL, fR, wa, T(c.gamma), T(c.inv_gm1), out);
+    if constexpr (WONLY) {
+        auto ld = [&](int s, T w[5]) {
+#pragma unroll
+            for (int q = 0; q < 5; q++) w[q] = W[q * b.fstride + o0 + s * step];
+        };
+        face_flux64_w<DIR, CHAR, BORGES, PHYS>(ld, c, out);
+    } else if constexpr (sizeof(T) == 8) {
+        face_flux64_wu<DIR, CHAR, BORGES, PHYS>(W, U, b, c, o0, step, out);
+    } else {
+        T fL[5][5], fR[5][5], wa[5];
+        face_stencil<DIR, CHAR, PHYS, T>(W, U, b, c, o0, step, fL, fR, wa);
+        if constexpr (!CHAR)
+            face_comp<T, BORGES>(fL, fR, out);
+        else
+            face_char<DIR, PHYS, T, BORGES>(fL, fR, wa, T(c.gamma), T(c.inv_gm1), out);
+    }
     long long fo = fb.at(aa, bb, kk);
 #pragma unroll
     for (int q = 0; q < 5; q++) F[q * fb.fstride + fo] = TF(out[q]);
@@ -911,18 +912,11 @@ __global__ void __launch_bounds__(128, XupdMinBlocks<CHAR, PHYS>::value)
     auto xface = [&](int a, double out[5]) {
         long long step;
         const long long o0 = face_origin<0>(b, a, j, k, step);
-        auto ld = [&](int s, double w[5], double u[5]) {
-            const long long os = o0 + s * step;
+        auto ld = [&](int s, double w[5]) {
 #pragma unroll
-            for (int q = 0; q < 5; q++) w[q] = W[q * b.fstride + os];
-            cons_from_prim(w, c.inv_gm1, u);
+            for (int q = 0; q < 5; q++) w[q] = W[q * b.fstride + o0 + s * step];
         };
-        double fL[5][5], fR[5][5], wa[5];
-        face_stencil_from<0, CHAR, PHYS, double>(ld, c, fL, fR, wa);
-        if constexpr (!CHAR)
-            face_comp<double, BORGES>(fL, fR, out);
-        else
-            face_char<0, PHYS, double, BORGES>(fL, fR, wa, c.gamma, c.inv_gm1, out);
+        face_flux64_w<0, CHAR, BORGES, PHYS>(ld, c, out);
     };
     const bool convz = flags & UPD_CONVZ;
     // one face call site: the pass i = x0 - 1 only forms the first x-face

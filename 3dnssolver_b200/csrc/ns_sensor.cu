@@ -37,6 +37,7 @@
 #include "ns_common.cuh"
 #include "ns_eos.cuh"
 #include "ns_face.cuh"
+#include "ns_face64.cuh"
 #include "ns_sensor.h"
 #include "ns_tcgen05.cuh"
 
@@ -300,10 +301,9 @@ __global__ void __launch_bounds__(128) k_sensor_harvest(const double* __restrict
     if (kk >= fb.n2 || bb >= fb.n1) return;
     long long step;
     long long o0 = face_origin<DIR>(b, aa, bb, kk, step);
-    double fL[5][5], fR[5][5], wa[5], fc[5], fx[5];
-    face_stencil<DIR, true, PHYS, double>(W, U, b, c, o0, step, fL, fR, wa);
-    face_comp<double, BORGES>(fL, fR, fc);
-    face_char<DIR, PHYS, double, BORGES>(fL, fR, wa, c.gamma, c.inv_gm1, fx);
+    double fc[5], fx[5];
+    face_flux64_wu<DIR, false, BORGES, PHYS>(W, U, b, c, o0, step, fc);
+    face_flux64_wu<DIR, true, BORGES, PHYS>(W, U, b, c, o0, step, fx);
     double dn = 0, nn = 0;
 #pragma unroll
     for (int q = 0; q < 5; q++) {

@@ -11,7 +11,7 @@
 // tile, the TMA engine fetches the block's next tile, so the stencil loads
 // leave the warps' critical path (the per-thread kernel k_face_flux waits on
 // its 30 global loads per face).  The face arithmetic is the same code
-// (face_stencil_from + face_comp/face_char), so the fluxes are bit-identical.
+// (face_flux64_w), so the fluxes are the same.
 // (A pass that formed U, the half flux and the wave speed once per cell of the
 // tile in shared memory, instead of once per face through the cell, ran 2-6%
 // slower on B200 at 256^3: the extra barrier and shared-memory traffic cost
@@ -39,7 +39,7 @@
 
 #include "ns_common.cuh"
 #include "ns_eos.cuh"
-#include "ns_face.cuh"
+#include "ns_face64.cuh"
 #include "ns_kernels.h"
 #include "ns_tcgen05.cuh"
 #include "ns_tma.cuh"
@@ -118,17 +118,12 @@ __global__ void __launch_bounds__(128, TmaFaceMinBlocks<CHAR>::value)
             const int kk = tz * 32 + lane, bb = tyi * 4 + ty;
             if (kk < b.nz && bb < b.ny) {
                 const double* sm = buf + s * TD::STRIDE + ty * FT::BZ + FT::Z0 + lane;
-                auto ld = [&](int st, double w[5], double u[5]) {
+                auto ld = [&](int st, double w[5]) {
 #pragma unroll
                     for (int q = 0; q < 5; q++) w[q] = sm[q * TD::QS + st * FT::SS];
-                    cons_from_prim(w, c.inv_gm1, u);
                 };
-                double fL[5][5], fR[5][5], wa[5], out[5];
-                face_stencil_from<DIR, CHAR, PHYS, double>(ld, c, fL, fR, wa);
-                if constexpr (!CHAR)
-                    face_comp<double, BORGES>(fL, fR, out);
-                else
-                    face_char<DIR, PHYS, double, BORGES>(fL, fR, wa, c.gamma, c.inv_gm1, out);
+                double out[5];
+                face_flux64_w<DIR, CHAR, BORGES, PHYS>(ld, c, out);
                 const long long fo = fb.at(aa, bb, kk);
 #pragma unroll
                 for (int q = 0; q < 5; q++) F[q * fb.fstride + fo] = out[q];
@@ -239,18 +234,12 @@ __global__ void __launch_bounds__(128, CHAR ? NS_XT_MINB_CHAR : 3)
     const int cc = ty * XL::BZ + lane + 1;
     // x-face a (between cells a-1 and a) of this thread's column: cells a-3 .. a+2
     auto xface = [&](int a, double out[5]) {
-        auto ld = [&](int st, double w[5], double u[5]) {
+        auto ld = [&](int st, double w[5]) {
             const double* P = ring + sl(a - 3 + st) * XL::STRIDE + cc;
 #pragma unroll
             for (int q = 0; q < 5; q++) w[q] = P[q * XL::QS];
-            cons_from_prim(w, c.inv_gm1, u);
         };
-        double fL[5][5], fR[5][5], wa[5];
-        face_stencil_from<0, CHAR, PHYS, double>(ld, c, fL, fR, wa);
-        if constexpr (!CHAR)
-            face_comp<double, BORGES>(fL, fR, out);
-        else
-            face_char<0, PHYS, double, BORGES>(fL, fR, wa, c.gamma, c.inv_gm1, out);
+        face_flux64_w<0, CHAR, BORGES, PHYS>(ld, c, out);
     };
     const bool convz = flags & UPD_CONVZ;
     for (int i = x0 - 1; i < x1; i++) {

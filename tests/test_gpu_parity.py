@@ -310,3 +310,35 @@ def test_weno_quotient_within_one_ulp_of_ieee_division():
     q, r = pkg.div_selftest(1 << 22, seed=7)
     assert q <= 1, q
     assert r <= 2, r  # the sound-speed 1/sqrt against CUDA's rsqrt (each within an ulp)
+
+
+# The FP64 faces work on differences, with the acoustic fields taken 2c times as
+# large and the WENO epsilon scaled along: states whose magnitudes are far from 1
+# (air in SI units; amplitudes where the indicators fall below the epsilon) on odd
+# grids.  Tolerance: the rounding of a flux, about 50 operations of 1.1e-16, over the
+# fraction (here above 1e-2) that a flux difference is of the flux: below 1e-12.
+SCALE_CASES = [
+    ((7, 9, 11), 1, 0, 0, 1.0e5, 300.0),
+    ((33, 5, 35), 1, 1, 1, 1.0e5, 300.0),
+    ((6, 33, 7), 2, 0, 1, 1.0e5, 300.0),
+    ((9, 6, 33), 2, 1, 1, 1.0e5, 300.0),
+    ((8, 7, 34), 1, 1, 0, 1.0e-4, 1.0e-2),
+    ((34, 8, 5), 2, 0, 1, 1.0e-4, 1.0e-2),
+]
+
+
+@pytest.mark.parametrize("shape,conv,weights,sem,pscale,vscale", SCALE_CASES)
+def test_face_flux_scales_match_oracle(oracle, shape, conv, weights, sem, pscale, vscale):
+    p = pkg.make_params(*shape, convection=conv, weights=weights, semantics=sem, bc=(N, P, N), mu=0.0,
+                        diffusion=pkg.DIFF_NONE)
+    W = wl.random_field(p, seed=31, smooth=False)
+    W[..., 1] *= pscale
+    W[..., 2:] *= vscale
+    with pkg.Solver(p) as s:
+        R = s.rhs(W)
+        Wg, Ug = W.copy(), s.new_array()
+        s.time_step(Wg, Ug)
+    err = rel_l2(interior(R), interior(oracle.rhs(p, W)))
+    assert (err <= TOL).all(), err
+    _, Uo, _ = oracle.run(p, W, 1)
+    _assert_close(Ug, Uo, what="U after a step")
