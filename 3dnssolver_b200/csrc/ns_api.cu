@@ -271,42 +271,15 @@ static void prof_mark(ns_ctx* ctx, int cls) {
     g_prof->cls[g_prof->n++] = cls;
 }
 
-// TMA-staged FP64 kernels: the y/z faces and the viscous terms of the physical
-// semantics, the x-march of both (build switches, on by default)
-#ifndef NS_FACE_TMA
-#define NS_FACE_TMA 1
-#endif
-#ifndef NS_VISC_TMA_MAX_ORDER
-#define NS_VISC_TMA_MAX_ORDER 6  // CD orders whose viscous terms march over TMA planes
-#endif
-#ifndef NS_VISC_TMA_REF
-#define NS_VISC_TMA_REF 1  // the reference semantics' viscous terms too
-#endif
-#ifndef NS_XUPD_TMA
-#define NS_XUPD_TMA 1
-#endif
-#ifndef NS_FACE_TMA_REF
-#define NS_FACE_TMA_REF 0  // the TMA face tiles for the reference semantics' y/z faces too
-#endif
+// the TMA tensor maps of the context's current W (FP64 steps)
+static const nsb::WTmaMaps& tma_maps(const ns_ctx* ctx) { return ctx->tma[ctx->tma[0].W == ctx->W ? 0 : 1]; }
 
-// the TMA tensor maps of the context's current W (FP64 steps), or null
-static const nsb::WTmaMaps* tma_maps(const ns_ctx* ctx) {
-    if (fp32(ctx)) return nullptr;
-    for (const nsb::WTmaMaps& t : ctx->tma)
-        if (t.ok && t.W == ctx->W) return &t;
-    return nullptr;
-}
-
-// face fluxes of the current (W, U) along every convected axis from first_dir on
-// (U: the context's, or the stage input Uin); pl: the x-planes of the y- and
-// z-faces of an FP64 time step (w_only), all planes by default
-static ns_status faces(ns_ctx* ctx, int first_dir = 0, const double* Uin = nullptr, bool w_only = false,
-                       Planes pl = Planes()) {
+// face fluxes of the current (W, U) along every convected axis (operator calls)
+static ns_status faces(ns_ctx* ctx) {
     const ns_params& p = ctx->p;
-    const double* U = Uin ? Uin : ctx->U;
     if (p.convection == NS_CONV_NONE) return NS_OK;
     int nd = p.dim == 3 ? 3 : 2;
-    for (int d = first_dir; d < nd; d++) {
+    for (int d = 0; d < nd; d++) {
         if (p.sensor) {
             if (sensor_face_flux(ctx->sensor, d, ctx->W, ctx->U, ctx->box, ctx->c, p.sensor_threshold,
                                  p.weights == NS_WEIGHTS_BORGES, phys(ctx), ctx->F[d], ctx->fb[d], ctx->stream,
@@ -314,22 +287,22 @@ static ns_status faces(ns_ctx* ctx, int first_dir = 0, const double* Uin = nullp
                 return fail(NS_ERR_CUDA, "gated face kernel launch failed: %s",
                             cudaGetErrorString(cudaGetLastError()));
         } else {
-            // the TMA tiles serve the physical semantics, whose face stencils read
-            // every cell twice (local LF speed, then the split): from shared memory
-            // that is 7-8% faster than the per-thread kernels on B200, which are 3-7%
-            // faster for the reference semantics' single pass (256^3)
-            const nsb::WTmaMaps* m =
-                (NS_FACE_TMA && w_only && d > 0 && (phys(ctx) || NS_FACE_TMA_REF)) ? tma_maps(ctx) : nullptr;
-            if (m)
-                launch_face_flux_tma(d, p.convection == NS_CONV_WENO5_CHAR, p.weights == NS_WEIGHTS_BORGES,
-                                     phys(ctx), *m, ctx->W, ctx->box, ctx->c, ctx->F[d], ctx->fb[d], ctx->sms,
-                                     ctx->slot + 4, ctx->stream, pl);
-            else
-                launch_face_flux(d, p.convection == NS_CONV_WENO5_CHAR, p.weights == NS_WEIGHTS_BORGES,
-                                 phys(ctx), fp32(ctx), ctx->W, U, ctx->box, ctx->c, ctx->F[d],
-                                 ctx->fb[d], ctx->stream, w_only, w_only ? pl : Planes());
+            launch_face_flux(d, p.convection == NS_CONV_WENO5_CHAR, p.weights == NS_WEIGHTS_BORGES, phys(ctx),
+                             fp32(ctx), ctx->W, ctx->U, ctx->box, ctx->c, ctx->F[d], ctx->fb[d], ctx->stream);
             NS_TRY(check_launch(ctx, d > 0 ? 2 : 1));  // y and z: the face grid and its last plane
         }
+        prof_mark(ctx, NS_PROF_FACE_X + d);
+    }
+    return NS_OK;
+}
+
+// y- and z-faces of an FP64 stage from the current W (W = prim(U)), on the x-planes pl
+static ns_status step_faces(ns_ctx* ctx, Planes pl) {
+    const ns_params& p = ctx->p;
+    for (int d = 1; d < (p.dim == 3 ? 3 : 2); d++) {
+        launch_step_faces(d, p.convection == NS_CONV_WENO5_CHAR, p.weights == NS_WEIGHTS_BORGES, phys(ctx), ctx->W,
+                          ctx->box, ctx->c, (double*)ctx->F[d], ctx->fb[d], ctx->stream, pl);
+        NS_TRY(check_launch(ctx, 1));
         prof_mark(ctx, NS_PROF_FACE_X + d);
     }
     return NS_OK;
@@ -445,45 +418,41 @@ static const double kRkM2[3] = {0.0, 1.0 / 4.0, 2. / 3.};
 static const double kRkMc[3] = {-1.0, -(1. / 4.), -(2. / 3.)};
 
 // FP64 stage st after its fill, on the x-planes pl: the y- and z-faces (with
-// faces), the viscous terms, then the x-faces marched together with the cell
+// with_faces), the viscous terms, then the x-faces marched together with the cell
 // update from Uin into Uout (and the next stage's W into W2)
 static ns_status xstage(ns_ctx* ctx, int st, double* Uin, double* Uout, unsigned long long* cur,
                         unsigned long long* nxt, bool with_faces, Planes pl) {
     cudaStream_t s = ctx->stream;
-    if (with_faces) NS_TRY(faces(ctx, 1, Uin, true, pl));  // W = prim(U) here: the stencils read W only
-    UpdateArgs a = update_args(ctx, MODE_STAGE, true, true);
-    if (a.viscous) {  // into the x-face array, which the x-march leaves unused
-        a.V = (const double*)ctx->F[0];
-        a.vs = ctx->fb[0].fstride;
-        const nsb::WTmaMaps* m = tma_maps(ctx);
-        if (m && ctx->c.order <= NS_VISC_TMA_MAX_ORDER && (phys(ctx) || NS_VISC_TMA_REF))
-            launch_viscous_tma(ctx->c.order / 2, phys(ctx), *m, ctx->W, ctx->box, ctx->c, (double*)ctx->F[0],
-                               ctx->fb[0].fstride, ctx->slot + 4, s, pl);
-        else if (pl.n < 0)
-            launch_viscous(ctx->c.order / 2, phys(ctx), ctx->W, ctx->box, ctx->c, (double*)ctx->F[0],
-                           ctx->fb[0].fstride, s);
-        else
-            return fail(NS_ERR_UNSUPPORTED, "a plane range of the viscous terms needs their TMA kernel");
+    if (with_faces) NS_TRY(step_faces(ctx, pl));
+    const bool visc = ctx->p.diffusion == NS_DIFF_CENTERED;
+    if (visc) {  // into the x-face array, which a step leaves unused otherwise
+        launch_viscous_tma(ctx->c.order / 2, phys(ctx), tma_maps(ctx), ctx->W, ctx->box, ctx->c, (double*)ctx->F[0],
+                           ctx->fb[0].fstride, ctx->slot + 4, ctx->sms, s, pl);
         NS_TRY(check_launch(ctx, 1));
         prof_mark(ctx, NS_PROF_VISCOUS);
     }
+    XMarchArgs a;
+    a.W = ctx->W;
     a.U = Uin;
-    a.Unext = Uout;
+    a.U0 = ctx->U0;
+    a.Uout = Uout;
     a.Wnext = ctx->W2;
+    a.Fy = (const double*)ctx->F[1];
+    a.Fz = (const double*)ctx->F[2];
+    a.V = visc ? (const double*)ctx->F[0] : nullptr;
+    a.vs = ctx->fb[0].fstride;
+    a.b = ctx->box;
+    a.fy = ctx->fb[1];
+    a.fz = ctx->fb[2];
+    a.c = ctx->c;
     a.slot = cur;
     a.slot_next = (st == 2) ? nxt : nullptr;
     a.m1 = kRkM1[st];
     a.m2 = kRkM2[st];
     a.mc = kRkMc[st];
     a.clock = (st == 0) ? ctx->clock : nullptr;
-    const nsb::WTmaMaps* xm = NS_XUPD_TMA ? tma_maps(ctx) : nullptr;
-    if (xm)
-        launch_xface_update_tma(ctx->p.convection == NS_CONV_WENO5_CHAR, ctx->p.weights == NS_WEIGHTS_BORGES, a, *xm,
-                                ctx->slot + 4, s, pl);
-    else if (pl.n < 0)
-        launch_xface_update(ctx->p.convection == NS_CONV_WENO5_CHAR, ctx->p.weights == NS_WEIGHTS_BORGES, a, s);
-    else
-        return fail(NS_ERR_UNSUPPORTED, "a plane range of the x-march needs its TMA kernel");
+    a.sms = ctx->sms;
+    launch_xmarch(ctx->p.convection == NS_CONV_WENO5_CHAR, ctx->p.weights == NS_WEIGHTS_BORGES, phys(ctx), a, s, pl);
     NS_TRY(check_launch(ctx, 1));
     prof_mark(ctx, NS_PROF_XFACE_UPDATE);
     return NS_OK;
@@ -532,8 +501,8 @@ static ns_status do_step(ns_ctx* ctx) {
         ctx->steps++;
         return NS_OK;
     }
-    // FP64 with convection: per stage the fill, the y- and z-faces, then the
-    // x-faces marched together with the cell update into the other buffer:
+    // FP64 with convection: per stage the fill, the y- and z-faces, the viscous terms,
+    // then the x-faces marched together with the cell update into the other buffer:
     // U0 -> U -> U2 -> U (stage 1 reads the step's start U0 directly).  The
     // fill copies the stage input's halos into the output buffer, so the step
     // ends with the halos the reference's U holds.  The third stage also forms
@@ -557,9 +526,9 @@ static ns_status do_step(ns_ctx* ctx) {
     for (int st = 0; st < 3; st++) {
         NS_TRY(exchange(ctx, NS_EXCHANGE_HALO, in[st], nullptr));
         if (st == 0 && !w_ready)
-            launch_fill_prim(ctx->W, in[st], ctx->box, ctx->c, s, out[st]);
+            launch_fill_prim(ctx->W, in[st], ctx->box, ctx->c, s, out[st], phys(ctx));
         else
-            launch_fill_halo(ctx->W, in[st], ctx->box, ctx->c, s, out[st]);
+            launch_fill_halo(ctx->W, in[st], ctx->box, ctx->c, s, out[st], phys(ctx));
         NS_TRY(check_launch(ctx, 1));
         prof_mark(ctx, NS_PROF_FILL);
         NS_TRY(xstage(ctx, st, in[st], out[st], cur, nxt, true, Planes()));
@@ -714,7 +683,12 @@ ns_status ns_create(const ns_params* p, ns_ctx** out) {
         return fail(NS_ERR_CUDA, "cudaStreamCreate failed");
     }
     ctx->stream = ctx->own;
-    A((void**)&ctx->W, soa_bytes(ctx->box));
+    // FP64 steps of the physical semantics keep the sound speed beside W, as a sixth
+    // plane that every writer of a stage's W fills: the Lax-Friedrichs speeds of the 18
+    // faces that a cell belongs to read it
+    const int wplanes = p->precision == NS_PREC_FP64 && p->convection != NS_CONV_NONE && phys(ctx) ? NS_NQ + 1 : NS_NQ;
+    const size_t wbytes = soa_bytes(ctx->box) / NS_NQ * wplanes;
+    A((void**)&ctx->W, wbytes);
     A((void**)&ctx->U, soa_bytes(ctx->box));
     A((void**)&ctx->U0, soa_bytes(ctx->box));
     size_t fe = fp32(ctx) ? sizeof(float) : sizeof(double);
@@ -730,17 +704,15 @@ ns_status ns_create(const ns_params* p, ns_ctx** out) {
     ctx->fused = p->precision == NS_PREC_FP32;
     ctx->xfused = !ctx->fused && p->precision == NS_PREC_FP64 && p->convection != NS_CONV_NONE;
     if (ctx->fused || ctx->xfused) A((void**)&ctx->U2, soa_bytes(ctx->box));
-    if (ctx->xfused) A((void**)&ctx->W2, soa_bytes(ctx->box));
-    if (st == NS_OK && ctx->xfused) {
-        // the y/z faces of the FP64 steps read W (and W2, which swaps with it) through TMA tiles
-        nsb::w_tma_encode(&ctx->tma[0], ctx->W, ctx->box);
-        nsb::w_tma_encode(&ctx->tma[1], ctx->W2, ctx->box);
-    }
+    if (ctx->xfused) A((void**)&ctx->W2, wbytes);
+    if (st == NS_OK && ctx->xfused && !(nsb::w_tma_encode(&ctx->tma[0], ctx->W, ctx->box, wplanes) &&
+                                        nsb::w_tma_encode(&ctx->tma[1], ctx->W2, ctx->box, wplanes)))
+        st = fail(NS_ERR_CUDA, "the driver makes no tensor map of the primitive field");
     A((void**)&ctx->diag, 8 * sizeof(double));
     A((void**)&ctx->clock, 2 * sizeof(double));
     if (st == NS_OK) {
         // zero the state so halos/corners hold defined values before the first upload
-        cudaMemsetAsync(ctx->W, 0, soa_bytes(ctx->box), ctx->stream);
+        cudaMemsetAsync(ctx->W, 0, wbytes, ctx->stream);
         cudaMemsetAsync(ctx->U, 0, soa_bytes(ctx->box), ctx->stream);
         cudaMemsetAsync(ctx->U0, 0, soa_bytes(ctx->box), ctx->stream);
         cudaMemsetAsync(ctx->clock, 0, 2 * sizeof(double), ctx->stream);
@@ -877,9 +849,8 @@ static ns_status device_status(ns_ctx* ctx);
 #define NS_STEP_PIPELINE 1  // ns_time_step overlaps its host transfers with the stages
 #endif
 
-// x-planes per chunk of ns_time_step's transfer pipeline: whole marches of the
-// TMA viscous kernel and of the TMA x-march
-static int pipe_chunk() { return std::max(xmarch_planes(), viscous_march_planes()); }
+// x-planes per chunk of ns_time_step's transfer pipeline
+static int pipe_chunk() { return 64; }
 
 static bool pinned(const void* p) {
     cudaPointerAttributes a;
@@ -891,16 +862,12 @@ static bool pinned(const void* p) {
 }
 
 // whether ns_time_step runs time_step_pipelined: an FP64 step of do_step's
-// x-march form whose kernels all take plane ranges (TMA maps of both W
-// buffers), on a single domain, at least two chunks long, from and to pinned
+// x-march form, on a single domain, at least two chunks long, from and to pinned
 // host memory (to pageable memory a copy blocks the calling thread and
 // serialises the chunks)
 static bool pipelined(const ns_ctx* ctx, const double* W, const double* U) {
     const ns_params& p = ctx->p;
-    if (!NS_STEP_PIPELINE || !NS_XUPD_TMA || !ctx->xfused || ctx->fused || slab(ctx) || p.sensor) return false;
-    if (!ctx->tma[0].ok || !ctx->tma[1].ok || p.nx < 2 * pipe_chunk()) return false;
-    if (p.diffusion == NS_DIFF_CENTERED && (ctx->c.order > NS_VISC_TMA_MAX_ORDER || !(phys(ctx) || NS_VISC_TMA_REF)))
-        return false;
+    if (!NS_STEP_PIPELINE || !ctx->xfused || slab(ctx) || p.sensor || p.nx < 2 * pipe_chunk()) return false;
     return pinned(W) && (!U || pinned(U));
 }
 
@@ -979,26 +946,26 @@ static ns_status time_step_pipelined_run(ns_ctx* ctx, const double* Wh, double* 
         NS_CUDA(cudaStreamWaitEvent(s, ev[c], 0));
         launch_aos_to_soa(ctx->stage, ctx->W, ctx->box, s, sp);
         launch_step_begin(false, phys(ctx), ctx->W, ctx->U, ctx->U0, ctx->box, ctx->c, cur, s, sp);
-        launch_fill_prim(ctx->W, ctx->U0, ctx->box, ctx->c, s, ctx->U, halo_interior(c));
+        launch_fill_prim(ctx->W, ctx->U0, ctx->box, ctx->c, s, ctx->U, phys(ctx), halo_interior(c));
         NS_TRY(check_launch(ctx, 3));
-        NS_TRY(faces(ctx, 1, ctx->U0, true, interior(c)));
+        NS_TRY(step_faces(ctx, interior(c)));
     }
     // the x ghost planes fold onto planes of other chunks
-    launch_fill_prim(ctx->W, ctx->U0, ctx->box, ctx->c, s, ctx->U, ghost_lo);
-    launch_fill_prim(ctx->W, ctx->U0, ctx->box, ctx->c, s, ctx->U, ghost_hi);
+    launch_fill_prim(ctx->W, ctx->U0, ctx->box, ctx->c, s, ctx->U, phys(ctx), ghost_lo);
+    launch_fill_prim(ctx->W, ctx->U0, ctx->box, ctx->c, s, ctx->U, phys(ctx), ghost_hi);
     NS_TRY(check_launch(ctx, 2));
     NS_TRY(xstage(ctx, 0, ctx->U0, ctx->U, cur, nxt, false, Planes()));
     std::swap(ctx->W, ctx->W2);
 
     // stage 2 (U -> U2)
-    launch_fill_halo(ctx->W, ctx->U, ctx->box, ctx->c, s, ctx->U2);
+    launch_fill_halo(ctx->W, ctx->U, ctx->box, ctx->c, s, ctx->U2, phys(ctx));
     NS_TRY(check_launch(ctx, 1));
     NS_TRY(xstage(ctx, 1, ctx->U, ctx->U2, cur, nxt, true, Planes()));
     std::swap(ctx->W, ctx->W2);
 
     // stage 3 (U2 -> U) chunk by chunk into W2, which then holds prim(U) on every
     // cell (finalize_w); U's ghost cells are final after the fill
-    launch_fill_halo(ctx->W, ctx->U2, ctx->box, ctx->c, s, ctx->U);
+    launch_fill_halo(ctx->W, ctx->U2, ctx->box, ctx->c, s, ctx->U, phys(ctx));
     launch_prim_all(ctx->W2, ctx->U, ctx->box, ctx->c, s, ghost_lo);
     launch_prim_all(ctx->W2, ctx->U, ctx->box, ctx->c, s, ghost_hi);
     NS_TRY(check_launch(ctx, 3));

@@ -37,6 +37,12 @@ __device__ __forceinline__ void cons_from_prim(const double w[5], double inv_gm1
     u[1] = __fma_rn(w[1], inv_gm1, kin);
 }
 
+// sqrt(gamma p / rho) as gamma p / sqrt(gamma p rho), for the Lax-Friedrichs speeds
+__device__ __forceinline__ double sound_speed(const double w[5], double gamma) {
+    const double gp = __dmul_rn(gamma, w[1]);
+    return __dmul_rn(gp, rsqrt_pos_nr(__dmul_rn(gp, w[0])));
+}
+
 // EqOfState::local_dt (src/eq_of_state.cpp:89-101), min over directions
 // max(|u+c|, |u-c|) is |u| + c for c >= 0, exactly and in rounding; the minimum
 // over the axes of d/(|u|+c) is taken as one reciprocal of the largest (|u|+c)/d

