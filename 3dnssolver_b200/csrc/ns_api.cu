@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "ns_common.cuh"
+#include "ns_eos.cuh"
 #include "ns_kernels.h"
 #include "ns_sensor.h"
 
@@ -86,7 +87,7 @@ struct ns_ctx {
     unsigned long long* xslot = nullptr;     // the CFL minimum reduced over the slabs
     bool flags_valid = false;                // the sensor's flags belong to the current state's run
     int sms = 148;                           // multiprocessors of the context's device
-    nsb::WTmaMaps tma[2];                    // FP64 steps: tensor maps of W and W2 (face tiles, viscous planes)
+    nsb::VTmaMap vmap[2];                    // FP64 steps: tensor maps of W and W2 for the CD-2 viscous march
     // ns_time_step's transfer pipeline: the copy stream and its events (lazy)
     cudaStream_t copy = nullptr;
     std::vector<cudaEvent_t> ev;
@@ -271,8 +272,12 @@ static void prof_mark(ns_ctx* ctx, int cls) {
     g_prof->cls[g_prof->n++] = cls;
 }
 
-// the TMA tensor maps of the context's current W (FP64 steps)
-static const nsb::WTmaMaps& tma_maps(const ns_ctx* ctx) { return ctx->tma[ctx->tma[0].W == ctx->W ? 0 : 1]; }
+// the tensor map of the context's current W for the CD-2 viscous march, or null
+static const nsb::VTmaMap* visc_map(const ns_ctx* ctx) {
+    for (const nsb::VTmaMap& m : ctx->vmap)
+        if (m.W == ctx->W) return &m;
+    return nullptr;
+}
 
 // face fluxes of the current (W, U) along every convected axis (operator calls)
 static ns_status faces(ns_ctx* ctx) {
@@ -426,8 +431,8 @@ static ns_status xstage(ns_ctx* ctx, int st, double* Uin, double* Uout, unsigned
     if (with_faces) NS_TRY(step_faces(ctx, pl));
     const bool visc = ctx->p.diffusion == NS_DIFF_CENTERED;
     if (visc) {  // into the x-face array, which a step leaves unused otherwise
-        launch_viscous_tma(ctx->c.order / 2, phys(ctx), tma_maps(ctx), ctx->W, ctx->box, ctx->c, (double*)ctx->F[0],
-                           ctx->fb[0].fstride, ctx->slot + 4, ctx->sms, s, pl);
+        launch_viscous(ctx->c.order / 2, phys(ctx), visc_map(ctx), ctx->W, ctx->box, ctx->c, (double*)ctx->F[0],
+                       ctx->fb[0].fstride, ctx->slot + 4, ctx->sms, s, pl);
         NS_TRY(check_launch(ctx, 1));
         prof_mark(ctx, NS_PROF_VISCOUS);
     }
@@ -464,6 +469,7 @@ static void end_xstep(ns_ctx* ctx) {
     ctx->parity ^= 1;
     ctx->fused_ready = true;
     ctx->w_next_ready = true;
+    ctx->halos_stale = true;
     ctx->u_valid = true;
     ctx->w_valid = false;
     ctx->steps++;
@@ -526,9 +532,9 @@ static ns_status do_step(ns_ctx* ctx) {
     for (int st = 0; st < 3; st++) {
         NS_TRY(exchange(ctx, NS_EXCHANGE_HALO, in[st], nullptr));
         if (st == 0 && !w_ready)
-            launch_fill_prim(ctx->W, in[st], ctx->box, ctx->c, s, out[st], phys(ctx));
+            launch_fill_w(phys(ctx), ctx->W, in[st], ctx->box, ctx->c, s);
         else
-            launch_fill_halo(ctx->W, in[st], ctx->box, ctx->c, s, out[st], phys(ctx));
+            launch_fill_shell(phys(ctx), ctx->W, in[st], ctx->box, ctx->c, s);
         NS_TRY(check_launch(ctx, 1));
         prof_mark(ctx, NS_PROF_FILL);
         NS_TRY(xstage(ctx, st, in[st], out[st], cur, nxt, true, Planes()));
@@ -544,10 +550,15 @@ static ns_status do_step(ns_ctx* ctx) {
 static ns_status finalize_w(ns_ctx* ctx) {
     if (!ctx->w_valid) {
         ctx->w_next_ready = false;  // W is about to hold prim(U), not the next stage's W
-        if (ctx->halos_stale)
+        if (ctx->halos_stale && !ctx->xfused) {
             launch_fill_prim(ctx->W, ctx->U, ctx->box, ctx->c, ctx->stream);
-        else
+        } else {
+            if (ctx->halos_stale) {
+                launch_fill_uhalo(ctx->U, ctx->U2, ctx->box, ctx->c, ctx->stream);
+                NS_TRY(check_launch(ctx, 1));
+            }
             launch_prim_all(ctx->W, ctx->U, ctx->box, ctx->c, ctx->stream);
+        }
         NS_TRY(check_launch(ctx, 1));
         ctx->w_valid = true;
         ctx->halos_stale = false;
@@ -683,10 +694,9 @@ ns_status ns_create(const ns_params* p, ns_ctx** out) {
         return fail(NS_ERR_CUDA, "cudaStreamCreate failed");
     }
     ctx->stream = ctx->own;
-    // FP64 steps of the physical semantics keep the sound speed beside W, as a sixth
-    // plane that every writer of a stage's W fills: the Lax-Friedrichs speeds of the 18
-    // faces that a cell belongs to read it
-    const int wplanes = p->precision == NS_PREC_FP64 && p->convection != NS_CONV_NONE && phys(ctx) ? NS_NQ + 1 : NS_NQ;
+    // an FP64 stage's W has further planes in the physical semantics (ns_eos.cuh, store_w)
+    const bool planes = p->precision == NS_PREC_FP64 && p->convection != NS_CONV_NONE && phys(ctx);
+    const int wplanes = planes ? WPlanes<true>::value : WPlanes<false>::value;
     const size_t wbytes = soa_bytes(ctx->box) / NS_NQ * wplanes;
     A((void**)&ctx->W, wbytes);
     A((void**)&ctx->U, soa_bytes(ctx->box));
@@ -705,9 +715,12 @@ ns_status ns_create(const ns_params* p, ns_ctx** out) {
     ctx->xfused = !ctx->fused && p->precision == NS_PREC_FP64 && p->convection != NS_CONV_NONE;
     if (ctx->fused || ctx->xfused) A((void**)&ctx->U2, soa_bytes(ctx->box));
     if (ctx->xfused) A((void**)&ctx->W2, wbytes);
-    if (st == NS_OK && ctx->xfused && !(nsb::w_tma_encode(&ctx->tma[0], ctx->W, ctx->box, wplanes) &&
-                                        nsb::w_tma_encode(&ctx->tma[1], ctx->W2, ctx->box, wplanes)))
-        st = fail(NS_ERR_CUDA, "the driver makes no tensor map of the primitive field");
+    // the CD-2 viscous march reads tiles 32 cells wide through TMA where at least half of
+    // them is filled (measured: ns_viscous64.cu)
+    if (st == NS_OK && ctx->xfused && p->nz >= 16) {
+        nsb::visc_tma_encode(&ctx->vmap[0], ctx->W, ctx->box, wplanes);
+        nsb::visc_tma_encode(&ctx->vmap[1], ctx->W2, ctx->box, wplanes);
+    }
     A((void**)&ctx->diag, 8 * sizeof(double));
     A((void**)&ctx->clock, 2 * sizeof(double));
     if (st == NS_OK) {
@@ -946,29 +959,30 @@ static ns_status time_step_pipelined_run(ns_ctx* ctx, const double* Wh, double* 
         NS_CUDA(cudaStreamWaitEvent(s, ev[c], 0));
         launch_aos_to_soa(ctx->stage, ctx->W, ctx->box, s, sp);
         launch_step_begin(false, phys(ctx), ctx->W, ctx->U, ctx->U0, ctx->box, ctx->c, cur, s, sp);
-        launch_fill_prim(ctx->W, ctx->U0, ctx->box, ctx->c, s, ctx->U, phys(ctx), halo_interior(c));
+        launch_fill_w(phys(ctx), ctx->W, ctx->U0, ctx->box, ctx->c, s, halo_interior(c));
         NS_TRY(check_launch(ctx, 3));
         NS_TRY(step_faces(ctx, interior(c)));
     }
     // the x ghost planes fold onto planes of other chunks
-    launch_fill_prim(ctx->W, ctx->U0, ctx->box, ctx->c, s, ctx->U, phys(ctx), ghost_lo);
-    launch_fill_prim(ctx->W, ctx->U0, ctx->box, ctx->c, s, ctx->U, phys(ctx), ghost_hi);
+    launch_fill_w(phys(ctx), ctx->W, ctx->U0, ctx->box, ctx->c, s, ghost_lo);
+    launch_fill_w(phys(ctx), ctx->W, ctx->U0, ctx->box, ctx->c, s, ghost_hi);
     NS_TRY(check_launch(ctx, 2));
     NS_TRY(xstage(ctx, 0, ctx->U0, ctx->U, cur, nxt, false, Planes()));
     std::swap(ctx->W, ctx->W2);
 
     // stage 2 (U -> U2)
-    launch_fill_halo(ctx->W, ctx->U, ctx->box, ctx->c, s, ctx->U2, phys(ctx));
+    launch_fill_shell(phys(ctx), ctx->W, ctx->U, ctx->box, ctx->c, s);
     NS_TRY(check_launch(ctx, 1));
     NS_TRY(xstage(ctx, 1, ctx->U, ctx->U2, cur, nxt, true, Planes()));
     std::swap(ctx->W, ctx->W2);
 
     // stage 3 (U2 -> U) chunk by chunk into W2, which then holds prim(U) on every
     // cell (finalize_w); U's ghost cells are final after the fill
-    launch_fill_halo(ctx->W, ctx->U2, ctx->box, ctx->c, s, ctx->U, phys(ctx));
+    launch_fill_shell(phys(ctx), ctx->W, ctx->U2, ctx->box, ctx->c, s);
+    launch_fill_uhalo(ctx->U, ctx->U2, ctx->box, ctx->c, s);
     launch_prim_all(ctx->W2, ctx->U, ctx->box, ctx->c, s, ghost_lo);
     launch_prim_all(ctx->W2, ctx->U, ctx->box, ctx->c, s, ghost_hi);
-    NS_TRY(check_launch(ctx, 3));
+    NS_TRY(check_launch(ctx, 4));
     for (int c = 0; c < K; c++) {
         NS_TRY(xstage(ctx, 2, ctx->U2, ctx->U, cur, nxt, true, interior(c)));
         const Planes sp = span(c);
@@ -1072,7 +1086,7 @@ static ns_status device_status(ns_ctx* ctx) {
     unsigned long long werr = 0;
     NS_CUDA(cudaMemcpy(&werr, ctx->slot + 4, sizeof werr, cudaMemcpyDeviceToHost));
     if (werr & 2) return fail(NS_ERR_CUDA, "a TMA kernel found its shared-memory ring misaligned and did nothing");
-    if (werr) return fail(NS_ERR_TIMEOUT, "a TMA tile wait of a face, x-march or viscous kernel ran out of polls");
+    if (werr) return fail(NS_ERR_TIMEOUT, "a TMA tile wait of a viscous kernel ran out of polls");
     return NS_OK;
 }
 

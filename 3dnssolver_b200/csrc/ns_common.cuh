@@ -4,7 +4,7 @@
 // each plane the halo'd box (nx+6) x (ny+6) x NZp doubles with k fastest.
 // NZp = nz+6 rounded up to 8, and the plane stride (fstride) a multiple of 8
 // doubles, so every plane and every k-row starts on a 64-byte boundary (the
-// TMA tensor maps of the FP64 face kernels need 16-byte row strides).
+// TMA tensor maps of the CD-2 viscous march need 16-byte row strides).
 // Halos are real storage: the boundary fill writes them (the single-GPU form
 // of Domain::apply_boundary_conditions + Communicator::communicate), and the
 // per-operator entry points accept a caller's halos verbatim.
@@ -87,6 +87,23 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+#endif
+
+// Columns (j, k) of the marches along x: a block of 32 x 4 threads takes 4 neighbouring
+// rows, and its lanes run through the rows' columns group after group of 4 rows, so
+// that warps are full at any nz and the rows' neighbours along y are the block's own.
+inline long long row_tiles(const Box& b) { return ((long long)((b.ny + 3) / 4) * b.nz + 31) / 32; }
+#ifdef __CUDACC__
+// this thread's column; false (and some column of the grid) if it has none
+__device__ __forceinline__ bool row_tile(const Box& b, int& j, int& k) {
+    const long long e = (long long)blockIdx.x * 32 + threadIdx.x;
+    const long long g = e / b.nz;
+    j = (int)(g * 4 + threadIdx.y);
+    k = (int)(e % b.nz);
+    if (j < b.ny) return true;
+    j = 0;
+    return false;
+}
 #endif
 
 // Periodic wrap or Neumann clamp of an interior-coordinate index.

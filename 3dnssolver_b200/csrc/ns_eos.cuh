@@ -43,6 +43,25 @@ __device__ __forceinline__ double sound_speed(const double w[5], double gamma) {
     return __dmul_rn(gp, rsqrt_pos_nr(__dmul_rn(gp, w[0])));
 }
 
+// A stage's W in device memory: W in planes 0..4 and, for the physical semantics, what
+// its stencils need of every cell besides: T = p / rho in plane 5 (the heat flux of its
+// neighbours) and the sound speed in plane 6 (the Lax-Friedrichs speeds of the 18 faces
+// that a cell belongs to).
+template <bool PHYS>
+struct WPlanes {
+    static constexpr int value = PHYS ? 7 : 5;
+};
+template <bool PHYS>
+__device__ __forceinline__ void store_w(double* __restrict__ W, long long fs, long long o, const double w[5],
+                                        double gamma) {
+#pragma unroll
+    for (int q = 0; q < 5; q++) W[q * fs + o] = w[q];
+    if constexpr (PHYS) {
+        W[5 * fs + o] = div_pos_nr(w[1], w[0]);
+        W[6 * fs + o] = sound_speed(w, gamma);
+    }
+}
+
 // EqOfState::local_dt (src/eq_of_state.cpp:89-101), min over directions
 // max(|u+c|, |u-c|) is |u| + c for c >= 0, exactly and in rounding; the minimum
 // over the axes of d/(|u|+c) is taken as one reciprocal of the largest (|u|+c)/d

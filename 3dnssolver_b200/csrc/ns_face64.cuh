@@ -244,14 +244,14 @@ __device__ __forceinline__ void face_flux64(LoadW ld, LoadU ldu, Speed lam, cons
 }
 
 // The faces of a time step: U = cons(W), and at(q, s) gives plane q of stencil cell
-// s, W in planes 0..4 and (physical semantics) the sound speed in plane 5.
+// s, W in planes 0..4 and (physical semantics) the sound speed in plane 6.
 template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename At>
 __device__ __forceinline__ void face_flux64_w(At at, const Consts& c, double out[5]) {
     auto ld = [&](int s, double w[5]) {
 #pragma unroll
         for (int q = 0; q < 5; q++) w[q] = at(q, s);
     };
-    auto lam = [&](int s) { return fabs(at(2 + DIR, s)) + at(5, s); };
+    auto lam = [&](int s) { return fabs(at(2 + DIR, s)) + at(6, s); };
     face_flux64<DIR, CHAR, BORGES, PHYS, true>(ld, [](int, double*) {}, lam, c, out);
 }
 

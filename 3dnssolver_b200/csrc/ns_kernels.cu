@@ -9,8 +9,7 @@
 //                    (Weno5::compute_residual, CenteredDiffusion::compute_residual,
 //                    TimeScheme::substep), for operator calls and steps without
 //                    convection
-//   k_viscous_tma    centered viscous terms of an FP64 time step; its convection runs
-//                    in ns_sweeps.cu and ns_tma.cu
+// (an FP64 time step with convection: ns_stage64.cu and ns_viscous64.cu)
 // Per step: k_step_begin (dt reduction over W, then U = cons(W), U0 = U).
 #include <cuda_runtime.h>
 
@@ -25,7 +24,6 @@
 #include "ns_face64.cuh"
 #include "ns_kernels.h"
 #include "ns_tcgen05.cuh"
-#include "ns_tma.cuh"
 #include "ns_viscous.cuh"
 
 namespace nsb {
@@ -131,10 +129,10 @@ __global__ void __launch_bounds__(128) k_min_dt(const double* __restrict__ W, Bo
 // then W = prim(U) on every cell (eq_of_state.cpp:61-87).
 
 __global__ void __launch_bounds__(128) k_fill_prim(double* __restrict__ W, double* __restrict__ U,
-                                                   Box b, Consts c, double* __restrict__ Uhalo, bool speed, int ih0) {
+                                                   Box b, Consts c) {
     int kh = blockIdx.x * 32 + threadIdx.x;
     int jh = blockIdx.y * 4 + threadIdx.y;
-    int ih = blockIdx.z + ih0;
+    int ih = blockIdx.z;
     if (kh >= b.nz + 2 * NG || jh >= b.NY) return;
     int i = ih - NG, j = jh - NG, k = kh - NG;
     bool ox = i < 0 || i >= b.nx, oy = j < 0 || j >= b.ny, oz = k < 0 || k >= b.nz;
@@ -152,28 +150,57 @@ __global__ void __launch_bounds__(128) k_fill_prim(double* __restrict__ W, doubl
         for (int q = 0; q < 5; q++) {
             u[q] = U[q * b.fstride + s];
             U[q * b.fstride + o] = u[q];
-            if (Uhalo) Uhalo[q * b.fstride + o] = u[q];  // the stage's output buffer keeps the same halos
         }
     } else {
 #pragma unroll
         for (int q = 0; q < 5; q++) u[q] = U[q * b.fstride + o];
-        if (Uhalo && (i < 0 || i >= b.nx || oy || oz)) {  // edges, corners, exchanged planes travel unchanged
-#pragma unroll
-            for (int q = 0; q < 5; q++) Uhalo[q * b.fstride + o] = u[q];
-        }
     }
     prim_from_cons(u, c.gm1, w);
 #pragma unroll
     for (int q = 0; q < 5; q++) W[q * b.fstride + o] = w[q];
-    if (speed) W[5 * b.fstride + o] = sound_speed(w, c.gamma);
 }
 
-// Face halos only (the regions apply_boundary_conditions + communicate fill):
-// U there from its folded source, the same values into Uhalo, W = prim(U)
-// there.  The interior of W is the previous x-update's output.  Grid:
-// (ceil(3 * max face area / 128), 6 regions: x-, x+, y-, y+, z-, z+).
-__global__ void __launch_bounds__(128) k_fill_halo(double* __restrict__ W, double* __restrict__ U,
-                                                   Box b, Consts c, double* __restrict__ Uhalo, bool speed) {
+// An FP64 stage's W from its input U: W = prim(U) of the cell that each cell folds
+// onto, ghost cells beyond edges and corners too (the mixed derivatives of the
+// viscous terms read them); U's own ghost cells are left as they are, except that a
+// slab's exchanged x ghost planes are neighbours' cells.  On every cell of the planes
+// from ih0 on, or (SHELL) on the ghost cells alone.  Grid: cells as k_fill_prim's, or
+// (ceil(cells / 128), 3 parts of the shell: x ghost planes, y ghost rows, z ghost cells).
+template <bool PHYS, bool SHELL>
+__global__ void __launch_bounds__(128) k_fill_w(double* __restrict__ W, const double* __restrict__ U, Box b, Consts c,
+                                                int ih0) {
+    const int NZ = b.nz + 2 * NG;
+    int i, j, k;
+    if constexpr (SHELL) {
+        const long long t = (long long)blockIdx.x * 128 + threadIdx.x;
+        const int part = blockIdx.y;
+        const int n0 = part == 0 ? 2 * NG : b.nx, n1 = part == 0 ? b.NY : (part == 1 ? 2 * NG : b.ny),
+                  n2 = part == 2 ? 2 * NG : NZ;
+        if (t >= (long long)n0 * n1 * n2) return;
+        const int a0 = (int)(t / ((long long)n1 * n2)), a1 = (int)(t / n2 % n1), a2 = (int)(t % n2);
+        auto ghost = [](int a, int n) { return a < NG ? a - NG : a - NG + n; };
+        i = part == 0 ? ghost(a0, b.nx) : a0;
+        j = part == 0 ? a1 - NG : (part == 1 ? ghost(a1, b.ny) : a1);
+        k = part == 2 ? ghost(a2, b.nz) : a2 - NG;
+    } else {
+        k = blockIdx.x * 32 + threadIdx.x - NG;
+        j = blockIdx.y * 4 + threadIdx.y - NG;
+        i = blockIdx.z + ih0 - NG;
+        if (k >= b.nz + NG || j >= b.ny + NG) return;
+    }
+    const long long s = b.at(fold_x(i, b.nx, c) + NG, fold(j, b.ny, c.periodic[1]) + NG, fold(k, b.nz, c.periodic[2]) + NG);
+    double u[5], w[5];
+#pragma unroll
+    for (int q = 0; q < 5; q++) u[q] = U[q * b.fstride + s];
+    prim_from_cons(u, c.gm1, w);
+    store_w<PHYS>(W, b.fstride, b.at(i + NG, j + NG, k + NG), w, c.gamma);
+}
+
+// The face halos of U that a step leaves behind (the regions
+// apply_boundary_conditions + communicate fill): the third stage's input Us at the cell
+// each folds onto.  Grid: (ceil(3 * max face area / 128), 6 regions: x-, x+, y-, y+, z-, z+).
+__global__ void __launch_bounds__(128) k_fill_uhalo(double* __restrict__ U, const double* __restrict__ Us, Box b,
+                                                    Consts c) {
     const int ax = blockIdx.y >> 1, hi = blockIdx.y & 1;
     const long long t = (long long)blockIdx.x * 128 + threadIdx.x;
     // on a slab the y and z ghost rows of exchanged x ghost planes are filled too
@@ -194,30 +221,11 @@ __global__ void __launch_bounds__(128) k_fill_halo(double* __restrict__ W, doubl
         k = hi ? b.nz + layer : layer - NG;
     }
     const long long o = b.at(i + NG, j + NG, k + NG);
-    double u[5], w[5];
-    if (ax == 0 && x_exchanged(hi, b.nx, c)) {
-        // a neighbour's cells, already in place
+    const int sj = ax == 1 ? fold(j, b.ny, c.periodic[1]) : j;
+    const int sk = ax == 2 ? fold(k, b.nz, c.periodic[2]) : k;
+    const long long src = b.at(fold_x(i, b.nx, c) + NG, sj + NG, sk + NG);
 #pragma unroll
-        for (int q = 0; q < 5; q++) {
-            u[q] = U[q * b.fstride + o];
-            if (Uhalo) Uhalo[q * b.fstride + o] = u[q];
-        }
-    } else {
-        const int si = ax == 0 ? fold(i, b.nx, c.periodic[0]) : i;
-        const int sj = ax == 1 ? fold(j, b.ny, c.periodic[1]) : j;
-        const int sk = ax == 2 ? fold(k, b.nz, c.periodic[2]) : k;
-        const long long src = b.at(si + NG, sj + NG, sk + NG);
-#pragma unroll
-        for (int q = 0; q < 5; q++) {
-            u[q] = U[q * b.fstride + src];
-            U[q * b.fstride + o] = u[q];
-            if (Uhalo) Uhalo[q * b.fstride + o] = u[q];
-        }
-    }
-    prim_from_cons(u, c.gm1, w);
-#pragma unroll
-    for (int q = 0; q < 5; q++) W[q * b.fstride + o] = w[q];
-    if (speed) W[5 * b.fstride + o] = sound_speed(w, c.gamma);
+    for (int q = 0; q < 5; q++) U[q * b.fstride + o] = Us[q * b.fstride + src];
 }
 
 // ---------------------------------------------------------------------------
@@ -376,157 +384,6 @@ __device__ __forceinline__ void viscous_reference(const double* __restrict__ W, 
     }
     viscous_reference_terms<TV>(Dx, Dy, Dxx, Dyy, Dxy, Dyx, TV(W[2 * fs + o]), TV(W[3 * fs + o]),
                                 TV(W[1 * fs + o]), TV(W[o]), c, r);
-}
-
-// Reference semantics: the terms of viscous_reference above, in the same
-// arithmetic order, from an accessor at(q, ox, oy) of W at offsets ox along x
-// and oy along y of the cell (the TMA-marched kernel reads its shared-memory
-// planes through it).  The mixed derivatives read the rows/columns the
-// per-thread kernel wraps to; the box holds them as the filled face halos.
-template <int H, typename TV, typename At>
-__device__ __forceinline__ void viscous_reference_core(At at, const Box& b, const Consts& c, int i, int j,
-                                                       TV r[5]) {
-    TV cx1[2 * H + 1], cy1[2 * H + 1], cxx[2 * H + 1], cyy[2 * H + 1];
-#pragma unroll
-    for (int t = 0; t <= 2 * H; t++) {
-        cx1[t] = TV(c.df[3 - H + t] * c.inv_dx);
-        cy1[t] = TV(c.df[3 - H + t] * c.inv_dy);
-        cxx[t] = TV(c.ddf[3 - H + t] * c.inv_dx * c.inv_dx);
-        cyy[t] = TV(c.ddf[3 - H + t] * c.inv_dy * c.inv_dy);
-    }
-    TV Dx[4], Dy[4], Dxx[4], Dyy[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        TV sx1 = 0, sy1 = 0, sxx = 0, syy = 0;
-#pragma unroll
-        for (int t = 0; t <= 2 * H; t++) {
-            TV wx = TV(at(q, t - H, 0));
-            TV wy = TV(at(q, 0, t - H));
-            if (t != H) { sx1 += wx * cx1[t]; sy1 += wy * cy1[t]; }
-            sxx += wx * cxx[t];
-            syy += wx * cyy[t];
-        }
-        Dx[q] = sx1; Dy[q] = sy1; Dxx[q] = sxx; Dyy[q] = syy;
-    }
-    TV Dxy[2], Dyx[2];
-#pragma unroll
-    for (int v = 0; v < 2; v++) {
-        const int q = 2 + v;
-        TV sxy = 0, syx = 0;
-#pragma unroll
-        for (int s = 0; s <= 2 * H; s++) {
-            if (s == H) continue;
-            const int jj = j + s - H;
-            {
-                TV dx = 0;
-#pragma unroll
-                for (int t = 0; t <= 2 * H; t++)
-                    if (t != H) dx += TV(at(q, t - H, s - H)) * cx1[t];
-                if ((jj >= 0 && jj < b.ny) || c.periodic[1]) sxy += dx * cy1[s];
-            }
-            const int ii = i + s - H;
-            {
-                TV dy = 0;
-#pragma unroll
-                for (int t = 0; t <= 2 * H; t++)
-                    if (t != H) dy += TV(at(q, s - H, t - H)) * cy1[t];
-                if (x_inside(ii, b.nx, c)) syx += dy * cx1[s];
-            }
-        }
-        Dxy[v] = sxy; Dyx[v] = syx;
-    }
-    viscous_reference_terms<TV>(Dx, Dy, Dxx, Dyy, Dxy, Dyx, TV(at(2, 0, 0)), TV(at(3, 0, 0)), TV(at(1, 0, 0)),
-                                TV(at(0, 0, 0)), c, r);
-}
-
-// Physical semantics: the full 3D viscous terms of viscous_physical below, in
-// the same arithmetic order (p / rho by div_pos_nr, within an ulp of the
-// division), from two accessors of W around the cell (the
-// TMA-marched kernel reads its shared-memory planes through them; the
-// per-thread kernel keeps its own loads, which compile to fewer registers):
-// ld1(q, ax, t) = field q at offset t - H along axis ax, ld2(q, a, s, bx, t) =
-// field q at offsets s - H along a and t - H along bx (mixed derivatives).
-// All axis loops unroll at compile time (2D skips the z terms at run time).
-template <int H, typename TV, typename Ld1, typename Ld2>
-__device__ __forceinline__ void viscous_physical_core(Ld1 ld1, Ld2 ld2, const Consts& c, TV r[5]) {
-    constexpr int NS = 2 * H + 1;
-    const bool three = c.dim == 3;
-    const double inv[3] = {c.inv_dx, c.inv_dy, c.inv_dz};
-    TV c1[3][NS], c2[3][NS];
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int t = 0; t < NS; t++) {
-            c1[a][t] = TV(c.df[3 - H + t] * inv[a]);
-            c2[a][t] = TV(c.ddf[3 - H + t] * inv[a] * inv[a]);
-        }
-    TV gu[3][3], lap[3], gdiv[3], lapT = 0;
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        lap[a] = 0;
-        gdiv[a] = 0;
-#pragma unroll
-        for (int bx = 0; bx < 3; bx++) gu[a][bx] = 0;
-    }
-#pragma unroll
-    for (int bx = 0; bx < 3; bx++) {
-        if (bx == 2 && !three) continue;
-#pragma unroll
-        for (int t = 0; t < NS; t++) {
-            // p / rho (rho > 0): the Newton-Raphson quotient of the WENO weights in FP64
-            TV T;
-            if constexpr (sizeof(TV) == 8) T = div_pos_nr(ld1(1, bx, t), ld1(0, bx, t));
-            else T = TV(ld1(1, bx, t)) / TV(ld1(0, bx, t));
-#pragma unroll
-            for (int a = 0; a < 3; a++) {
-                const TV va = TV(ld1(2 + a, bx, t));
-                if (t != H) gu[a][bx] += va * c1[bx][t];
-                lap[a] += va * c2[bx][t];
-                if (a == bx) gdiv[a] += va * c2[bx][t];
-            }
-            lapT += T * c2[bx][t];
-        }
-    }
-    // grad(div u)_a += d/dx_a (d u_b / dx_b) for b != a
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int bx = 0; bx < 3; bx++) {
-            if (a == bx || ((a == 2 || bx == 2) && !three)) continue;
-            TV acc = 0;
-#pragma unroll
-            for (int s = 0; s < NS; s++) {
-                if (s == H) continue;
-                TV inner = 0;
-#pragma unroll
-                for (int t = 0; t < NS; t++) {
-                    if (t == H) continue;
-                    inner += TV(ld2(2 + bx, a, s, bx, t)) * c1[bx][t];
-                }
-                acc += inner * c1[a][s];
-            }
-            gdiv[a] += acc;
-        }
-    const TV mu = TV(c.mu), lamb = TV(c.lamb);
-    const TV uv[3] = {TV(ld1(2, 0, H)), TV(ld1(3, 0, H)), TV(ld1(4, 0, H))};
-    const TV div = gu[0][0] + gu[1][1] + gu[2][2];
-    TV work = 0, diss = 0, mom[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        mom[a] = mu * lap[a] + (mu + lamb) * gdiv[a];
-        work += uv[a] * mom[a];
-    }
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int bx = 0; bx < 3; bx++) {
-            const TV tab = mu * (gu[a][bx] + gu[bx][a]) + (a == bx ? lamb * div : TV(0));
-            diss += tab * gu[a][bx];
-        }
-    r[2] -= mom[0];
-    r[3] -= mom[1];
-    r[4] -= mom[2];
-    r[1] -= work + diss + TV(c.heat) * mu * lapT;
 }
 
 // Physical semantics: full 3D viscous stress and heat flux with constant mu
@@ -696,127 +553,6 @@ __global__ void __launch_bounds__(128, NS_UPDATE_MINB) k_update(const double* __
 #pragma unroll
             for (int q = 0; q < 5; q++) Rout[q * b.fstride + o] += r[q];
         }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// The viscous terms of every interior cell (residual components 1..4) into V, from
-// planes of W that the TMA unit loads into a ring while the block marches lx
-// cells along x.  A block owns 4
-// rows x 32 columns; one plane is the box of ViscTile<H> (5 fields; 8.2, 12.2
-// and 15.2 KB for CD-2, 4, 6), so each cell of W crosses L2 once per block
-// instead of once per stencil.  The ring holds the 2H+1 planes of the current
-// cell and, for CD-2 and CD-4, the next plane in flight; CD-6 keeps 7 slots
-// (two blocks per SM) and loads the next plane as the last one is released.
-// A cell within H cells of the boundary along two axes or more needs folded
-// edge or corner ghost cells for its mixed derivatives, which no fill writes
-// and so the box does not hold: it reads the device state, folding.  Waits are
-// bounded (the error word receives 1 and the block ends).
-template <int H>
-struct ViscRing {
-    using VT = ViscTile<H>;
-    static constexpr int QS = VT::BZ * VT::BY, ELEMS = 5 * QS;
-    static constexpr int STRIDE = (ELEMS + 15) / 16 * 16;  // 128-byte aligned slots
-    static constexpr uint32_t BYTES = ELEMS * 8;
-    static constexpr int LEAD = H < 3 ? 1 : 0;             // planes in flight beyond the stencil
-    static constexpr int NSLOT = 2 * H + 1 + LEAD;
-    // the ring, then its mbarriers: no static shared memory, so the dynamic ring
-    // starts at the window's base (TMA writes want 128-byte aligned destinations)
-    static constexpr size_t smem = (size_t)NSLOT * STRIDE * 8 + NSLOT * 8;
-    static constexpr int MINB = H == 1 ? 4 : (H == 2 ? 3 : 2);
-};
-
-template <int H, bool PHYS>
-__global__ void __launch_bounds__(128, ViscRing<H>::MINB)
-    k_viscous_tma(const __grid_constant__ CUtensorMap map, const double* __restrict__ W, Box b, Consts c,
-                  double* __restrict__ V, long long vs, unsigned long long* __restrict__ err, int xlo, int xhi,
-                  int lx) {
-    using VT = ViscTile<H>;
-    using VR = ViscRing<H>;
-    constexpr int NSLOT = VR::NSLOT, STRIDE = VR::STRIDE, QS = VR::QS, BZ = VT::BZ;
-    extern __shared__ __align__(128) double vring[];  // [NSLOT][5][BY][BZ], then NSLOT mbarriers
-    unsigned long long* full = reinterpret_cast<unsigned long long*>(vring + NSLOT * STRIDE);
-    const int lane = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + lane;
-    if (tc::smem_u32(vring) & 127u) {  // a TMA destination must be 128-byte aligned: report, touch nothing
-        if (tid == 0) atomicOr(err, 2ull);
-        return;
-    }
-    const int k0 = blockIdx.x * 32, j0 = blockIdx.y * 4, x0 = xlo + blockIdx.z * lx;
-    const int x1 = min(x0 + lx, xhi);
-    const int k = k0 + lane, j = j0 + ty;
-    const bool live = k < b.nz && j < b.ny;
-    // plane p (x0 - H <= p <= x1 - 1 + H) is the (p - x0 + H)-th load of the block
-    auto slot = [&](int p) { return (p - x0 + H) % NSLOT; };
-    auto bar = [&](int p) { return tc::smem_u32(&full[slot(p)]); };
-    auto par = [&](int p) { return (uint32_t)(((p - x0 + H) / NSLOT) & 1); };
-    auto issue = [&](int p) {
-        mbar_expect_tx(bar(p), VR::BYTES);
-        tma_load_4d(tc::smem_u32(vring + slot(p) * STRIDE), &map, k0 + VT::Z0, j0 + NG - H, p + NG, 0, bar(p));
-    };
-    if (tid == 0)
-        for (int q = 0; q < NSLOT; q++) tc::mbar_init(tc::smem_u32(&full[q]), 1);
-    __syncthreads();
-    const int last = x1 - 1 + H;  // the last plane the block reads
-    if (tid == 0)
-        for (int p = x0 - H; p <= min(x0 + H + VR::LEAD, last); p++) issue(p);
-    bool ok = true;
-    for (int p = x0 - H; p < x0 + H; p++) ok = ok && tc::mbar_wait(bar(p), par(p), kTilePolls);
-    int waited = ok ? x0 + H - 1 : x0 - H - 1;  // planes up to this one have landed
-    // within H cells of the boundary along two axes or more, a mixed derivative
-    // reaches an edge or corner ghost cell
-    const int nbjk = (j < H || j >= b.ny - H) + (k < H || k >= b.nz - H);
-    const int cc = (ty + H) * BZ + lane + VT::C0;
-    for (int i = x0; i < x1; i++) {
-        if (ok && i + H > waited) {
-            ok = tc::mbar_wait(bar(i + H), par(i + H), kTilePolls);
-            if (ok) waited = i + H;
-        }
-        if (ok && live) {
-            double rv[5] = {0, 0, 0, 0, 0};
-            if (nbjk + (i < H || i >= b.nx - H) >= 2) {
-                if constexpr (PHYS)
-                    viscous_physical<H, double>(W, b, c, i, j, k, rv);
-                else
-                    viscous_reference<H, double>(W, b, c, i, j, k, rv);
-            } else if constexpr (!PHYS) {
-                const double* P[2 * H + 1];
-#pragma unroll
-                for (int s = 0; s <= 2 * H; s++) P[s] = vring + slot(i - H + s) * STRIDE;
-                auto at = [&](int q, int ox, int oy) { return P[H + ox][q * QS + cc + oy * BZ]; };
-                viscous_reference_core<H, double>(at, b, c, i, j, rv);
-            } else {
-                const double* P[2 * H + 1];
-#pragma unroll
-                for (int s = 0; s <= 2 * H; s++) P[s] = vring + slot(i - H + s) * STRIDE;
-                auto at = [&](int q, int ox, int oy, int oz) { return P[H + ox][q * QS + cc + oy * BZ + oz]; };
-                auto ld1 = [&](int q, int ax, int t) {
-                    const int d = t - H;
-                    return at(q, ax == 0 ? d : 0, ax == 1 ? d : 0, ax == 2 ? d : 0);
-                };
-                auto ld2 = [&](int q, int a, int s, int bx, int t) {
-                    int o[3] = {0, 0, 0};
-                    o[a] += s - H;
-                    o[bx] += t - H;
-                    return at(q, o[0], o[1], o[2]);
-                };
-                viscous_physical_core<H, double>(ld1, ld2, c, rv);
-            }
-#pragma unroll
-            for (int q = 1; q < 5; q++) V[(q - 1) * vs + ((long long)i * b.ny + j) * b.nz + k] = rv[q];
-        }
-        // every thread is done with plane i - H (and agrees on whether a wait ran out)
-        if (__syncthreads_or(!ok)) {
-            if (tid == 0) {
-                atomicOr(err, 1ull);
-                // the loads still in flight: planes waited + 1 .. the last one issued
-                const int issued = min(i + H + VR::LEAD, last);
-                for (int p = waited + 1; p <= issued; p++) tc::mbar_wait(bar(p), par(p), kTilePolls);
-            }
-            __syncthreads();
-            return;
-        }
-        const int next = i + H + 1 + VR::LEAD;  // into the slot of plane i - H
-        if (tid == 0 && next <= last) issue(next);
     }
 }
 
@@ -1038,15 +774,28 @@ void launch_min_dt(bool phys, const double* W, const Box& b, const Consts& c, un
     else k_min_dt<false><<<interior_grid(b), dim3(32, 4), 0, s>>>(W, b, c, slot);
 }
 
-void launch_fill_halo(double* W, double* U, const Box& b, const Consts& c, cudaStream_t s, double* Uhalo, bool speed) {
-    const long long nxe = b.nx + (c.ext_x ? 2 * NG : 0);  // slabs: y/z ghost rows of the x ghost planes too
-    const long long area = std::max(std::max((long long)b.ny * b.nz, nxe * b.nz), nxe * b.ny);
-    k_fill_halo<<<dim3((unsigned)((3 * area + 127) / 128), 6), 128, 0, s>>>(W, U, b, c, Uhalo, speed);
+void launch_fill_prim(double* W, double* U, const Box& b, const Consts& c, cudaStream_t s) {
+    k_fill_prim<<<cell_grid(b), dim3(32, 4), 0, s>>>(W, U, b, c);
 }
 
-void launch_fill_prim(double* W, double* U, const Box& b, const Consts& c, cudaStream_t s, double* Uhalo,
-                      bool speed, Planes pl) {
-    k_fill_prim<<<cell_grid(b, pl), dim3(32, 4), 0, s>>>(W, U, b, c, Uhalo, speed, pl.lo);
+void launch_fill_w(bool phys, double* W, const double* U, const Box& b, const Consts& c, cudaStream_t s, Planes pl) {
+    const dim3 g = cell_grid(b, pl), blk(32, 4);
+    if (phys) k_fill_w<true, false><<<g, blk, 0, s>>>(W, U, b, c, pl.lo);
+    else k_fill_w<false, false><<<g, blk, 0, s>>>(W, U, b, c, pl.lo);
+}
+
+void launch_fill_shell(bool phys, double* W, const double* U, const Box& b, const Consts& c, cudaStream_t s) {
+    const long long NZ = b.nz + 2 * NG;
+    const long long n = 2 * NG * std::max(std::max(b.NY * NZ, b.nx * NZ), (long long)b.nx * b.ny);
+    const dim3 g((unsigned)((n + 127) / 128), 3);
+    if (phys) k_fill_w<true, true><<<g, 128, 0, s>>>(W, U, b, c, 0);
+    else k_fill_w<false, true><<<g, 128, 0, s>>>(W, U, b, c, 0);
+}
+
+void launch_fill_uhalo(double* U, const double* Us, const Box& b, const Consts& c, cudaStream_t s) {
+    const long long nxe = b.nx + (c.ext_x ? 2 * NG : 0);  // slabs: y/z ghost rows of the x ghost planes too
+    const long long area = std::max(std::max((long long)b.ny * b.nz, nxe * b.nz), nxe * b.ny);
+    k_fill_uhalo<<<dim3((unsigned)((3 * area + 127) / 128), 6), 128, 0, s>>>(U, Us, b, c);
 }
 
 template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename T, typename TF>
@@ -1130,34 +879,6 @@ void launch_update(const UpdateArgs& a, cudaStream_t s) {
     else update_mode<MODE_RHS>(a, s);
 }
 
-template <int H, bool PHYS>
-static void visc_tma_one(const WTmaMaps& m, const double* W, const Box& b, const Consts& c, double* V, long long vs,
-                         unsigned long long* err, int sms, cudaStream_t s, Planes pl) {
-    constexpr size_t bytes = ViscRing<H>::smem;
-    // the attribute is per device; a refusal surfaces as the launch's error
-    cudaFuncSetAttribute(k_viscous_tma<H, PHYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    const int x0 = pl.n < 0 ? 0 : pl.lo, np = pl.n < 0 ? b.nx : pl.n;
-    dim3 grid((b.nz + 31) / 32, (b.ny + 3) / 4);
-    // a segment costs its cells and the latency of its first 2H planes
-    const int lx = march_length(np, (long long)grid.x * grid.y, sms * ViscRing<H>::MINB, 1.5 + 0.5 * H, 32);
-    grid.z = (np + lx - 1) / lx;
-    k_viscous_tma<H, PHYS><<<grid, dim3(32, 4), bytes, s>>>(*reinterpret_cast<const CUtensorMap*>(m.map[H - 1]), W, b, c, V,
-                                                             vs, err, x0, x0 + np, lx);
-}
-
-void launch_viscous_tma(int h, bool phys, const WTmaMaps& m, const double* W, const Box& b, const Consts& c, double* V,
-                        long long vs, unsigned long long* err, int sms, cudaStream_t s, Planes pl) {
-    if (phys) {
-        if (h == 1) visc_tma_one<1, true>(m, W, b, c, V, vs, err, sms, s, pl);
-        else if (h == 2) visc_tma_one<2, true>(m, W, b, c, V, vs, err, sms, s, pl);
-        else visc_tma_one<3, true>(m, W, b, c, V, vs, err, sms, s, pl);
-    } else {
-        if (h == 1) visc_tma_one<1, false>(m, W, b, c, V, vs, err, sms, s, pl);
-        else if (h == 2) visc_tma_one<2, false>(m, W, b, c, V, vs, err, sms, s, pl);
-        else visc_tma_one<3, false>(m, W, b, c, V, vs, err, sms, s, pl);
-    }
-}
-
 void launch_check_state(const double* A, bool prim, const Box& b, const Consts& c,
                         unsigned long long* count, cudaStream_t s) {
     if (prim) k_check_state<true><<<interior_grid(b), dim3(32, 4), 0, s>>>(A, b, c, count);
@@ -1181,6 +902,25 @@ void launch_soa_to_aos(const double* S, double* A, const Box& b, cudaStream_t s,
 }
 void launch_diagnostics(const double* U, const Box& b, const Consts& c, double* acc, cudaStream_t s) {
     k_diagnostics<<<interior_grid(b), dim3(32, 4), 0, s>>>(U, b, c, acc);
+}
+
+// The bounded wait of the tensor-core kernels, on a phase that no
+// arrival or transaction completes: it must give up after `polls` polls.
+__global__ void k_wait_probe(unsigned polls, unsigned long long* __restrict__ out) {
+    __shared__ __align__(8) unsigned long long bar;
+    if (threadIdx.x == 0) tc::mbar_init(tc::smem_u32(&bar), 1);
+    __syncthreads();
+    const bool done = tc::mbar_wait(tc::smem_u32(&bar), 0, polls);
+    if (__syncthreads_or(done)) {
+        if (threadIdx.x == 0) out[0] = 0;
+    } else if (threadIdx.x == 0) {
+        out[0] = 1;
+    }
+}
+
+cudaError_t launch_wait_probe(unsigned polls, unsigned long long* out, cudaStream_t s) {
+    k_wait_probe<<<1, 32, 0, s>>>(polls, out);
+    return cudaGetLastError();
 }
 
 }  // namespace nsb

@@ -115,37 +115,21 @@ void launch_prim_all(double* W, const double* U, const Box& b, const Consts& c, 
 void launch_cons_all(const double* W, double* U, const Box& b, const Consts& c, cudaStream_t s);
 void launch_min_dt(bool phys, const double* W, const Box& b, const Consts& c, unsigned long long* slot,
                    cudaStream_t s);
-// face halos of U and W only (the interior of W is already the stage's)
-// speed: W has a sixth plane, which receives the sound speed
-void launch_fill_halo(double* W, double* U, const Box& b, const Consts& c, cudaStream_t s,
-                      double* Uhalo = nullptr, bool speed = false);
-// Uhalo (nullable) receives the same face-halo values as U; speed as above
-void launch_fill_prim(double* W, double* U, const Box& b, const Consts& c, cudaStream_t s,
-                      double* Uhalo = nullptr, bool speed = false, Planes pl = Planes());
+// U's face halos from its interior, then W = prim(U) on every cell (operator calls,
+// and steps without convection or in FP32)
+void launch_fill_prim(double* W, double* U, const Box& b, const Consts& c, cudaStream_t s);
+// W (and, phys, its two further planes) of an FP64 stage from the stage's input U, on
+// every cell (of planes pl) or on the ghost cells alone
+void launch_fill_w(bool phys, double* W, const double* U, const Box& b, const Consts& c, cudaStream_t s,
+                   Planes pl = Planes());
+void launch_fill_shell(bool phys, double* W, const double* U, const Box& b, const Consts& c, cudaStream_t s);
+// U's face halos after an FP64 step, from the third stage's input Us
+void launch_fill_uhalo(double* U, const double* Us, const Box& b, const Consts& c, cudaStream_t s);
 void launch_face_flux(int dir, bool chr, bool borges, bool phys, bool fp32, const double* W,
                       const double* U, const Box& b, const Consts& c, void* F, const FaceBox& fb, cudaStream_t s);
 // the y- (dir 1) or z-faces (dir 2) of an FP64 stage, from W (and the sound speed plane) alone
 void launch_step_faces(int dir, bool chr, bool borges, bool phys, const double* W, const Box& b, const Consts& c,
                        double* F, const FaceBox& fb, cudaStream_t s, Planes pl = Planes());
-// TMA tensor maps of one W buffer (ns_tma.cu): map[h - 1] the planes of the viscous
-// march of half-width h (CD-2h); each holds a CUtensorMap (128 bytes, 64-byte aligned)
-struct WTmaMaps {
-    alignas(64) unsigned char map[3][128];
-    const double* W = nullptr;
-};
-// one plane of the TMA-marched viscous kernel of half-width H for a block of
-// 4 rows x 32 columns (halo'd coordinates): rows j0+3-H .. j0+6+H, columns from
-// k0+3-H rounded down to even (TMA's innermost start rule), 32 + 2H (+1) wide
-// rounded up to even; lane 0's cell sits in column C0
-template <int H>
-struct ViscTile {
-    static constexpr int Z0 = (3 - H) & ~1;          // box start minus k0
-    static constexpr int C0 = 3 - Z0;                // lane 0's cell column in the box
-    static constexpr int BZ = (C0 + 32 + H + 1) & ~1;  // columns
-    static constexpr int BY = 4 + 2 * H;             // rows
-};
-// W: `planes` planes (5, or 6 with the sound speed); false if no map can be made
-bool w_tma_encode(WTmaMaps* m, const double* W, const Box& b, int planes);
 // largest ulp distance between div_pos_nr and the IEEE quotient over n draws
 cudaError_t launch_div_check(long long n, unsigned long long seed, unsigned long long* max_ulp, cudaStream_t s);
 // one block waits (bounded) on an mbarrier phase nothing completes; out[0] = 1
@@ -154,12 +138,18 @@ cudaError_t launch_wait_probe(unsigned polls, unsigned long long* out, cudaStrea
 void launch_update(const UpdateArgs& a, cudaStream_t s);
 // x-faces + update of an FP64 stage in one march
 void launch_xmarch(bool chr, bool borges, bool phys, const XMarchArgs& a, cudaStream_t s, Planes pl = Planes());
-// viscous terms (components 1..4) of every interior cell into V (as XMarchArgs's),
-// from TMA-loaded planes of the W that m maps, marched along x (half-width
-// h = 1, 2, 3 of the centered scheme); *err receives 1 if a wait ran out
-void launch_viscous_tma(int h, bool phys, const WTmaMaps& m, const double* W, const Box& b, const Consts& c,
-                        double* V, long long vs, unsigned long long* err, int sms, cudaStream_t s,
-                        Planes pl = Planes());
+// TMA tensor map of a stage's W (of 5 or 7 planes) for the CD-2 viscous march (a
+// CUtensorMap: 128 bytes, 64-byte aligned); false if none can be made
+struct VTmaMap {
+    alignas(64) unsigned char map[128];
+    const double* W = nullptr;
+};
+bool visc_tma_encode(VTmaMap* m, const double* W, const Box& b, int planes);
+// viscous terms (components 1..4) of every interior cell into V (as XMarchArgs's) from
+// a stage's W; half-width h = 1, 2, 3 of the centered scheme; m: W's map (nullable);
+// *err receives 1 if a wait ran out
+void launch_viscous(int h, bool phys, const VTmaMap* m, const double* W, const Box& b, const Consts& c, double* V,
+                    long long vs, unsigned long long* err, int sms, cudaStream_t s, Planes pl = Planes());
 // slab halo exchange: pack the outer interior planes of a side / unpack into its ghost planes
 void launch_slab_pack(const double* U, const Box& b, int side, double* buf, cudaStream_t s);
 void launch_slab_unpack(double* U, const Box& b, int side, const double* buf, cudaStream_t s);

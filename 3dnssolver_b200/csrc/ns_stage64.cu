@@ -103,13 +103,12 @@ __global__ void __launch_bounds__(128, kXMarchBlocks)
              double m1, double m2, double mc, double* __restrict__ clock, int xlo, int xhi, int lx) {
     constexpr int NF = XMarchLayout<PHYS>::NF, NS = XMarchLayout<PHYS>::NS;
     extern __shared__ double xsm[];
-    const int t = threadIdx.x;
+    const int t = threadIdx.y * 32 + threadIdx.x;
     double* ring = xsm + t;                // [NS][NF][128]
     double* fprev = ring + NS * NF * 128;  // [5][128]
     double* opnd = fprev + 5 * 128;        // [10][128]: U0 and U of the cell
-    const long long col = (long long)blockIdx.x * 128 + t;
-    const bool live = col < (long long)b.ny * b.nz;
-    const int j = live ? (int)(col / b.nz) : 0, k = live ? (int)(col % b.nz) : 0;
+    int j, k;
+    const bool live = row_tile(b, j, k);
     // threads outside the grid march no cells but join the block reduction of LAST
     const int x0 = xlo + blockIdx.y * lx, x1 = live ? min(x0 + lx, xhi) : x0 - 1;
     double best = INFINITY;
@@ -124,7 +123,7 @@ __global__ void __launch_bounds__(128, kXMarchBlocks)
         const double* w = W + b.at(p + NG, j + NG, k + NG);
         double* d = ring + ((p - x0 + 3) % NS) * NF * 128;
 #pragma unroll
-        for (int q = 0; q < NF; q++) cp_async8(d + q * 128, w + q * b.fstride);
+        for (int q = 0; q < NF; q++) cp_async8(d + q * 128, w + (q < 5 ? q : 6) * b.fstride);
     };
     if (live)
         for (int p = x0 - 3; p < x0 + 3; p++) load_plane(p);
@@ -144,7 +143,7 @@ __global__ void __launch_bounds__(128, kXMarchBlocks)
         const double* P[6];
 #pragma unroll
         for (int s = 0; s < 6; s++) P[s] = ring + ((i - x0 + 1 + s) % NS) * NF * 128;
-        auto at = [&](int q, int s) { return P[s][q * 128]; };
+        auto at = [&](int q, int s) { return P[s][(q < 5 ? q : 5) * 128]; };
         double f[5];
         face_flux64_w<0, CHAR, BORGES, PHYS>(at, c, f);
         if (i < x0) {
@@ -179,9 +178,7 @@ __global__ void __launch_bounds__(128, kXMarchBlocks)
             for (int q = 0; q < 5; q++) U0[q * b.fstride + o] = u0[q];
             prim_from_cons(u0, c.gm1, w);  // the next step's first stage reads prim(U0)
         }
-#pragma unroll
-        for (int q = 0; q < 5; q++) Wn[q * b.fstride + o] = w[q];
-        if constexpr (PHYS) Wn[5 * b.fstride + o] = sound_speed(w, c.gamma);
+        store_w<PHYS>(Wn, b.fstride, o, w, c.gamma);
     }
     cp_async_wait_all();
     if constexpr (LAST) block_min_to(best, slot_next);
@@ -256,10 +253,10 @@ static void xmarch_one(const XMarchArgs& a, cudaStream_t s, Planes pl) {
     // the attribute is per device; a refusal surfaces as the launch's error
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     const int x0 = pl.n < 0 ? 0 : pl.lo, np = pl.n < 0 ? a.b.nx : pl.n;
-    const long long blocks = ((long long)a.b.ny * a.b.nz + 127) / 128;
+    const long long blocks = row_tiles(a.b);
     // a segment costs its cells, its first face and the latency of its first planes
     const int lx = march_length(np, blocks, a.sms * kXMarchBlocks, 2.0, 64);
-    kern<<<dim3((unsigned)blocks, (np + lx - 1) / lx), 128, bytes, s>>>(
+    kern<<<dim3((unsigned)blocks, (np + lx - 1) / lx), dim3(32, 4), bytes, s>>>(
         a.W, a.U, a.U0, a.Uout, a.Wnext, a.Fy, a.Fz, a.V, a.vs, a.b, a.fy, a.fz, a.c, a.slot,
         LAST ? a.slot_next : nullptr, a.m1, a.m2, a.mc, a.clock, x0, x0 + np, lx);
 }
