@@ -94,7 +94,7 @@ __device__ __forceinline__ float gelu_grad(float x) {
 }
 
 // smem copy of the network: bf16 weight tiles (row = output unit), FP32 vectors
-struct MlpSmem {
+struct alignas(16) MlpSmem {
     __nv_bfloat16 W1[SH * XS];
     __nv_bfloat16 W2[SH * XS];
     __nv_bfloat16 W2T[SH * XS];  // backward only
@@ -320,17 +320,25 @@ __global__ void __launch_bounds__(128) k_sensor_harvest(const double* __restrict
 }
 
 // ---------------------------------------------------------------------------
-// training: fused forward + backward of 128 samples per block (4 warps x 32),
-// BCE-with-logits loss with positive-class weight, gradients summed in shared
-// memory then added to the global FP32 gradient.
+// training: a mini-batch is two kernels.  k_mlp_train runs forward and backward, a warp
+// per tile of 16 samples, BCE-with-logits loss with positive-class weight; the
+// gradient stays in the warp's registers (the weights' as MMA accumulators, over all
+// its tiles) and every block writes one row of partial sums.  k_adam adds the rows,
+// takes the Adam step and leaves the network in the form that the next batch copies
+// to shared memory.  No atomics: a run repeats bit for bit.
+// (With the gradients summed by shared-memory atomics, some 150 a thread on 2145
+// addresses, a batch of 4096 took 138 us in the first kernel alone; now 12 us, and 4.6 in
+// the second.)
+
+constexpr int SPR = (SP + 1 + 3) / 4 * 4;  // floats per row of partial sums: the parameters', then the loss
+constexpr int kTrainWarps = 2, kTrainBlocks = 148;
 
 struct TrainSmem {
     MlpSmem m;
-    __nv_bfloat16 X[4][32 * XS];   // per warp: inputs
-    __nv_bfloat16 H[4][32 * XS];   // per warp: GELU(z1) (then reused)
-    __nv_bfloat16 D[4][32 * XS];   // per warp: dZ2, then dZ1
-    float grad[SP];
-    float loss;
+    __nv_bfloat16 X[kTrainWarps][16 * XS];  // per warp: inputs
+    __nv_bfloat16 H[kTrainWarps][16 * XS];  // per warp: GELU(z1)
+    __nv_bfloat16 D[kTrainWarps][16 * XS];  // per warp: dZ2, then dZ1
+    float sum[SPR];                         // the warps before the last one
 };
 
 __device__ __forceinline__ unsigned long long perm_index(unsigned long long i, unsigned long long n,
@@ -338,184 +346,286 @@ __device__ __forceinline__ unsigned long long perm_index(unsigned long long i, u
     return (a * i + c) % n;  // a coprime with n: a bijection of [0, n)
 }
 
-__global__ void __launch_bounds__(128) k_mlp_train(const float* __restrict__ feat,
-                                                   const float* __restrict__ label, long long n,
-                                                   long long start, int count, unsigned long long pa,
-                                                   unsigned long long pc, float pos_weight,
-                                                   float inv_batch, const float* __restrict__ w,
-                                                   float* __restrict__ grad, float* __restrict__ loss) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
+__global__ void __launch_bounds__(32 * kTrainWarps) k_mlp_train(
+    const float* __restrict__ feat, const float* __restrict__ label, long long n, long long start, int count,
+    unsigned long long pa, unsigned long long pc, float pos_weight, float inv_batch, const MlpSmem* __restrict__ net,
+    float* __restrict__ part) {
+    __shared__ __align__(16) TrainSmem S;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
-    mlp_load(S.m, w, true);
-    for (int e = tid; e < SP; e += blockDim.x) S.grad[e] = 0.f;
-    if (tid == 0) S.loss = 0.f;
-    // inputs of this warp's 32 samples (rows beyond count are zero with zero weight)
-    const int row0 = blockIdx.x * 128 + warp * 32;
-    __nv_bfloat16* X = S.X[warp];
-    float yv = 0.f, valid = 0.f;
-    {
-        int r = row0 + lane;
-        bool ok = r < count;
-        long long src = ok ? (long long)perm_index((unsigned long long)(start + r), (unsigned long long)n, pa, pc) : 0;
-        for (int e = 0; e < XS; e++) X[lane * XS + e] = __float2bfloat16(ok && e < SF ? feat[src * SF + e] : 0.f);
-        yv = ok ? label[src] : 0.f;
-        valid = ok ? 1.f : 0.f;
-    }
+    for (int e = tid; e < (int)(sizeof(MlpSmem) / 16); e += 32 * kTrainWarps)
+        reinterpret_cast<uint4*>(&S.m)[e] = reinterpret_cast<const uint4*>(net)[e];
+    __nv_bfloat16 *X = S.X[warp], *H = S.H[warp], *D = S.D[warp];
+    for (int e = lane; e < 16 * XS; e += 32) X[e] = __float2bfloat16(0.f);  // the columns past the features
     __syncthreads();
-    MlpFwd f;
-    mlp_forward(S.m, X, f);
-    // per-row dL/dz for rows (16mt+g) and (16mt+g+8): fetch label/valid from the owning lanes
-    float dz[2][2];
-#pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            int r = 16 * mt + g + 8 * h;
-            float y = __shfl_sync(0xffffffffu, yv, r);
-            float ok = __shfl_sync(0xffffffffu, valid, r);
-            float z = f.lg[mt][h];
-            float sg = 1.f / (1.f + __expf(-z));
-            // loss = pw y softplus(-z) + (1-y) softplus(z); dloss/dz = sg (pw y + 1 - y) - pw y
-            float sp_pos = fmaxf(-z, 0.f) + log1pf(__expf(-fabsf(z)));
-            float sp_neg = fmaxf(z, 0.f) + log1pf(__expf(-fabsf(z)));
-            float l = pos_weight * y * sp_pos + (1.f - y) * sp_neg;
-            dz[mt][h] = ok * inv_batch * (sg * (pos_weight * y + 1.f - y) - pos_weight * y);
-            if (q == 0 && ok > 0.f) atomicAdd(&S.loss, l * inv_batch);
+    // gradient sums of this lane: dW2 and dW1 as accumulator tiles, the columns
+    // 8 nt + 2 q + h of dw3, db2, db1 (to be summed over g), db3, the loss
+    float a2[2][4][4] = {}, a1[2][3][4] = {}, gw3[8] = {}, gb2[8] = {}, gb1[8] = {}, gb3 = 0.f, gl = 0.f;
+    for (int row0 = (blockIdx.x * kTrainWarps + warp) * 16; row0 < count; row0 += gridDim.x * kTrainWarps * 16) {
+        // inputs of 16 samples (rows beyond count are zero with zero weight)
+        const bool own = lane < 16 && row0 + lane < count;
+        const unsigned long long src =
+            own ? perm_index((unsigned long long)(start + row0 + lane), (unsigned long long)n, pa, pc) : 0;
+        const float yv = own ? label[src] : 0.f;
+        for (int e0 = 0; e0 < 16 * SF; e0 += 32) {  // whole warps, for the shuffle
+            const int e = e0 + lane, r = min(e / SF, 15), col = e - r * SF;
+            const unsigned long long sr = __shfl_sync(0xffffffffu, src, r);
+            if (e < 16 * SF) X[r * XS + col] = __float2bfloat16(row0 + r < count ? feat[sr * SF + col] : 0.f);
         }
-    // layer 3 and dZ2
-    float dz2[2][4][4];
-#pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                int col = 8 * nt + 2 * q + (e & 1);
-                float d = dz[mt][e >> 1];
-                float z2 = f.z2[mt][nt][e];
-                // dw3 += dz * h2, db2 += dz2
-                atomicAdd(&S.grad[OFF_W3 + col], d * gelu(z2));
-                dz2[mt][nt][e] = d * S.m.w3[col] * gelu_grad(z2);
-                atomicAdd(&S.grad[OFF_B2 + col], dz2[mt][nt][e]);
-            }
-    if (q == 0)
-#pragma unroll
-        for (int mt = 0; mt < 2; mt++) atomicAdd(&S.grad[OFF_B3], dz[mt][0] + dz[mt][1]);
-    // stage H1 = GELU(z1) and dZ2 as [sample][unit] bf16 tiles
-    __nv_bfloat16* H = S.H[warp];
-    __nv_bfloat16* D = S.D[warp];
-#pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                int r = 16 * mt + g + 8 * (e >> 1), col = 8 * nt + 2 * q + (e & 1);
-                H[r * XS + col] = __float2bfloat16(gelu(f.z1[mt][nt][e]));
-                D[r * XS + col] = __float2bfloat16(dz2[mt][nt][e]);
-            }
-    __syncwarp();
-    // dW2[out][in] += sum_s dZ2[s][out] H1[s][in]: M = out, N = in, K = samples
-#pragma unroll
-    for (int mo = 0; mo < 2; mo++)
-#pragma unroll
-        for (int ni = 0; ni < 4; ni++) {
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int ks = 0; ks < 2; ks++) {
-                uint32_t a[4], bb[2];
-                afrag_t(D, mo, ks, g, q, a);
-                bfrag_kn(H, ni, ks, g, q, bb);
-                mma16816(acc, a, bb);
-            }
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                int o = 16 * mo + g + 8 * (e >> 1), i = 8 * ni + 2 * q + (e & 1);
-                atomicAdd(&S.grad[OFF_W2 + o * 32 + i], acc[e]);
-            }
-        }
-    // dH1 = dZ2 W2 (M = samples, N = in, K = out): A = dZ2 from the accumulator layout
-    float dz1[2][4][4];
-#pragma unroll
-    for (int mt = 0; mt < 2; mt++) {
-        uint32_t a[2][4];
-#pragma unroll
-        for (int t = 0; t < 2; t++) {
-            a[t][0] = pack_bf16(dz2[mt][2 * t][0], dz2[mt][2 * t][1]);
-            a[t][1] = pack_bf16(dz2[mt][2 * t][2], dz2[mt][2 * t][3]);
-            a[t][2] = pack_bf16(dz2[mt][2 * t + 1][0], dz2[mt][2 * t + 1][1]);
-            a[t][3] = pack_bf16(dz2[mt][2 * t + 1][2], dz2[mt][2 * t + 1][3]);
-        }
+        __syncwarp();
+        // forward: z1, z2 in accumulator layout [nt][4]
+        uint32_t a[2][4], h1a[2][4];
+        float z1[4][4], z2[4][4], dz[2];
+        afrag(X, 0, 0, g, q, a[0]);
+        afrag(X, 0, 1, g, q, a[1]);
 #pragma unroll
         for (int nt = 0; nt < 4; nt++) {
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+            const float bl = S.m.b1[8 * nt + 2 * q], bh = S.m.b1[8 * nt + 2 * q + 1];
+            z1[nt][0] = bl; z1[nt][1] = bh; z1[nt][2] = bl; z1[nt][3] = bh;
 #pragma unroll
             for (int kt = 0; kt < 2; kt++) {
-                uint32_t bb[2];
-                bfrag(S.m.W2T, nt, kt, g, q, bb);  // B(k = out, n = in) = W2[out][in] = W2T[in][out]
-                mma16816(acc, a[kt], bb);
-            }
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                int col = 8 * nt + 2 * q + (e & 1);
-                dz1[mt][nt][e] = acc[e] * gelu_grad(f.z1[mt][nt][e]);
-                atomicAdd(&S.grad[OFF_B1 + col], dz1[mt][nt][e]);
+                uint32_t b[2];
+                bfrag(S.m.W1, nt, kt, g, q, b);
+                mma16816(z1[nt], a[kt], b);
             }
         }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int mt = 0; mt < 2; mt++)
+        // H = GELU(z1): layer 2's A fragments (accumulator tiles 2t, 2t+1 are k-tile t) and a [sample][unit] tile
 #pragma unroll
         for (int nt = 0; nt < 4; nt++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                int r = 16 * mt + g + 8 * (e >> 1), col = 8 * nt + 2 * q + (e & 1);
-                D[r * XS + col] = __float2bfloat16(dz1[mt][nt][e]);
+            for (int h = 0; h < 2; h++) {
+                const uint32_t v = pack_bf16(gelu(z1[nt][2 * h]), gelu(z1[nt][2 * h + 1]));
+                h1a[nt >> 1][2 * (nt & 1) + h] = v;
+                *reinterpret_cast<uint32_t*>(H + (g + 8 * h) * XS + 8 * nt + 2 * q) = v;
             }
-    __syncwarp();
-    // dW1[out][in] += sum_s dZ1[s][out] X[s][in]
+        float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-    for (int mo = 0; mo < 2; mo++)
+        for (int nt = 0; nt < 4; nt++) {
+            const float bl = S.m.b2[8 * nt + 2 * q], bh = S.m.b2[8 * nt + 2 * q + 1];
+            z2[nt][0] = bl; z2[nt][1] = bh; z2[nt][2] = bl; z2[nt][3] = bh;
 #pragma unroll
-        for (int ni = 0; ni < 3; ni++) {  // in-columns 0..23 cover the 21 features
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int ks = 0; ks < 2; ks++) {
-                uint32_t a[4], bb[2];
-                afrag_t(D, mo, ks, g, q, a);
-                bfrag_kn(X, ni, ks, g, q, bb);
-                mma16816(acc, a, bb);
+            for (int kt = 0; kt < 2; kt++) {
+                uint32_t b[2];
+                bfrag(S.m.W2, nt, kt, g, q, b);
+                mma16816(z2[nt], h1a[kt], b);
             }
+            const float wl = S.m.w3[8 * nt + 2 * q], wh = S.m.w3[8 * nt + 2 * q + 1];
+            s0 += gelu(z2[nt][0]) * wl + gelu(z2[nt][1]) * wh;
+            s1 += gelu(z2[nt][2]) * wl + gelu(z2[nt][3]) * wh;
+        }
+        s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+        s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
+        // per-row loss and dL/dz of rows g and g + 8: label from the owning lane
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                int o = 16 * mo + g + 8 * (e >> 1), i = 8 * ni + 2 * q + (e & 1);
-                if (i < SF) atomicAdd(&S.grad[OFF_W1 + o * 32 + i], acc[e]);
+        for (int h = 0; h < 2; h++) {
+            const float z = (h ? s1 : s0) + S.m.b3;
+            const float y = __shfl_sync(0xffffffffu, yv, g + 8 * h);
+            const float ok = row0 + g + 8 * h < count ? 1.f : 0.f;
+            const float sg = 1.f / (1.f + __expf(-z));
+            // loss = pw y softplus(-z) + (1-y) softplus(z); dloss/dz = sg (pw y + 1 - y) - pw y
+            const float sp_pos = fmaxf(-z, 0.f) + log1pf(__expf(-fabsf(z)));
+            const float sp_neg = fmaxf(z, 0.f) + log1pf(__expf(-fabsf(z)));
+            dz[h] = ok * inv_batch * (sg * (pos_weight * y + 1.f - y) - pos_weight * y);
+            if (q == 0) {
+                gl += ok * inv_batch * (pos_weight * y * sp_pos + (1.f - y) * sp_neg);
+                gb3 += dz[h];
             }
         }
-    __syncthreads();
-    for (int e = tid; e < SP; e += blockDim.x)
-        if (S.grad[e] != 0.f) atomicAdd(&grad[e], S.grad[e]);
-    if (tid == 0) atomicAdd(loss, S.loss);
-}
-
-// Adam (Kingma & Ba 2015) on the FP32 master weights; clears the gradient
-__global__ void k_adam(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
-                       float* __restrict__ grad, float lr, float b1, float b2, float eps, float c1,
-                       float c2) {
-    for (int e = threadIdx.x + blockIdx.x * blockDim.x; e < SP; e += blockDim.x * gridDim.x) {
-        float gr = grad[e];
-        grad[e] = 0.f;
-        bool unused = (e < OFF_B1) && ((e % 32) >= SF);  // padded input columns of W1 stay zero
-        if (unused) continue;
-        float mm = b1 * m[e] + (1.f - b1) * gr;
-        float vv = b2 * v[e] + (1.f - b2) * gr * gr;
-        m[e] = mm;
-        v[e] = vv;
-        w[e] -= lr * (mm * c1) / (sqrtf(vv * c2) + eps);
+        // layer 3 and dZ2, as layer 2's A fragments and a [sample][unit] tile
+        uint32_t d2a[2][4];
+#pragma unroll
+        for (int nt = 0; nt < 4; nt++) {
+            float d[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int col = 8 * nt + 2 * q + (e & 1);
+                const float v = dz[e >> 1];
+                gw3[2 * nt + (e & 1)] += v * gelu(z2[nt][e]);
+                d[e] = v * S.m.w3[col] * gelu_grad(z2[nt][e]);
+                gb2[2 * nt + (e & 1)] += d[e];
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t v = pack_bf16(d[2 * h], d[2 * h + 1]);
+                d2a[nt >> 1][2 * (nt & 1) + h] = v;
+                *reinterpret_cast<uint32_t*>(D + (g + 8 * h) * XS + 8 * nt + 2 * q) = v;
+            }
+        }
+        __syncwarp();
+        // dW2[out][in] += sum_s dZ2[s][out] H[s][in]: M = out, N = in, K = the 16 samples
+#pragma unroll
+        for (int mo = 0; mo < 2; mo++) {
+            uint32_t at[4];
+            afrag_t(D, mo, 0, g, q, at);
+#pragma unroll
+            for (int ni = 0; ni < 4; ni++) {
+                uint32_t b[2];
+                bfrag_kn(H, ni, 0, g, q, b);
+                mma16816(a2[mo][ni], at, b);
+            }
+        }
+        __syncwarp();
+        // dZ1 = (dZ2 W2) GELU'(z1) (M = samples, N = in, K = out)
+#pragma unroll
+        for (int nt = 0; nt < 4; nt++) {
+            float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int kt = 0; kt < 2; kt++) {
+                uint32_t b[2];
+                bfrag(S.m.W2T, nt, kt, g, q, b);  // B(k = out, n = in) = W2[out][in] = W2T[in][out]
+                mma16816(d, d2a[kt], b);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                d[e] *= gelu_grad(z1[nt][e]);
+                gb1[2 * nt + (e & 1)] += d[e];
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                *reinterpret_cast<uint32_t*>(D + (g + 8 * h) * XS + 8 * nt + 2 * q) = pack_bf16(d[2 * h], d[2 * h + 1]);
+        }
+        __syncwarp();
+        // dW1[out][in] += sum_s dZ1[s][out] X[s][in]; in-columns 0..23 cover the 21 features
+#pragma unroll
+        for (int mo = 0; mo < 2; mo++) {
+            uint32_t at[4];
+            afrag_t(D, mo, 0, g, q, at);
+#pragma unroll
+            for (int ni = 0; ni < 3; ni++) {
+                uint32_t b[2];
+                bfrag_kn(X, ni, 0, g, q, b);
+                mma16816(a1[mo][ni], at, b);
+            }
+        }
+        __syncwarp();
+    }
+    // sums over the rows a lane's columns came from
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            gw3[e] += __shfl_xor_sync(0xffffffffu, gw3[e], o);
+            gb2[e] += __shfl_xor_sync(0xffffffffu, gb2[e], o);
+            gb1[e] += __shfl_xor_sync(0xffffffffu, gb1[e], o);
+        }
+        gb3 += __shfl_xor_sync(0xffffffffu, gb3, o);
+        gl += __shfl_xor_sync(0xffffffffu, gl, o);
+    }
+    // the warps' sums in order, the last one writes the block's row
+    float* row = part + (size_t)blockIdx.x * SPR;
+    for (int w = 0; w < kTrainWarps; w++) {
+        if (warp == w) {
+            auto put = [&](int e, float v) {
+                if (w > 0) v += S.sum[e];
+                if (w + 1 < kTrainWarps) S.sum[e] = v;
+                else row[e] = v;
+            };
+#pragma unroll
+            for (int mo = 0; mo < 2; mo++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int o = 16 * mo + g + 8 * (e >> 1);
+#pragma unroll
+                    for (int ni = 0; ni < 4; ni++) put(OFF_W2 + o * 32 + 8 * ni + 2 * q + (e & 1), a2[mo][ni][e]);
+#pragma unroll
+                    for (int ni = 0; ni < 3; ni++) {
+                        const int i = 8 * ni + 2 * q + (e & 1);
+                        if (i < SF) put(OFF_W1 + o * 32 + i, a1[mo][ni][e]);
+                    }
+                }
+            if (g == 0) {
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    const int col = 8 * (e >> 1) + 2 * q + (e & 1);
+                    put(OFF_W3 + col, gw3[e]);
+                    put(OFF_B2 + col, gb2[e]);
+                    put(OFF_B1 + col, gb1[e]);
+                }
+                if (q == 0) {
+                    put(OFF_B3, gb3);
+                    put(SP, gl);
+                }
+            }
+        }
+        __syncthreads();
     }
 }
+
+// whether parameter e is one of W1's padded input columns, which stay zero
+__device__ __forceinline__ bool padded(int e) { return e < OFF_B1 && (e % 32) >= SF; }
+
+// parameter e of the network in the form that the kernels copy to shared memory
+__device__ __forceinline__ void net_put(MlpSmem* __restrict__ net, int e, float v) {
+    const int r = (e % 1056) / 32, col = e % 32;  // of W1 and, 1056 further, W2
+    if (e < OFF_B1) {
+        net->W1[r * XS + col] = __float2bfloat16(v);
+    } else if (e < OFF_W2) {
+        net->b1[e - OFF_B1] = v;
+    } else if (e < OFF_B2) {
+        net->W2[r * XS + col] = __float2bfloat16(v);
+        net->W2T[col * XS + r] = __float2bfloat16(v);
+    } else if (e < OFF_W3) {
+        net->b2[e - OFF_B2] = v;
+    } else if (e < OFF_B3) {
+        net->w3[e - OFF_W3] = v;
+    } else {
+        net->b3 = v;
+    }
+}
+
+__global__ void k_net_pack(const float* __restrict__ w, MlpSmem* __restrict__ net) {
+    for (int e = threadIdx.x; e < (int)(sizeof(MlpSmem) / 4); e += blockDim.x) reinterpret_cast<float*>(net)[e] = 0.f;
+    __syncthreads();
+    for (int e = threadIdx.x; e < SP; e += blockDim.x) net_put(net, e, padded(e) ? 0.f : w[e]);
+}
+
+// Sums the rows of partial gradients of 32 parameters a block (8 threads each, in a
+// fixed order), then takes the Adam step (Kingma & Ba 2015) on the FP32 master weights
+// and updates the network's packed form; parameter SP is the loss, added to *loss.
+// grad (nullable): the gradient goes there instead of into a step.
+__global__ void __launch_bounds__(256) k_adam(const float* __restrict__ part, int rows, float* __restrict__ w,
+                                              float* __restrict__ m, float* __restrict__ v,
+                                              MlpSmem* __restrict__ net, float* __restrict__ loss,
+                                              float* __restrict__ grad, float lr, float b1, float b2, float eps,
+                                              float c1, float c2) {
+    __shared__ float sum[8][32];
+    const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
+    const bool live = e <= SP && !padded(e);
+    float s = 0.f;
+    if (live)
+        for (int r = grp; r < rows; r += 8) s += part[(size_t)r * SPR + e];
+    sum[grp][lane] = s;
+    __syncthreads();
+    if (grp != 0 || !live) return;
+#pragma unroll
+    for (int r = 1; r < 8; r++) s += sum[r][lane];
+    if (e == SP) {
+        *loss += s;
+    } else if (grad) {
+        grad[e] = s;
+    } else {
+        const float mm = b1 * m[e] + (1.f - b1) * s;
+        const float vv = b2 * v[e] + (1.f - b2) * s * s;
+        const float we = w[e] - lr * (mm * c1) / (sqrtf(vv * c2) + eps);
+        m[e] = mm;
+        v[e] = vv;
+        w[e] = we;
+        net_put(net, e, we);
+    }
+}
+
+// One mini-batch: `count` samples from `start` in the order (pa i + pc) mod n; the
+// gradient's partial sums into part.  Returns the rows written.
+static int train_batch(const float* feat, const float* label, long long n, long long start, int count,
+                       unsigned long long pa, unsigned long long pc, float pos_weight, const MlpSmem* net, float* part,
+                       cudaStream_t s) {
+    const int per = kTrainWarps * 16, rows = std::min((count + per - 1) / per, kTrainBlocks);
+    k_mlp_train<<<rows, 32 * kTrainWarps, 0, s>>>(feat, label, n, start, count, pa, pc, pos_weight, 1.f / count, net,
+                                                  part);
+    return rows;
+}
+constexpr int kAdamBlocks = (SP + 1 + 31) / 32;
 
 // logits of n samples (4 warps x 32 samples per block)
 __global__ void __launch_bounds__(128) k_mlp_predict(const float* __restrict__ feat, long long n,
@@ -1029,7 +1139,29 @@ unsigned long long splitmix(unsigned long long& s) {
     return z ^ (z >> 31);
 }
 
-size_t train_smem() { return sizeof(TrainSmem); }
+// a training call's device buffers, one allocation (six took 0.5 ms of a call)
+struct TrainBuffers {
+    void* base = nullptr;
+    float *w = nullptr, *m = nullptr, *v = nullptr, *loss = nullptr, *part = nullptr;
+    MlpSmem* net = nullptr;
+    bool alloc(int epochs) {
+        const size_t vec = (SP * sizeof(float) + 255) / 256 * 256, losses = ((size_t)epochs * sizeof(float) + 255) / 256 * 256,
+                     nets = (sizeof(MlpSmem) + 255) / 256 * 256;
+        if (cudaMalloc(&base, nets + 3 * vec + losses + (size_t)kTrainBlocks * SPR * sizeof(float)) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        char* p = (char*)base;
+        net = (MlpSmem*)p;
+        w = (float*)(p += nets);
+        m = (float*)(p += vec);
+        v = (float*)(p += vec);
+        loss = (float*)(p += vec);
+        part = (float*)(p += losses);
+        return true;
+    }
+    ~TrainBuffers() { cudaFree(base); }
+};
 
 }  // namespace
 
@@ -1054,27 +1186,21 @@ NS_API ns_status ns_sensor_gradients(const float* feat, const float* label, int 
                                      const float* w, float* grad, float* loss, void* stream) {
     if (!feat || !label || !w || !grad || n <= 0) return NS_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    float *dw = nullptr, *dg = nullptr, *dl = nullptr;
-    if (cudaMalloc(&dw, SP * sizeof(float)) != cudaSuccess || cudaMalloc(&dg, SP * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&dl, sizeof(float)) != cudaSuccess) {
-        cudaFree(dw); cudaFree(dg); cudaFree(dl);
-        cudaGetLastError();
-        return NS_ERR_OOM;
-    }
-    cudaMemcpyAsync(dw, w, SP * sizeof(float), cudaMemcpyHostToDevice, s);
-    cudaMemsetAsync(dg, 0, SP * sizeof(float), s);
-    cudaMemsetAsync(dl, 0, sizeof(float), s);
-    cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem());
+    TrainBuffers t;
+    if (!t.alloc(1)) return NS_ERR_OOM;
+    cudaMemcpyAsync(t.w, w, SP * sizeof(float), cudaMemcpyHostToDevice, s);
+    cudaMemsetAsync(t.m, 0, SP * sizeof(float), s);  // receives the gradient; the padded columns' is zero
+    cudaMemsetAsync(t.loss, 0, sizeof(float), s);
+    k_net_pack<<<1, 1024, 0, s>>>(t.w, t.net);
     // identity order: a = 1, c = 0
-    k_mlp_train<<<(n + 127) / 128, 128, train_smem(), s>>>(feat, label, n, 0, n, 1, 0, pos_weight,
-                                                          1.f / n, dw, dg, dl);
+    const int rows = train_batch(feat, label, n, 0, n, 1, 0, pos_weight, t.net, t.part, s);
+    k_adam<<<kAdamBlocks, 256, 0, s>>>(t.part, rows, t.w, t.m, t.v, t.net, t.loss, t.m, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
-        cudaMemcpyAsync(grad, dg, SP * sizeof(float), cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(loss, dl, sizeof(float), cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(grad, t.m, SP * sizeof(float), cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(loss, t.loss, sizeof(float), cudaMemcpyDeviceToHost, s);
         e = cudaStreamSynchronize(s);
     }
-    cudaFree(dw); cudaFree(dg); cudaFree(dl);
     return e == cudaSuccess ? NS_OK : NS_ERR_CUDA;
 }
 
@@ -1084,23 +1210,15 @@ NS_API ns_status ns_sensor_train(const float* feat, const float* label, long lon
     if (!feat || !label || !w || n <= 0 || epochs <= 0 || batch <= 0 || !(lr > 0.f))
         return NS_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    float *dw = nullptr, *dm = nullptr, *dv = nullptr, *dg = nullptr, *dl = nullptr;
-    bool ok = cudaMalloc(&dw, SP * sizeof(float)) == cudaSuccess && cudaMalloc(&dm, SP * sizeof(float)) == cudaSuccess &&
-              cudaMalloc(&dv, SP * sizeof(float)) == cudaSuccess && cudaMalloc(&dg, SP * sizeof(float)) == cudaSuccess &&
-              cudaMalloc(&dl, (size_t)epochs * sizeof(float)) == cudaSuccess;
-    if (!ok) {
-        cudaFree(dw); cudaFree(dm); cudaFree(dv); cudaFree(dg); cudaFree(dl);
-        cudaGetLastError();
-        return NS_ERR_OOM;
-    }
-    cudaMemcpyAsync(dw, w, SP * sizeof(float), cudaMemcpyHostToDevice, s);
-    cudaMemsetAsync(dm, 0, SP * sizeof(float), s);
-    cudaMemsetAsync(dv, 0, SP * sizeof(float), s);
-    cudaMemsetAsync(dg, 0, SP * sizeof(float), s);
-    cudaMemsetAsync(dl, 0, (size_t)epochs * sizeof(float), s);
-    cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem());
+    TrainBuffers t;
+    if (!t.alloc(epochs)) return NS_ERR_OOM;
+    cudaMemcpyAsync(t.w, w, SP * sizeof(float), cudaMemcpyHostToDevice, s);
+    cudaMemsetAsync(t.m, 0, SP * sizeof(float), s);
+    cudaMemsetAsync(t.v, 0, SP * sizeof(float), s);
+    cudaMemsetAsync(t.loss, 0, (size_t)epochs * sizeof(float), s);
+    k_net_pack<<<1, 1024, 0, s>>>(t.w, t.net);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    unsigned long long rs = seed, t = 0;
+    unsigned long long rs = seed, step = 0;
     const long long nb = (n + batch - 1) / batch;
     for (int ep = 0; ep < epochs; ep++) {
         // a fresh pseudo-random order of the samples each epoch: i -> (a i + c) mod n
@@ -1109,26 +1227,25 @@ NS_API ns_status ns_sensor_train(const float* feat, const float* label, long lon
         for (long long bi = 0; bi < nb; bi++) {
             long long start = bi * batch;
             int cnt = (int)((n - start) < batch ? (n - start) : batch);
-            k_mlp_train<<<(cnt + 127) / 128, 128, train_smem(), s>>>(
-                feat, label, n, start, cnt, pa, pc, pos_weight, 1.f / cnt, dw, dg, dl + ep);
-            t++;
-            float c1 = 1.f / (1.f - std::pow(b1, (float)t)), c2 = 1.f / (1.f - std::pow(b2, (float)t));
-            k_adam<<<3, 1024, 0, s>>>(dw, dm, dv, dg, lr, b1, b2, eps, c1, c2);
+            const int rows = train_batch(feat, label, n, start, cnt, pa, pc, pos_weight, t.net, t.part, s);
+            step++;
+            float c1 = 1.f / (1.f - std::pow(b1, (float)step)), c2 = 1.f / (1.f - std::pow(b2, (float)step));
+            k_adam<<<kAdamBlocks, 256, 0, s>>>(t.part, rows, t.w, t.m, t.v, t.net, t.loss + ep, nullptr, lr, b1, b2,
+                                               eps, c1, c2);
         }
     }
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
-        cudaMemcpyAsync(w, dw, SP * sizeof(float), cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(w, t.w, SP * sizeof(float), cudaMemcpyDeviceToHost, s);
         if (epoch_loss) {
             std::vector<float> h(epochs);
-            cudaMemcpyAsync(h.data(), dl, (size_t)epochs * sizeof(float), cudaMemcpyDeviceToHost, s);
+            cudaMemcpyAsync(h.data(), t.loss, (size_t)epochs * sizeof(float), cudaMemcpyDeviceToHost, s);
             e = cudaStreamSynchronize(s);
             for (int ep = 0; ep < epochs; ep++) epoch_loss[ep] = h[ep] / (float)nb;
         } else {
             e = cudaStreamSynchronize(s);
         }
     }
-    cudaFree(dw); cudaFree(dm); cudaFree(dv); cudaFree(dg); cudaFree(dl);
     return e == cudaSuccess ? NS_OK : NS_ERR_CUDA;
 }
 
