@@ -162,8 +162,8 @@ static Consts make_consts(const ns_params* p) {
     c.gamma = p->gamma;
     c.gm1 = p->gamma - 1.0;
     c.inv_gm1 = 1.0 / (p->gamma - 1.0);
-    c.sqrt_gamma = std::sqrt(p->gamma);
-    c.inv_sqrt_gamma = 1.0 / std::sqrt(p->gamma);
+    c.two_sqrt_gamma = 2.0 * std::sqrt(p->gamma);
+    c.half_inv_sqrt_gamma = 0.5 / std::sqrt(p->gamma);
     c.mu = p->mu;
     c.lamb = (-2. / 3.) * p->mu;
     c.heat = p->gamma / (p->Pr * (p->gamma - 1.0));
@@ -173,6 +173,9 @@ static Consts make_consts(const ns_params* p) {
     c.inv_dx = 1.0 / c.dx;
     c.inv_dy = 1.0 / c.dy;
     c.inv_dz = 1.0 / c.dz;
+    c.half_inv[0] = 0.5 * c.inv_dx;
+    c.half_inv[1] = 0.5 * c.inv_dy;
+    c.half_inv[2] = 0.5 * c.inv_dz;
     c.cfl = p->cfl;
     for (int a = 0; a < 3; a++) c.periodic[a] = (p->bc[a] == NS_BC_PERIODIC);
     c.ext_x = p->bc[0] == NS_BC_EXTERNAL;

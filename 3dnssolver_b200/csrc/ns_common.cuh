@@ -65,9 +65,10 @@ inline FaceBox make_facebox(int nx, int ny, int nz, int dir) {
 // Kernel-side constants derived from ns_params.
 struct Consts {
     double gamma, gm1, inv_gm1;
-    double sqrt_gamma, inv_sqrt_gamma;
+    double two_sqrt_gamma, half_inv_sqrt_gamma;
     double mu, lamb, heat;      // lamb = -2/3 mu, heat = gamma/(Pr(gamma-1))
     double dx, dy, dz, inv_dx, inv_dy, inv_dz;
+    double half_inv[3];         // half of inv_dx, inv_dy, inv_dz
     double cfl;
     int periodic[3];
     int dim;
@@ -227,33 +228,31 @@ __device__ __forceinline__ void weno_right_nd(T a, T b, T c, T d, T e, T& num, T
 }
 
 // x / d for a positive, normal d (the WENO denominators: sums of products of
-// squared smoothness indicators, each at least the epsilon): the reciprocal by
-// two Newton-Raphson iterations y <- y + y (1 - d y) from the hardware estimate
-// (PTX rcp.approx.ftz.f64), then the quotient with one Markstein correction
-// (P. Markstein, IA-64 and Elementary Functions, 2000): q = x y, r = x - d q,
-// q + r y.  Within an ulp of the rounded quotient.
+// squared smoothness indicators, each at least the epsilon): the reciprocal from the
+// hardware estimate y (PTX rcp.approx.ftz.f64, about 20 bits) by one step of third order,
+// y (1 + e + e^2) with e = 1 - d y (the geometric series of 1/(1 - e); Householder,
+// The Numerical Treatment of a Single Nonlinear Equation, 1970), then the quotient with
+// one Markstein correction (P. Markstein, IA-64 and Elementary Functions, 2000): q = x y,
+// r = x - d q, q + r y.  Within an ulp of the rounded quotient.
 __device__ __forceinline__ double div_pos_nr(double x, double d) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    double e = fma(-d, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-d, y, 1.0);
-    y = fma(y, e, y);
+    const double e = fma(-d, y, 1.0);
+    y = fma(y, fma(e, e, e), y);
     const double q = x * y;
     const double r = fma(-d, q, x);
     return fma(r, y, q);
 }
 
-// 1 / sqrt(x) for a positive, normal x: two Newton-Raphson iterations
-// y <- y + (y / 2)(1 - x y^2) from the hardware estimate (PTX
-// rsqrt.approx.ftz.f64).  Within an ulp or two of the rounded value.
+// 1 / sqrt(x) for a positive, normal x, from the hardware estimate y (PTX
+// rsqrt.approx.ftz.f64) by one step of third order: y (1 + e/2 + 3 e^2/8) with
+// e = 1 - x y^2 (the binomial series of 1/sqrt(1 - e)).  Within an ulp or two of the
+// rounded value.
 __device__ __forceinline__ double rsqrt_pos_nr(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double e = fma(-x * y, y, 1.0);
-    y = fma(0.5 * y, e, y);
-    e = fma(-x * y, y, 1.0);
-    return fma(0.5 * y, e, y);
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 // f = WENO5_left(l) + WENO5_right(r), two fast reciprocals

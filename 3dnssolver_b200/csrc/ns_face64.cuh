@@ -8,7 +8,7 @@
 // (Weno5cw::compute_num_flux, src/convection_schemes/weno-5cw.cpp:4-28).
 //
 // The face kernels are bound by the FP64 pipe, so the flux is arranged for few
-// FP64 operations (about 660 characteristic-wise where the formulas taken
+// FP64 operations (about 645 characteristic-wise where the formulas taken
 // literally need about 1000).  All of it is exact algebra; results differ from
 // the literal form by rounding only:
 //   - A WENO-5 value is its centre cell plus a combination of the stencil's four
@@ -24,15 +24,17 @@
 //     density - K/c^2 h).  The acoustic fields are taken 2c times as large (WENO is
 //     homogeneous when its epsilon is scaled with them), the tangential ones up to
 //     their sign.
-//   - Everything is formed for the doubled flux F +- alpha U; the 1/2 and the
-//     candidates' 1/6 are applied once, at the end.
+//   - Everything is formed for the doubled flux F +- alpha U; the candidates' 1/6 is
+//     applied once, at the end, and the 1/2 left to the flux differences' 1/dx.
 //
 // Measured on B200 against the literal form (6 U/F/2 and ten projected columns a
-// face, weights on the stencil values), ms per step of 3 stages: Taylor-Green 384^3
-// physical characteristic-wise y/z faces 12.40/12.54 -> 9.53/9.56, x-march 15.18 ->
-// 12.76; shear layer 256^3 reference characteristic-wise 3.10/3.04 -> 2.33/2.18, x-march
-// 4.34 -> 3.71; Sod 512x128x128 component-wise 1.23/1.22 -> 0.95/0.92.  The error of the
-// right-hand side against 80-bit arithmetic falls too, 1.1 to 25 times
+// face, weights on the stencil values) in the kernels of the time, ms per step of 3
+// stages: Taylor-Green 384^3 physical characteristic-wise y/z faces 12.40/12.54 ->
+// 9.53/9.56, x-march 15.18 -> 12.76; shear layer 256^3 reference characteristic-wise
+// 3.10/3.04 -> 2.33/2.18, x-march 4.34 -> 3.71; Sod 512x128x128 component-wise 1.23/1.22
+// -> 0.95/0.92.  A further 25 operations (third-order reciprocals, factors left to the
+// caller) took the shear layer from 8.46 to 8.30 ms a step, faces 2.25/2.15 -> 2.18/2.09.
+// The error of the right-hand side against 80-bit arithmetic falls too, 1.1 to 25 times
 // over smooth, rough, Taylor-Green and shear states in every form.
 #pragma once
 
@@ -52,7 +54,7 @@ struct WenoEps {
 };
 
 // WENO-5 (weno-5.cpp:222-322) from the differences d0..d3 of the stencil
-// (d0 = b - a .. d3 = e - d): 6 (value - c) = d1 + 2 d2 + num/den.  The candidates
+// (d0 = b - a .. d3 = e - d): 6 (value - c) = d1 + 2 d2 + 2 num/den.  The candidates
 // are taken relative to the central one: 6 (f0 - f1) = 2 (D0 - D1), 6 (f2 - f1) =
 // D1 - D2 with the second differences D.  The nonlinear weights d_k / s_k^2 (Borges:
 // d_k (1 + tau/B_k)) are multiplied by the product of all denominators.
@@ -77,9 +79,8 @@ __device__ __forceinline__ void weno5_diff(double d0, double d1, double d2, doub
         y = p1 * p1;
         z = p2 * p2;
     }
-    z *= 3.0;
-    num = fma(2.0, x * (D0 - D1), z * (D1 - D2));
-    den = fma(6.0, y, x + z);
+    num = fma(1.5, z * (D1 - D2), x * (D0 - D1));
+    den = fma(3.0, z, fma(6.0, y, x));
 }
 
 // 6 (WENO5_left(l) + WENO5_right(r) - centre cells) from the left stencil's
@@ -90,7 +91,7 @@ __device__ __forceinline__ double weno5_pair_diff(const double l[4], const doubl
     weno5_diff<BORGES>(l[0], l[1], l[2], l[3], eps, nL, dL);
     weno5_diff<BORGES>(r[0], r[1], r[2], r[3], eps, nR, dR);
     const double lin = fma(2.0, l[2] + r[2], l[1] + r[1]);
-    return lin + div_pos_nr(fma(nL, dR, nR * dL), dL * dR);
+    return fma(2.0, div_pos_nr(fma(nL, dR, nR * dL), dL * dR), lin);
 }
 
 // U and the Euler flux along DIR of one cell (ConvectionFlux::form_flux,
@@ -115,7 +116,7 @@ __device__ __forceinline__ void cell_flux(const double w[5], double inv_gm1, dou
     for (int a = 0; a < 3; a++) f[2 + a] = a == DIR ? fma(m[a], qn, w[1]) : m[a] * qn;
 }
 
-// Numerical flux of one face.  ld(s, w) gives W of stencil cell s = 0..5; ldu(s, u)
+// Twice the numerical flux of one face.  ld(s, w) gives W of stencil cell s = 0..5; ldu(s, u)
 // gives U unless WONLY (a time step's stencils, where U = cons(W)); lam(s) gives the
 // cell's |q_n| + c (physical semantics).
 template <int DIR, bool CHAR, bool BORGES, bool PHYS, bool WONLY, typename LoadW, typename LoadU, typename Speed>
@@ -138,21 +139,23 @@ __device__ __forceinline__ void face_flux64(LoadW ld, LoadU ldu, Speed lam, cons
         ld(2, wa);
         ld(3, wb);
 #pragma unroll
-        for (int q = 0; q < 5; q++) wa[q] = 0.5 * (wa[q] + wb[q]);
+        for (int q = 0; q < 5; q++) wa[q] = wa[q] + wb[q];  // twice the average
 #pragma unroll
-        for (int a = 0; a < 3; a++) v[a] = wa[2 + a];
+        for (int a = 0; a < 3; a++) v[a] = 0.5 * wa[2 + a];
         hq2 = 0.5 * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
         double ic, cs;  // 1/c and c
         if constexpr (PHYS) {
+            // rho r and gamma p r with r = 1/sqrt(gamma p rho): the doubling cancels
             const double gp = c.gamma * wa[1];
             const double r = rsqrt_pos_nr(gp * wa[0]);
             ic = wa[0] * r;
             cs = gp * r;
         } else {
+            // sqrt(p rho / gamma) and sqrt(gamma / (p rho)), with p rho four times as large
             const double pr = wa[1] * wa[0];
             const double r = rsqrt_pos_nr(pr);
-            ic = c.inv_sqrt_gamma * (pr * r);
-            cs = c.sqrt_gamma * r;
+            ic = c.half_inv_sqrt_gamma * (pr * r);
+            cs = c.two_sqrt_gamma * r;
         }
         cs2 = cs * cs;
         kc = c.gm1 * ic;    // K/c
@@ -223,10 +226,10 @@ __device__ __forceinline__ void face_flux64(LoadW ld, LoadU ldu, Speed lam, cons
     double ft[5];
 #pragma unroll
     for (int q = 0; q < 5; q++) ft[q] = weno5_pair_diff<BORGES>(gl[q], gr[q], q < 2 ? epsc : eps);
-    constexpr double k12 = 1.0 / 12.0;
+    constexpr double k6 = 1.0 / 6.0;
     if constexpr (!CHAR) {
 #pragma unroll
-        for (int q = 0; q < 5; q++) out[q] = fma(k12, ft[q], 0.5 * cen[q]);
+        for (int q = 0; q < 5; q++) out[q] = fma(k6, ft[q], cen[q]);
     } else {
         // back-projection R ft (textbook rows of R, convection_flux.cpp:153-158)
         const double p = inv2c * (ft[0] + ft[1]), hd = 0.5 * (ft[1] - ft[0]);  // ft+ + ft-, c (ft+ - ft-)
@@ -239,11 +242,11 @@ __device__ __forceinline__ void face_flux64(LoadW ld, LoadU ldu, Speed lam, cons
         const double H = fma(cs2, c.inv_gm1, hq2);
         tb[4] = fma(H, p, fma(v[DIR], hd, fma(v[T1], ft[2], fma(v[T2], ft[3], hq2 * ft[4]))));
 #pragma unroll
-        for (int t = 0; t < 5; t++) out[st<PHYS>(t)] = fma(k12, tb[t], 0.5 * cen[st<PHYS>(t)]);
+        for (int t = 0; t < 5; t++) out[st<PHYS>(t)] = fma(k6, tb[t], cen[st<PHYS>(t)]);
     }
 }
 
-// The faces of a time step: U = cons(W), and at(q, s) gives plane q of stencil cell
+// The faces of a time step, twice the flux: U = cons(W), and at(q, s) gives plane q of stencil cell
 // s, W in planes 0..4 and (physical semantics) the sound speed in plane 6.
 template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename At>
 __device__ __forceinline__ void face_flux64_w(At at, const Consts& c, double out[5]) {
@@ -275,6 +278,8 @@ __device__ __forceinline__ void face_flux64_wu(const double* __restrict__ W, con
         return fabs(w[2 + DIR]) + sound_speed(w, c.gamma);
     };
     face_flux64<DIR, CHAR, BORGES, PHYS, false>(ld, ldu, lam, c, out);
+#pragma unroll
+    for (int q = 0; q < 5; q++) out[q] *= 0.5;
 }
 
 }  // namespace nsb

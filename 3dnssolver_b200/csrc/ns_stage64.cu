@@ -25,7 +25,7 @@ namespace nsb {
 
 constexpr int kFaceBlocks = 4;  // per SM
 
-// y-faces: a block takes 4 face rows x 32 columns, the columns (i, k) of the x-planes
+// y-faces (twice the flux): a block takes 4 face rows x 32 columns, the columns (i, k) of the x-planes
 // numbered through.
 template <bool CHAR, bool BORGES, bool PHYS>
 __global__ void __launch_bounds__(128, kFaceBlocks)
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(128, kFaceBlocks)
     for (int q = 0; q < 5; q++) o[q * fb.fstride] = f[q];
 }
 
-// z-faces: one thread per face of the rows' nz + 1 faces, numbered through
+// z-faces (twice the flux): one thread per face of the rows' nz + 1 faces, numbered through
 template <bool CHAR, bool BORGES, bool PHYS>
 __global__ void __launch_bounds__(128, kFaceBlocks)
     k_faces_z(const double* __restrict__ W, Box b, Consts c, double* __restrict__ F, FaceBox fb, int x0,
@@ -159,10 +159,11 @@ __global__ void __launch_bounds__(128, kXMarchBlocks)
 #pragma unroll
         for (int q = 0; q < 5; q++) {
             // the residual in k_update's order: x, y, z differences, then the viscous terms
-            double r = (f[q] - fprev[q * 128]) * c.inv_dx;
+            // (the faces hold twice the flux)
+            double r = (f[q] - fprev[q * 128]) * c.half_inv[0];
             fprev[q * 128] = f[q];
-            r += (py[q * fy.fstride + b.nz] - py[q * fy.fstride]) * c.inv_dy;
-            if (Fz) r += (pz[q * fz.fstride + 1] - pz[q * fz.fstride]) * c.inv_dz;
+            r += (py[q * fy.fstride + b.nz] - py[q * fy.fstride]) * c.half_inv[1];
+            if (Fz) r += (pz[q * fz.fstride + 1] - pz[q * fz.fstride]) * c.half_inv[2];
             if (q && V) r += pv[(q - 1) * vs];
             const double u0 = opnd[q * 128], u = first ? u0 : opnd[(5 + q) * 128];
             un[q] = (u0 * m1) + (u * m2) + (r * m3);
