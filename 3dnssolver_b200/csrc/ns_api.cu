@@ -427,9 +427,10 @@ static const double kRkMc[3] = {-1.0, -(1. / 4.), -(2. / 3.)};
 
 // FP64 stage st after its fill, on the x-planes pl: the y- and z-faces (with
 // with_faces), the viscous terms, then the x-faces marched together with the cell
-// update from Uin into Uout (and the next stage's W into W2)
+// update from Uin into Uout (and the next stage's W into W2, with images its ghost
+// cells too)
 static ns_status xstage(ns_ctx* ctx, int st, double* Uin, double* Uout, unsigned long long* cur,
-                        unsigned long long* nxt, bool with_faces, Planes pl) {
+                        unsigned long long* nxt, bool with_faces, bool images, Planes pl) {
     cudaStream_t s = ctx->stream;
     if (with_faces) NS_TRY(step_faces(ctx, pl));
     const bool visc = ctx->p.diffusion == NS_DIFF_CENTERED;
@@ -459,11 +460,21 @@ static ns_status xstage(ns_ctx* ctx, int st, double* Uin, double* Uout, unsigned
     a.m2 = kRkM2[st];
     a.mc = kRkMc[st];
     a.clock = (st == 0) ? ctx->clock : nullptr;
+    a.slot_reset = nxt;
+    a.images = images;
     a.sms = ctx->sms;
     launch_xmarch(ctx->p.convection == NS_CONV_WENO5_CHAR, ctx->p.weights == NS_WEIGHTS_BORGES, phys(ctx), a, s, pl);
     NS_TRY(check_launch(ctx, 1));
     prof_mark(ctx, NS_PROF_XFACE_UPDATE);
     return NS_OK;
+}
+
+// Whether the x-march writes the ghost cells of the next stage's W itself.  That takes a
+// launch less per stage, and costs the warps at the boundary more than k_fill_w does:
+// ms per step with / without on B200: 96x64 0.124 / 0.138, 64^3 0.221 / 0.241, 101x75x130
+// 0.969 / 0.981, Sod 512x128x128 3.82 / 3.79, shear layer 256^3 8.39 / 8.30.
+static bool march_images(const ns_ctx* ctx) {
+    return !slab(ctx) && (long long)ctx->p.nx * ctx->p.ny * ctx->p.nz <= (1 << 20);
 }
 
 // the state after an FP64 step of do_step: U holds it, U0 and the other parity
@@ -512,9 +523,8 @@ static ns_status do_step(ns_ctx* ctx) {
     }
     // FP64 with convection: per stage the fill, the y- and z-faces, the viscous terms,
     // then the x-faces marched together with the cell update into the other buffer:
-    // U0 -> U -> U2 -> U (stage 1 reads the step's start U0 directly).  The
-    // fill copies the stage input's halos into the output buffer, so the step
-    // ends with the halos the reference's U holds.  The third stage also forms
+    // U0 -> U -> U2 -> U (stage 1 reads the step's start U0 directly).  U's ghost
+    // cells are filled when a state is read back (finalize_w).  The third stage also forms
     // the next step's start (U0, and the CFL minimum in the other parity slot),
     // so only the first step after a state change runs k_step_begin.
     unsigned long long* nxt = ctx->slot + (ctx->parity ^ 1);
@@ -524,23 +534,23 @@ static ns_status do_step(ns_ctx* ctx) {
         NS_TRY(check_launch(ctx, 1));
         prof_mark(ctx, NS_PROF_STEP_BEGIN);
     }
-    NS_CUDA(cudaMemsetAsync(nxt, 0xFF, sizeof(unsigned long long), s));
     double* in[3] = {ctx->U0, ctx->U, ctx->U2};
     double* out[3] = {ctx->U, ctx->U2, ctx->U};
-    // W's interior for a stage is the previous x-update's output (W and W2 swap
-    // each stage); the fill then covers the halos only.  A first stage without
-    // that output (after a state change or a download of W) fills all cells.
-    const bool w_ready = ctx->fused_ready && ctx->w_next_ready;
+    // W for a stage, its ghost cells included, is the previous x-march's output (W and
+    // W2 swap each stage), or its ghost cells are filled (on a slab after the exchange).  A
+    // first stage without that output (after a state change or a download of W) fills all
+    // cells.
+    const bool w_ready = ctx->fused_ready && ctx->w_next_ready, img = march_images(ctx);
     NS_TRY(exchange(ctx, NS_EXCHANGE_DT, nullptr, cur));
     for (int st = 0; st < 3; st++) {
         NS_TRY(exchange(ctx, NS_EXCHANGE_HALO, in[st], nullptr));
-        if (st == 0 && !w_ready)
-            launch_fill_w(phys(ctx), ctx->W, in[st], ctx->box, ctx->c, s);
-        else
-            launch_fill_shell(phys(ctx), ctx->W, in[st], ctx->box, ctx->c, s);
-        NS_TRY(check_launch(ctx, 1));
-        prof_mark(ctx, NS_PROF_FILL);
-        NS_TRY(xstage(ctx, st, in[st], out[st], cur, nxt, true, Planes()));
+        if ((st == 0 && !w_ready) || !img) {
+            if (st == 0 && !w_ready) launch_fill_w(phys(ctx), ctx->W, in[st], ctx->box, ctx->c, s);
+            else launch_fill_shell(phys(ctx), ctx->W, in[st], ctx->box, ctx->c, s);
+            NS_TRY(check_launch(ctx, 1));
+            prof_mark(ctx, NS_PROF_FILL);
+        }
+        NS_TRY(xstage(ctx, st, in[st], out[st], cur, nxt, true, img, Planes()));
         std::swap(ctx->W, ctx->W2);
     }
     end_xstep(ctx);
@@ -954,7 +964,6 @@ static ns_status time_step_pipelined_run(ns_ctx* ctx, const double* Wh, double* 
     unsigned long long* cur = ctx->slot + ctx->parity;
     unsigned long long* nxt = ctx->slot + (ctx->parity ^ 1);
     NS_CUDA(cudaMemsetAsync(cur, 0xFF, sizeof(unsigned long long), s));
-    NS_CUDA(cudaMemsetAsync(nxt, 0xFF, sizeof(unsigned long long), s));
 
     // stage 1 (U0 -> U): per chunk as it lands
     for (int c = 0; c < K; c++) {
@@ -970,13 +979,13 @@ static ns_status time_step_pipelined_run(ns_ctx* ctx, const double* Wh, double* 
     launch_fill_w(phys(ctx), ctx->W, ctx->U0, ctx->box, ctx->c, s, ghost_lo);
     launch_fill_w(phys(ctx), ctx->W, ctx->U0, ctx->box, ctx->c, s, ghost_hi);
     NS_TRY(check_launch(ctx, 2));
-    NS_TRY(xstage(ctx, 0, ctx->U0, ctx->U, cur, nxt, false, Planes()));
+    NS_TRY(xstage(ctx, 0, ctx->U0, ctx->U, cur, nxt, false, false, Planes()));
     std::swap(ctx->W, ctx->W2);
 
     // stage 2 (U -> U2)
     launch_fill_shell(phys(ctx), ctx->W, ctx->U, ctx->box, ctx->c, s);
     NS_TRY(check_launch(ctx, 1));
-    NS_TRY(xstage(ctx, 1, ctx->U, ctx->U2, cur, nxt, true, Planes()));
+    NS_TRY(xstage(ctx, 1, ctx->U, ctx->U2, cur, nxt, true, false, Planes()));
     std::swap(ctx->W, ctx->W2);
 
     // stage 3 (U2 -> U) chunk by chunk into W2, which then holds prim(U) on every
@@ -987,7 +996,7 @@ static ns_status time_step_pipelined_run(ns_ctx* ctx, const double* Wh, double* 
     launch_prim_all(ctx->W2, ctx->U, ctx->box, ctx->c, s, ghost_hi);
     NS_TRY(check_launch(ctx, 4));
     for (int c = 0; c < K; c++) {
-        NS_TRY(xstage(ctx, 2, ctx->U2, ctx->U, cur, nxt, true, interior(c)));
+        NS_TRY(xstage(ctx, 2, ctx->U2, ctx->U, cur, nxt, true, false, interior(c)));
         const Planes sp = span(c);
         launch_prim_all(ctx->W2, ctx->U, ctx->box, ctx->c, s, halo_interior(c));
         launch_soa_to_aos(ctx->W2, ctx->stage, ctx->box, s, sp);

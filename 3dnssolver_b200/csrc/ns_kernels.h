@@ -48,6 +48,8 @@ struct XMarchArgs {
                                      // the next step's start), else null
     double m1, m2, mc;               // U = U0*m1 + U*m2 + R*(mc*dt)
     double* clock;                   // first stage: [last dt, accumulated time]
+    unsigned long long* slot_reset;  // first stage: the slot that the third stage reduces into
+    bool images;                     // Wnext's ghost cells too (not on a slab)
     int sms;                         // multiprocessors of the device
 };
 

@@ -87,6 +87,9 @@ __global__ void __launch_bounds__(128, kFaceBlocks)
 // 3.33 / 1.58; planes through TMA on mbarriers with a block barrier per cell 12.27 /
 // 3.51 / 1.69; the faces' operands staged too 13.2 / 3.65 / 1.75; U not staged 12.27 /
 // 3.54 / 1.64, nor U0 15.3 / 4.53 / 2.18; four blocks of 128 registers 15.7 / 3.61 / 1.60.
+//
+// IMAGES: each cell's W also goes to the ghost cells that fold onto it, over edges and
+// corners too, so that the next stage needs no launch of its own for them.
 constexpr int kXMarchBlocks = 3;  // per SM
 template <bool PHYS>
 struct XMarchLayout {
@@ -94,13 +97,28 @@ struct XMarchLayout {
     static constexpr size_t bytes = (size_t)(NS * NF + 5 + 10) * 128 * 8;
 };
 
-template <bool CHAR, bool BORGES, bool PHYS, bool LAST>
+// The ghost indices -3 .. -1 (bits 0..2) and n .. n+2 (bits 3..5) that fold onto index a
+// of an axis of n cells, and a itself (bit 6).
+__device__ __forceinline__ unsigned images(int a, int n, int periodic) {
+    unsigned m = 64;
+    if (periodic) {
+        for (int g = 0; g < 6; g++)
+            if (fold(g < 3 ? g - 3 : n + g - 3, n, 1) == a) m |= 1u << g;
+    } else {
+        if (a == 0) m |= 7;
+        if (a == n - 1) m |= 56;
+    }
+    return m;
+}
+__device__ __forceinline__ int image(int bit, int a, int n) { return bit == 6 ? a : (bit < 3 ? bit - 3 : n + bit - 3); }
+template <bool CHAR, bool BORGES, bool PHYS, bool LAST, bool IMAGES>
 __global__ void __launch_bounds__(128, kXMarchBlocks)
     k_xmarch(const double* __restrict__ W, const double* __restrict__ U, double* __restrict__ U0,
              double* __restrict__ Uout, double* __restrict__ Wn, const double* __restrict__ Fy,
              const double* __restrict__ Fz, const double* __restrict__ V, long long vs, Box b, FaceBox fy, FaceBox fz,
              Consts c, const unsigned long long* __restrict__ slot, unsigned long long* __restrict__ slot_next,
-             double m1, double m2, double mc, double* __restrict__ clock, int xlo, int xhi, int lx) {
+             double m1, double m2, double mc, double* __restrict__ clock, unsigned long long* __restrict__ slot_reset,
+             int xlo, int xhi, int lx) {
     constexpr int NF = XMarchLayout<PHYS>::NF, NS = XMarchLayout<PHYS>::NS;
     extern __shared__ double xsm[];
     const int t = threadIdx.y * 32 + threadIdx.x;
@@ -117,6 +135,13 @@ __global__ void __launch_bounds__(128, kXMarchBlocks)
     if (clock && (blockIdx.x | blockIdx.y | t) == 0) {
         clock[0] = dt;
         clock[1] += dt;
+        *slot_reset = ~0ull;  // for the third stage
+    }
+    // the column's images along y and z (in 2D no stencil runs along z)
+    unsigned mj = 64, mk = 64;
+    if constexpr (IMAGES) {
+        mj = images(j, b.ny, c.periodic[1]);
+        if (c.dim == 3) mk = images(k, b.nz, c.periodic[2]);
     }
     const bool first = U == U0;  // the first stage's input is the step's start
     auto load_plane = [&](int p) {  // plane p of W into slot (p - x0 + 3) % NS
@@ -180,6 +205,18 @@ __global__ void __launch_bounds__(128, kXMarchBlocks)
             prim_from_cons(u0, c.gm1, w);  // the next step's first stage reads prim(U0)
         }
         store_w<PHYS>(Wn, b.fstride, o, w, c.gamma);
+        if constexpr (IMAGES) {
+            const unsigned mi = i < NG || i >= b.nx - NG ? images(i, b.nx, c.periodic[0]) : 64;
+            if ((mi | mj | mk) == 64) continue;
+            for (unsigned x = mi; x; x &= x - 1)
+                for (unsigned y = mj; y; y &= y - 1) {
+                    const long long row = b.at(image(__ffs(x) - 1, i, b.nx) + NG, image(__ffs(y) - 1, j, b.ny) + NG, NG);
+                    for (unsigned z = mk; z; z &= z - 1) {
+                        const long long g = row + image(__ffs(z) - 1, k, b.nz);
+                        if (g != o) store_w<PHYS>(Wn, b.fstride, g, w, c.gamma);
+                    }
+                }
+        }
     }
     cp_async_wait_all();
     if constexpr (LAST) block_min_to(best, slot_next);
@@ -247,10 +284,10 @@ void launch_step_faces(int dir, bool chr, bool borges, bool phys, const double* 
     }
 }
 
-template <bool CHAR, bool BORGES, bool PHYS, bool LAST>
+template <bool CHAR, bool BORGES, bool PHYS, bool LAST, bool IMAGES>
 static void xmarch_one(const XMarchArgs& a, cudaStream_t s, Planes pl) {
     constexpr size_t bytes = XMarchLayout<PHYS>::bytes;
-    auto kern = k_xmarch<CHAR, BORGES, PHYS, LAST>;
+    auto kern = k_xmarch<CHAR, BORGES, PHYS, LAST, IMAGES>;
     // the attribute is per device; a refusal surfaces as the launch's error
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     const int x0 = pl.n < 0 ? 0 : pl.lo, np = pl.n < 0 ? a.b.nx : pl.n;
@@ -259,13 +296,18 @@ static void xmarch_one(const XMarchArgs& a, cudaStream_t s, Planes pl) {
     const int lx = march_length(np, blocks, a.sms * kXMarchBlocks, 2.0, 64);
     kern<<<dim3((unsigned)blocks, (np + lx - 1) / lx), dim3(32, 4), bytes, s>>>(
         a.W, a.U, a.U0, a.Uout, a.Wnext, a.Fy, a.Fz, a.V, a.vs, a.b, a.fy, a.fz, a.c, a.slot,
-        LAST ? a.slot_next : nullptr, a.m1, a.m2, a.mc, a.clock, x0, x0 + np, lx);
+        LAST ? a.slot_next : nullptr, a.m1, a.m2, a.mc, a.clock, a.slot_reset, x0, x0 + np, lx);
 }
 
 template <bool CHAR, bool BORGES, bool PHYS>
 static void xmarch_last(const XMarchArgs& a, cudaStream_t s, Planes pl) {
-    if (a.slot_next) xmarch_one<CHAR, BORGES, PHYS, true>(a, s, pl);
-    else xmarch_one<CHAR, BORGES, PHYS, false>(a, s, pl);
+    if (a.images) {
+        if (a.slot_next) xmarch_one<CHAR, BORGES, PHYS, true, true>(a, s, pl);
+        else xmarch_one<CHAR, BORGES, PHYS, false, true>(a, s, pl);
+    } else {
+        if (a.slot_next) xmarch_one<CHAR, BORGES, PHYS, true, false>(a, s, pl);
+        else xmarch_one<CHAR, BORGES, PHYS, false, false>(a, s, pl);
+    }
 }
 
 void launch_xmarch(bool chr, bool borges, bool phys, const XMarchArgs& a, cudaStream_t s, Planes pl) {

@@ -398,3 +398,26 @@ def test_viscous_stage_terms_match_oracle(oracle, shape, dim, order, sem, bc):
         sl = [slice(3, -3)] * 3
         sl[ax] = slice(0, 3)
         assert (rel_l2(Wg[tuple(sl)], Wo[tuple(sl)]) <= 10 * TOL).all()
+
+
+# Grids of up to 2^20 cells keep the ghost cells of a stage's W in the x-march, larger
+# ones fill them in a pass of their own: the same state bit for bit from both sides of
+# the line, boundaries of every kind, over several steps.  The larger grid is the
+# smaller one continued periodically along y, whose rows see the same neighbours.
+@pytest.mark.parametrize("bc,order,sem", [((N, P, P), 2, 1), ((P, P, N), 4, 1), ((N, P, N), 2, 0), ((P, P, P), 6, 0)])
+def test_ghost_cells_from_the_march_and_from_the_fill_agree(bc, order, sem):
+    kw = dict(convection=2, diffusion_order=order, bc=bc, mu=0.02, cfl=0.2, semantics=sem)
+    small = pkg.make_params(64, 128, 128, L=(1.0, 1.0, 1.0), **kw)
+    large = pkg.make_params(64, 256, 128, L=(1.0, 2.0, 1.0), **kw)
+    W0 = wl.random_field(small, seed=61, smooth=True)
+    W1 = wl.random_field(large, seed=61, smooth=True)
+    interior(W1)[:, :128] = interior(W0)
+    interior(W1)[:, 128:] = interior(W0)
+    with pkg.Solver(small) as a, pkg.Solver(large) as b:
+        a.upload_primitive(W0)
+        b.upload_primitive(W1)
+        a.advance(3)
+        b.advance(3)
+        Ua, Ub = interior(a.download_conservative()), interior(b.download_conservative())
+    # (the last case's state turns non-finite in the oracle's second step too)
+    assert np.array_equal(Ua, Ub[:, :128], equal_nan=True) and np.array_equal(Ua, Ub[:, 128:], equal_nan=True)
