@@ -366,6 +366,7 @@ static ns_status do_step_fused(ns_ctx* ctx) {
     a.U0 = ctx->U0;
     a.slot = cur;
     a.slot_next = nxt;
+    a.sms = ctx->sms;
     const bool gated = p.sensor && a.conv_dims > 0;
     GateLists gl;
     if (gated) {

@@ -40,7 +40,7 @@
 namespace nsb {
 
 // ---------------------------------------------------------------------------
-// A block marches LX cells along x over a TY x TZ column: 2.2 plane loads per
+// A block marches lx cells along x over a TY x TZ column: 2.2 plane loads per
 // cell (a 3D box tile with the same shared memory needed 7.4 and ran 20%
 // slower on B200), x-face fluxes carried in registers, y- and z-faces of the
 // current plane through small shared face buffers.
@@ -52,13 +52,6 @@ namespace nsb {
 #ifndef NS_MARCH_TY
 #define NS_MARCH_TY 8
 #endif
-// cells a block marches along x: 64 ran 2.2% faster than 32 for the
-// characteristic-wise stage on B200 at 256^3 and 0.5% slower for the
-// component-wise one
-template <bool CHAR>
-struct MarchLen {
-    static constexpr int value = CHAR ? 64 : 32;
-};
 //
 // Plane i reads planes i-2..i+3 (x-faces) and i-H..i+H (viscous terms).  With
 // H <= 1 ("lean") the ring holds 6 planes and the y/z face buffers alternate
@@ -261,7 +254,7 @@ __global__ void __launch_bounds__(MarchTile<T, H>::FT, MarchTile<T, H>::MINB)
     k_stage_march(const double* __restrict__ Uin, double* U0, double* __restrict__ Uout, Box b,
                   Consts c, int conv_dims, double m1, double m2, double mc,
                   const unsigned long long* __restrict__ slot, unsigned long long* slot_next,
-                  double* clock, const unsigned char* __restrict__ skip) {
+                  double* clock, const unsigned char* __restrict__ skip, int lx) {
     using M = MarchTile<T, H>;
     constexpr int FT = M::FT;
     static_assert(M::NFY <= 2 * FT && M::NFZ <= 2 * FT, "a face pass takes at most two rounds");
@@ -271,9 +264,8 @@ __global__ void __launch_bounds__(MarchTile<T, H>::FT, MarchTile<T, H>::MINB)
     T* FZb = FYb + M::NBUF * 5 * M::NFY;         // [NBUF][5][NFZ]
     double* S = reinterpret_cast<double*>(FZb + M::NBUF * 5 * M::NFZ);  // [5][NP] U_in of the plane in flight
     const int tid = threadIdx.x, ty = tid / M::TZ, tz = tid % M::TZ;
-    constexpr int LX = MarchLen<CHAR>::value;
-    const int k0 = blockIdx.x * M::TZ, j0 = blockIdx.y * M::TY, x0 = blockIdx.z * LX;
-    const int x1 = min(x0 + LX, b.nx);
+    const int k0 = blockIdx.x * M::TZ, j0 = blockIdx.y * M::TY, x0 = blockIdx.z * lx;
+    const int x1 = min(x0 + lx, b.nx);
     auto plane = [&](int i) { return ring + ring_slot<M::RING>(i, x0) * 5 * M::NP; };
     // U_in of plane i at folded positions, into S without waiting (each thread
     // later converts exactly the elements it copied, so S needs no barrier)
@@ -427,6 +419,18 @@ __global__ void __launch_bounds__(MarchTile<T, H>::FT, MarchTile<T, H>::MINB)
     if constexpr (LAST) block_min_to(best, slot_next);
 }
 
+// What a march costs besides its cells (its first face and the first planes' latency)
+// and its longest length: 64 cells for the characteristic-wise stage, 32 for the
+// component-wise one where those fill the GPU once (shorter ones that would even out the
+// last wave cost 1-2%: the blocks of a thin wave run faster), shorter marches on
+// smaller grids (ms per step at the longest throughout -> now: Taylor-Green 64^3 1.56 ->
+// 0.21, 32^3 0.81 -> 0.15, 200x130x70 2.60 -> 1.81; sensor-gated Sod 256x64x64 0.78 -> 0.64).
+constexpr double kMarchExtra = 3.0;
+template <bool CHAR>
+struct MarchLongest {
+    static constexpr int value = CHAR ? 64 : 32;
+};
+
 template <typename T, bool CHAR, bool BORGES, int H, bool LAST, bool PHYS>
 static cudaError_t fused_one(const FusedArgs& a, cudaStream_t s) {
     using M = MarchTile<T, H>;
@@ -434,10 +438,15 @@ static cudaError_t fused_one(const FusedArgs& a, cudaStream_t s) {
     // the attribute is per device; setting it on every launch keeps multi-device use correct
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::smem);
     if (e != cudaSuccess) return e;
-    constexpr int LX = MarchLen<CHAR>::value;
-    dim3 grid((a.b.nz + M::TZ - 1) / M::TZ, (a.b.ny + M::TY - 1) / M::TY, (a.b.nx + LX - 1) / LX);
+    dim3 grid((a.b.nz + M::TZ - 1) / M::TZ, (a.b.ny + M::TY - 1) / M::TY);
+    constexpr int longest = MarchLongest<CHAR>::value;
+    const long long across = (long long)grid.x * grid.y;
+    const int resident = a.sms * M::MINB;
+    const int lx = across * ((a.b.nx + longest - 1) / longest) >= resident
+                       ? longest : march_length(a.b.nx, across, resident, kMarchExtra, longest);
+    grid.z = (a.b.nx + lx - 1) / lx;
     kern<<<grid, M::FT, M::smem, s>>>(a.Uin, a.U0, a.Uout, a.b, a.c, a.conv_dims, a.m1, a.m2, a.mc, a.slot,
-                                   a.slot_next, a.clock, a.skip);
+                                   a.slot_next, a.clock, a.skip, lx);
     return cudaGetLastError();
 }
 

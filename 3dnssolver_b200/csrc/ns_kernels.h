@@ -88,6 +88,7 @@ struct FusedArgs {
     const unsigned long long* slot;   // CFL minimum of this step
     unsigned long long* slot_next;    // last stage: CFL minimum of the next step
     double* clock;                    // first stage: [last dt, accumulated time]
+    int sms;                          // multiprocessors of the device
     const unsigned char* skip;        // last stage: cells (interior order) whose next-step start a
                                       // correction pass forms instead (nullable)
 };
