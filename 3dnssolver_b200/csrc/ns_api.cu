@@ -286,21 +286,17 @@ static const nsb::VTmaMap* visc_map(const ns_ctx* ctx) {
 static ns_status faces(ns_ctx* ctx) {
     const ns_params& p = ctx->p;
     if (p.convection == NS_CONV_NONE) return NS_OK;
-    int nd = p.dim == 3 ? 3 : 2;
-    for (int d = 0; d < nd; d++) {
-        if (p.sensor) {
-            if (sensor_face_flux(ctx->sensor, d, ctx->W, ctx->U, ctx->box, ctx->c, p.sensor_threshold,
-                                 p.weights == NS_WEIGHTS_BORGES, phys(ctx), ctx->F[d], ctx->fb[d], ctx->stream,
-                                 &ctx->launches) != NS_OK)
-                return fail(NS_ERR_CUDA, "gated face kernel launch failed: %s",
-                            cudaGetErrorString(cudaGetLastError()));
-        } else {
-            launch_face_flux(d, p.convection == NS_CONV_WENO5_CHAR, p.weights == NS_WEIGHTS_BORGES, phys(ctx),
-                             fp32(ctx), ctx->W, ctx->U, ctx->box, ctx->c, ctx->F[d], ctx->fb[d], ctx->stream);
-            NS_TRY(check_launch(ctx, d > 0 ? 2 : 1));  // y and z: the face grid and its last plane
-        }
-        prof_mark(ctx, NS_PROF_FACE_X + d);
+    const int nd = p.dim == 3 ? 3 : 2;
+    if (!p.sensor) {
+        const int n = launch_faces(p.convection == NS_CONV_WENO5_CHAR, p.weights == NS_WEIGHTS_BORGES, phys(ctx), fp32(ctx),
+                                   nd, ctx->W, ctx->U, ctx->box, ctx->c, ctx->F, ctx->fb, ctx->stream);
+        return check_launch(ctx, n);
     }
+    for (int d = 0; d < nd; d++)
+        if (sensor_face_flux(ctx->sensor, d, ctx->W, ctx->U, ctx->box, ctx->c, p.sensor_threshold,
+                             p.weights == NS_WEIGHTS_BORGES, phys(ctx), ctx->F[d], ctx->fb[d], ctx->stream,
+                             &ctx->launches) != NS_OK)
+            return fail(NS_ERR_CUDA, "gated face kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     return NS_OK;
 }
 
@@ -1424,7 +1420,7 @@ extern "C" ns_status ns_convection_solve_noalloc(const ns_params* p, const doubl
     const bool chr = p->convection == NS_CONV_WENO5_CHAR;
     const bool borges = p->weights == NS_WEIGHTS_BORGES;
     const bool ph = p->semantics == NS_SEM_PHYSICAL;
-    for (int d = 0; d < nd; d++) launch_face_flux(d, chr, borges, ph, f32, W, U, b, c, F[d], fb[d], s);
+    launch_faces(chr, borges, ph, f32, nd, W, U, b, c, F, fb, s);
     UpdateArgs a;
     memset(&a, 0, sizeof a);
     a.W = W;

@@ -3,8 +3,9 @@
 // Per RK stage (TimeScheme::step, src/time_scheme.cpp:33-66):
 //   k_fill_prim      boundary fill + halo exchange of U on the face halos, then
 //                    W = prim(U) on every cell (time_scheme.cpp:133-135)
-//   k_face_flux<d>   WENO-5 face fluxes along axis d, one thread per face
-//                    (Weno5::x/y/z_sweep, Weno5cw::*_sweep), for operator calls
+//   k_op_faces       WENO-5 face fluxes along every axis, one thread per face
+//                    (Weno5::x/y/z_sweep, Weno5cw::*_sweep), for operator calls;
+//                    k_face_flux<d> in FP32
 //   k_update         flux differences + centered viscous terms + RK combination
 //                    (Weno5::compute_residual, CenteredDiffusion::compute_residual,
 //                    TimeScheme::substep), for operator calls and steps without
@@ -232,76 +233,89 @@ __global__ void __launch_bounds__(128) k_fill_uhalo(double* __restrict__ U, cons
 // WENO-5 face fluxes (device functions in ns_face.cuh)
 
 // Minimum resident blocks per SM requested from the register allocator for the
-// face kernels (128 threads each), per form.  Chosen by a sweep on B200 at
-// 256^3 (1, 3, 4 for FP64; 1, 5, 6 for FP32 characteristic): the caps trade a
-// few spilled registers for 12-20 resident warps instead of 8.
-#ifndef NS_FACE_MINB_F64CHAR
-#define NS_FACE_MINB_F64CHAR 3
-#endif
-#ifndef NS_FACE_MINB_F64COMP
-#define NS_FACE_MINB_F64COMP 4
-#endif
-#ifndef NS_FACE_MINB_F32CHAR
-#define NS_FACE_MINB_F32CHAR 5
-#endif
-#ifndef NS_FACE_MINB_F32COMP
-#define NS_FACE_MINB_F32COMP 1
-#endif
-template <bool CHAR, typename T>
+// FP32 face kernels (128 threads each), chosen by a sweep on B200 at 256^3 (1, 5, 6
+// characteristic-wise): the cap trades a few spilled registers for 20 resident warps
+// instead of 8.
+template <bool CHAR>
 struct FaceMinBlocks {
-    static constexpr int value = sizeof(T) == 8 ? (CHAR ? NS_FACE_MINB_F64CHAR : NS_FACE_MINB_F64COMP)
-                                                : (CHAR ? NS_FACE_MINB_F32CHAR : NS_FACE_MINB_F32COMP);
+    static constexpr int value = CHAR ? 5 : 1;
 };
 
-// one face of an operator call, from the caller's W and U
-template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename T, typename TF>
+// Every face of an FP64 operator call from the caller's W and U, one thread per face,
+// the axes one after the other in one launch (blocks n0, n1, n2 of the axes).  The
+// grids of these calls are small and their launches latency: three axes with a launch
+// each and two more for the last planes of y and z took 61 us of a 48x60x52 residual.
+struct OpFaces {
+    double* F[3];
+    FaceBox fb[3];
+    unsigned blocks[3];
+};
+template <int DIR, bool CHAR, bool BORGES, bool PHYS>
+__device__ __forceinline__ void op_face(const double* __restrict__ W, const double* __restrict__ U, const Box& b,
+                                        const Consts& c, const OpFaces& o, unsigned block) {
+    const FaceBox& fb = o.fb[DIR];
+    const long long e = (long long)block * 128 + threadIdx.x;
+    if (e >= (long long)fb.n0 * fb.n1 * fb.n2) return;
+    const int kk = (int)(e % fb.n2), bb = (int)(e / fb.n2 % fb.n1), aa = (int)(e / fb.n2 / fb.n1);
+    long long step;
+    const long long o0 = face_origin<DIR>(b, aa, bb, kk, step);
+    double f[5];
+    face_flux64_wu<DIR, CHAR, BORGES, PHYS>(W, U, b, c, o0, step, f);
+#pragma unroll
+    for (int q = 0; q < 5; q++) o.F[DIR][q * fb.fstride + e] = f[q];
+}
+template <bool CHAR, bool BORGES, bool PHYS>
+__global__ void __launch_bounds__(128, 3)
+    k_op_faces(const double* __restrict__ W, const double* __restrict__ U, Box b, Consts c, OpFaces o) {
+    if (blockIdx.x < o.blocks[0]) op_face<0, CHAR, BORGES, PHYS>(W, U, b, c, o, blockIdx.x);
+    else if (blockIdx.x < o.blocks[0] + o.blocks[1]) op_face<1, CHAR, BORGES, PHYS>(W, U, b, c, o, blockIdx.x - o.blocks[0]);
+    else op_face<2, CHAR, BORGES, PHYS>(W, U, b, c, o, blockIdx.x - o.blocks[0] - o.blocks[1]);
+}
+
+// one face of an FP32 operator call
+template <int DIR, bool CHAR, bool BORGES, bool PHYS>
 __device__ __forceinline__ void face_at(const double* __restrict__ W, const double* __restrict__ U,
-                                        const Box& b, const Consts& c, TF* __restrict__ F,
+                                        const Box& b, const Consts& c, float* __restrict__ F,
                                         const FaceBox& fb, int aa, int bb, int kk) {
     long long step;
     long long o0 = face_origin<DIR>(b, aa, bb, kk, step);
-    T out[5];
-    if constexpr (sizeof(T) == 8) {
-        face_flux64_wu<DIR, CHAR, BORGES, PHYS>(W, U, b, c, o0, step, out);
-    } else {
-        T fL[5][5], fR[5][5], wa[5];
-        face_stencil<DIR, CHAR, PHYS, T>(W, U, b, c, o0, step, fL, fR, wa);
-        if constexpr (!CHAR)
-            face_comp<T, BORGES>(fL, fR, out);
-        else
-            face_char<DIR, PHYS, T, BORGES>(fL, fR, wa, T(c.gamma), T(c.inv_gm1), out);
-    }
+    float fL[5][5], fR[5][5], wa[5], out[5];
+    face_stencil<DIR, CHAR, PHYS, float>(W, U, b, c, o0, step, fL, fR, wa);
+    if constexpr (!CHAR)
+        face_comp<float, BORGES>(fL, fR, out);
+    else
+        face_char<DIR, PHYS, float, BORGES>(fL, fR, wa, float(c.gamma), float(c.inv_gm1), out);
     long long fo = fb.at(aa, bb, kk);
 #pragma unroll
-    for (int q = 0; q < 5; q++) F[q * fb.fstride + fo] = TF(out[q]);
+    for (int q = 0; q < 5; q++) F[q * fb.fstride + fo] = out[q];
 }
 
-// Faces of one (i, j) tile row of 32 k-faces per warp, 4 rows per block.  Along
+// FP32 faces of one (i, j) tile row of 32 k-faces per warp, 4 rows per block.  Along
 // y and z the last face plane (j = ny, k = nz) is left to k_face_flux_tail: as
 // a 33rd k-face or a 4th-of-4 row it would occupy a whole block for one live
 // lane or warp per block.
-template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename T, typename TF>
-__global__ void __launch_bounds__(128, FaceMinBlocks<CHAR, T>::value)
+template <int DIR, bool CHAR, bool BORGES, bool PHYS>
+__global__ void __launch_bounds__(128, FaceMinBlocks<CHAR>::value)
     k_face_flux(const double* __restrict__ W, const double* __restrict__ U, Box b, Consts c,
-                TF* __restrict__ F, FaceBox fb) {
+                float* __restrict__ F, FaceBox fb) {
     int kk = blockIdx.x * 32 + threadIdx.x;
     int bb = blockIdx.y * 4 + threadIdx.y;
     int aa = blockIdx.z;
     if (kk >= fb.n2 - (DIR == 2) || bb >= fb.n1 - (DIR == 1)) return;
-    face_at<DIR, CHAR, BORGES, PHYS, T, TF>(W, U, b, c, F, fb, aa, bb, kk);
+    face_at<DIR, CHAR, BORGES, PHYS>(W, U, b, c, F, fb, aa, bb, kk);
 }
 
 // The last face plane along y (j = ny, threads along k) or z (k = nz, threads
 // along j), one face per thread.
-template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename T, typename TF>
-__global__ void __launch_bounds__(128, FaceMinBlocks<CHAR, T>::value)
+template <int DIR, bool CHAR, bool BORGES, bool PHYS>
+__global__ void __launch_bounds__(128, FaceMinBlocks<CHAR>::value)
     k_face_flux_tail(const double* __restrict__ W, const double* __restrict__ U, Box b, Consts c,
-                     TF* __restrict__ F, FaceBox fb) {
+                     float* __restrict__ F, FaceBox fb) {
     static_assert(DIR > 0, "x-faces have no tail plane");
     const int r = blockIdx.x * 128 + threadIdx.x, aa = blockIdx.y;
     if (r >= (DIR == 1 ? fb.n2 : fb.n1)) return;
     const int bb = DIR == 1 ? fb.n1 - 1 : r, kk = DIR == 1 ? r : fb.n2 - 1;
-    face_at<DIR, CHAR, BORGES, PHYS, T, TF>(W, U, b, c, F, fb, aa, bb, kk);
+    face_at<DIR, CHAR, BORGES, PHYS>(W, U, b, c, F, fb, aa, bb, kk);
 }
 
 // ---------------------------------------------------------------------------
@@ -798,51 +812,50 @@ void launch_fill_uhalo(double* U, const double* Us, const Box& b, const Consts& 
     k_fill_uhalo<<<dim3((unsigned)((3 * area + 127) / 128), 6), 128, 0, s>>>(U, Us, b, c);
 }
 
-template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename T, typename TF>
+template <int DIR, bool CHAR, bool BORGES, bool PHYS>
 static void face_one(const double* W, const double* U, const Box& b, const Consts& c, void* F,
                      const FaceBox& fb, cudaStream_t s) {
     const dim3 grid((fb.n2 - (DIR == 2) + 31) / 32, (fb.n1 - (DIR == 1) + 3) / 4, fb.n0);
-    k_face_flux<DIR, CHAR, BORGES, PHYS, T, TF><<<grid, dim3(32, 4), 0, s>>>(W, U, b, c, (TF*)F, fb);
+    k_face_flux<DIR, CHAR, BORGES, PHYS><<<grid, dim3(32, 4), 0, s>>>(W, U, b, c, (float*)F, fb);
     if constexpr (DIR > 0) {
         const dim3 tail(((DIR == 1 ? fb.n2 : fb.n1) + 127) / 128, fb.n0);
-        k_face_flux_tail<DIR, CHAR, BORGES, PHYS, T, TF><<<tail, 128, 0, s>>>(W, U, b, c, (TF*)F, fb);
+        k_face_flux_tail<DIR, CHAR, BORGES, PHYS><<<tail, 128, 0, s>>>(W, U, b, c, (float*)F, fb);
     }
 }
 
-template <int DIR, typename T, typename TF>
-static void face_dispatch(bool chr, bool borges, bool phys, const double* W, const double* U,
-                          const Box& b, const Consts& c, void* F, const FaceBox& fb, cudaStream_t s) {
-    if (chr) {
-        if (borges) {
-            if (phys) face_one<DIR, true, true, true, T, TF>(W, U, b, c, F, fb, s);
-            else face_one<DIR, true, true, false, T, TF>(W, U, b, c, F, fb, s);
-        } else {
-            if (phys) face_one<DIR, true, false, true, T, TF>(W, U, b, c, F, fb, s);
-            else face_one<DIR, true, false, false, T, TF>(W, U, b, c, F, fb, s);
-        }
-    } else {
-        if (borges) {
-            if (phys) face_one<DIR, false, true, true, T, TF>(W, U, b, c, F, fb, s);
-            else face_one<DIR, false, true, false, T, TF>(W, U, b, c, F, fb, s);
-        } else {
-            if (phys) face_one<DIR, false, false, true, T, TF>(W, U, b, c, F, fb, s);
-            else face_one<DIR, false, false, false, T, TF>(W, U, b, c, F, fb, s);
-        }
-    }
-}
-
-void launch_face_flux(int dir, bool chr, bool borges, bool phys, bool fp32, const double* W,
-                      const double* U, const Box& b, const Consts& c, void* F, const FaceBox& fb,
-                      cudaStream_t s) {
+template <bool CHAR, bool BORGES, bool PHYS>
+static int faces_one(bool fp32, int dims, const double* W, const double* U, const Box& b, const Consts& c, void* const F[3],
+                     const FaceBox fb[3], cudaStream_t s) {
     if (fp32) {
-        if (dir == 0) face_dispatch<0, float, float>(chr, borges, phys, W, U, b, c, F, fb, s);
-        else if (dir == 1) face_dispatch<1, float, float>(chr, borges, phys, W, U, b, c, F, fb, s);
-        else face_dispatch<2, float, float>(chr, borges, phys, W, U, b, c, F, fb, s);
-    } else {
-        if (dir == 0) face_dispatch<0, double, double>(chr, borges, phys, W, U, b, c, F, fb, s);
-        else if (dir == 1) face_dispatch<1, double, double>(chr, borges, phys, W, U, b, c, F, fb, s);
-        else face_dispatch<2, double, double>(chr, borges, phys, W, U, b, c, F, fb, s);
+        face_one<0, CHAR, BORGES, PHYS>(W, U, b, c, F[0], fb[0], s);
+        face_one<1, CHAR, BORGES, PHYS>(W, U, b, c, F[1], fb[1], s);
+        if (dims == 3) face_one<2, CHAR, BORGES, PHYS>(W, U, b, c, F[2], fb[2], s);
+        return dims == 3 ? 5 : 3;
     }
+    OpFaces o;
+    unsigned blocks = 0;
+    for (int d = 0; d < 3; d++) {
+        o.F[d] = (double*)F[d];
+        o.fb[d] = fb[d];
+        o.blocks[d] = d < dims ? (unsigned)(((long long)fb[d].n0 * fb[d].n1 * fb[d].n2 + 127) / 128) : 0;
+        blocks += o.blocks[d];
+    }
+    k_op_faces<CHAR, BORGES, PHYS><<<blocks, 128, 0, s>>>(W, U, b, c, o);
+    return 1;
+}
+
+int launch_faces(bool chr, bool borges, bool phys, bool fp32, int dims, const double* W, const double* U, const Box& b,
+                 const Consts& c, void* const F[3], const FaceBox fb[3], cudaStream_t s) {
+    if (chr) {
+        if (borges) return phys ? faces_one<true, true, true>(fp32, dims, W, U, b, c, F, fb, s)
+                                : faces_one<true, true, false>(fp32, dims, W, U, b, c, F, fb, s);
+        return phys ? faces_one<true, false, true>(fp32, dims, W, U, b, c, F, fb, s)
+                    : faces_one<true, false, false>(fp32, dims, W, U, b, c, F, fb, s);
+    }
+    if (borges) return phys ? faces_one<false, true, true>(fp32, dims, W, U, b, c, F, fb, s)
+                            : faces_one<false, true, false>(fp32, dims, W, U, b, c, F, fb, s);
+    return phys ? faces_one<false, false, true>(fp32, dims, W, U, b, c, F, fb, s)
+                : faces_one<false, false, false>(fp32, dims, W, U, b, c, F, fb, s);
 }
 
 template <int MODE, int H, bool PHYS, typename TF, typename TV>

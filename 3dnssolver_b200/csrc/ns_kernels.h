@@ -128,8 +128,10 @@ void launch_fill_w(bool phys, double* W, const double* U, const Box& b, const Co
 void launch_fill_shell(bool phys, double* W, const double* U, const Box& b, const Consts& c, cudaStream_t s);
 // U's face halos after an FP64 step, from the third stage's input Us
 void launch_fill_uhalo(double* U, const double* Us, const Box& b, const Consts& c, cudaStream_t s);
-void launch_face_flux(int dir, bool chr, bool borges, bool phys, bool fp32, const double* W,
-                      const double* U, const Box& b, const Consts& c, void* F, const FaceBox& fb, cudaStream_t s);
+// face fluxes of an operator call along the first `dims` axes, from W and U; returns
+// the kernels launched
+int launch_faces(bool chr, bool borges, bool phys, bool fp32, int dims, const double* W, const double* U, const Box& b,
+                 const Consts& c, void* const F[3], const FaceBox fb[3], cudaStream_t s);
 // the y- (dir 1) or z-faces (dir 2) of an FP64 stage, from W (and the sound speed plane) alone
 void launch_step_faces(int dir, bool chr, bool borges, bool phys, const double* W, const Box& b, const Consts& c,
                        double* F, const FaceBox& fb, cudaStream_t s, Planes pl = Planes());
