@@ -438,7 +438,6 @@ static ns_status xstage(ns_ctx* ctx, int st, double* Uin, double* Uout, unsigned
         prof_mark(ctx, NS_PROF_VISCOUS);
     }
     XMarchArgs a;
-    a.W = ctx->W;
     a.U = Uin;
     a.U0 = ctx->U0;
     a.Uout = Uout;

@@ -116,11 +116,11 @@ __device__ __forceinline__ void cell_flux(const double w[5], double inv_gm1, dou
     for (int a = 0; a < 3; a++) f[2 + a] = a == DIR ? fma(m[a], qn, w[1]) : m[a] * qn;
 }
 
-// Twice the numerical flux of one face.  ld(s, w) gives W of stencil cell s = 0..5; ldu(s, u)
-// gives U unless WONLY (a time step's stencils, where U = cons(W)); lam(s) gives the
-// cell's |q_n| + c (physical semantics).
-template <int DIR, bool CHAR, bool BORGES, bool PHYS, bool WONLY, typename LoadW, typename LoadU, typename Speed>
-__device__ __forceinline__ void face_flux64(LoadW ld, LoadU ldu, Speed lam, const Consts& c, double out[5]) {
+// Twice the numerical flux of one face.  Of stencil cell s = 0..5, cell(s, u, f) gives U
+// and the flux, prim(s, w) gives W (asked of cells 2 and 3), and lam(s) gives |q_n| + c
+// (physical semantics).
+template <int DIR, bool CHAR, bool BORGES, bool PHYS, typename Cell, typename Prim, typename Speed>
+__device__ __forceinline__ void face_flux64(Cell cell, Prim prim, Speed lam, const Consts& c, double out[5]) {
     // local Lax-Friedrichs speed, the largest of the 6 cells (physical semantics; the
     // reference's is the constant 3, convection_flux.cpp:241)
     double alpha = 3.0;
@@ -136,8 +136,8 @@ __device__ __forceinline__ void face_flux64(LoadW ld, LoadU ldu, Speed lam, cons
     double v[3], hq2 = 0, cs2 = 0, K2pc = 0, kc = 0, inv2c = 0;
     if constexpr (CHAR) {
         double wa[5], wb[5];
-        ld(2, wa);
-        ld(3, wb);
+        prim(2, wa);
+        prim(3, wb);
 #pragma unroll
         for (int q = 0; q < 5; q++) wa[q] = wa[q] + wb[q];  // twice the average
 #pragma unroll
@@ -191,10 +191,8 @@ __device__ __forceinline__ void face_flux64(LoadW ld, LoadU ldu, Speed lam, cons
     double gl[5][4], gr[5][4], cen[5], up[5], fp[5];
 #pragma unroll
     for (int s = 0; s < 6; s++) {
-        double w[5], u[5], f[5];
-        ld(s, w);
-        if constexpr (!WONLY) ldu(s, u);
-        cell_flux<DIR, WONLY>(w, c.inv_gm1, u, f);
+        double u[5], f[5];
+        cell(s, u, f);
         if (s > 0) {
             double l[5], r[5], g[5];
 #pragma unroll
@@ -254,8 +252,13 @@ __device__ __forceinline__ void face_flux64_w(At at, const Consts& c, double out
 #pragma unroll
         for (int q = 0; q < 5; q++) w[q] = at(q, s);
     };
+    auto cell = [&](int s, double u[5], double f[5]) {
+        double w[5];
+        ld(s, w);
+        cell_flux<DIR, true>(w, c.inv_gm1, u, f);
+    };
     auto lam = [&](int s) { return fabs(at(2 + DIR, s)) + at(6, s); };
-    face_flux64<DIR, CHAR, BORGES, PHYS, true>(ld, [](int, double*) {}, lam, c, out);
+    face_flux64<DIR, CHAR, BORGES, PHYS>(cell, ld, lam, c, out);
 }
 
 // the faces of an operator call: W and the caller's U in device memory, stencil
@@ -268,16 +271,19 @@ __device__ __forceinline__ void face_flux64_wu(const double* __restrict__ W, con
 #pragma unroll
         for (int q = 0; q < 5; q++) w[q] = W[q * b.fstride + o0 + s * step];
     };
-    auto ldu = [&](int s, double u[5]) {
+    auto cell = [&](int s, double u[5], double f[5]) {
+        double w[5];
+        ld(s, w);
 #pragma unroll
         for (int q = 0; q < 5; q++) u[q] = U[q * b.fstride + o0 + s * step];
+        cell_flux<DIR, false>(w, c.inv_gm1, u, f);
     };
     auto lam = [&](int s) {
         double w[5];
         ld(s, w);
         return fabs(w[2 + DIR]) + sound_speed(w, c.gamma);
     };
-    face_flux64<DIR, CHAR, BORGES, PHYS, false>(ld, ldu, lam, c, out);
+    face_flux64<DIR, CHAR, BORGES, PHYS>(cell, ld, lam, c, out);
 #pragma unroll
     for (int q = 0; q < 5; q++) out[q] *= 0.5;
 }

@@ -31,8 +31,7 @@ struct UpdateArgs {
 
 // the x-march of an FP64 stage (launch_xmarch)
 struct XMarchArgs {
-    const double* W;    // the stage's W (and sound speed plane), halos filled
-    const double* U;    // the stage's input
+    const double* U;    // the stage's input (on a slab with its exchanged ghost planes)
     double* U0;         // the step's start
     double* Uout;       // the stage's output buffer
     double* Wnext;      // receives the next stage's W (interior)

@@ -67,12 +67,15 @@ __global__ void __launch_bounds__(128, kFaceBlocks)
 // update of each cell as soon as both of its x-faces are known, so the x-faces
 // never reach HBM.  One thread per column (j, k), the columns numbered through so
 // that warps are full at any extent, marching lx cells.  A thread's stencil is its
-// own column's alone, so each keeps a private ring of 7 planes of W (and the sound
-// speed) in shared memory, filled with cp.async: planes i-2 .. i+3 feed the x-face
-// between cells i and i+1 while plane i+4 is in flight, with no barrier between the
-// threads.  U0 and U of the update come the same way; the face fluxes of the other
-// axes and the viscous terms are read at the update.  Uout is a second buffer: the
-// next stage's fill needs the halos of U.
+// own column's alone, so each keeps a private ring of 7 planes in shared memory, filled
+// with cp.async: planes i-2 .. i+3 feed the x-face between cells i and i+1 while plane
+// i+4 is in flight, with no barrier between the threads.  The ring holds the stage's
+// input U itself, which the update reads from it as well, and what a face needs besides:
+// p, 1/rho and (in registers) |u| + c, formed once as a plane arrives (the same W = prim(U) that the
+// other kernels read, and a cell's flux takes 6 operations instead of 13).  U0 of the
+// update comes by cp.async too; the face fluxes of the other axes and the viscous terms
+// are read at the update.  Ghost planes are U's folded planes.  Uout is a second
+// buffer: neighbouring segments still read U.
 //
 // LAST (third stage): the next step's start as well -- W = prim(U_out) for its
 // CFL minimum (time_scheme.cpp:69, 98-136) into slot_next and U0 = cons(W)
@@ -81,20 +84,21 @@ __global__ void __launch_bounds__(128, kFaceBlocks)
 // and U0 are one buffer, only read, and only once; U0 is written in the third stage
 // only, where it is not U (so the restrict qualifiers hold).
 //
-// Bound: half the FP64 pipe (63% busy), half memory (304 bytes a cell).  Three blocks
-// per SM hold the ring and U0, U in shared memory without spills; ms per step
-// (Taylor-Green 384^3 / shear layer 256^3 / Sod 512x128x128 component-wise): this 11.97 /
-// 3.33 / 1.58; planes through TMA on mbarriers with a block barrier per cell 12.27 /
-// 3.51 / 1.69; the faces' operands staged too 13.2 / 3.65 / 1.75; U not staged 12.27 /
-// 3.54 / 1.64, nor U0 15.3 / 4.53 / 2.18; four blocks of 128 registers 15.7 / 3.61 / 1.60.
+// Bound: memory first (about 280 bytes a cell, 9 ms a step at 384^3 at the copy rate
+// with the third stage's extra write), the FP64 pipe next (61% busy).  Three blocks per SM hold
+// the ring without spills.  ms per step (Taylor-Green 384^3 / shear layer 256^3 / Sod
+// 512x128x128 component-wise): this 11.4 / 3.25 / 1.53; a ring of W and U read besides
+// 12.0 / 3.31 / 1.58; planes of W through TMA on mbarriers with a block barrier per cell
+// 12.3 / 3.51 / 1.69; with the faces' operands staged too 13.2 / 3.65 / 1.75; U0 not staged
+// 15.3 / 4.53 / 2.18; four blocks of 128 registers 15.7 / 3.61 / 1.60.  |u| + c in the ring
+// instead of in registers: 13.6 at 384^3 (7 KB less L1 for the operands read at the update).
 //
 // IMAGES: each cell's W also goes to the ghost cells that fold onto it, over edges and
 // corners too, so that the next stage needs no launch of its own for them.
 constexpr int kXMarchBlocks = 3;  // per SM
-template <bool PHYS>
 struct XMarchLayout {
-    static constexpr int NF = PHYS ? 6 : 5, NS = 7;
-    static constexpr size_t bytes = (size_t)(NS * NF + 5 + 10) * 128 * 8;
+    static constexpr int NF = 7, NS = 7;  // U, p, 1/rho
+    static constexpr size_t bytes = (size_t)(NS * NF + 5 + 5) * 128 * 8;
 };
 
 // The ghost indices -3 .. -1 (bits 0..2) and n .. n+2 (bits 3..5) that fold onto index a
@@ -113,18 +117,18 @@ __device__ __forceinline__ unsigned images(int a, int n, int periodic) {
 __device__ __forceinline__ int image(int bit, int a, int n) { return bit == 6 ? a : (bit < 3 ? bit - 3 : n + bit - 3); }
 template <bool CHAR, bool BORGES, bool PHYS, bool LAST, bool IMAGES>
 __global__ void __launch_bounds__(128, kXMarchBlocks)
-    k_xmarch(const double* __restrict__ W, const double* __restrict__ U, double* __restrict__ U0,
+    k_xmarch(const double* __restrict__ U, double* __restrict__ U0,
              double* __restrict__ Uout, double* __restrict__ Wn, const double* __restrict__ Fy,
              const double* __restrict__ Fz, const double* __restrict__ V, long long vs, Box b, FaceBox fy, FaceBox fz,
              Consts c, const unsigned long long* __restrict__ slot, unsigned long long* __restrict__ slot_next,
              double m1, double m2, double mc, double* __restrict__ clock, unsigned long long* __restrict__ slot_reset,
              int xlo, int xhi, int lx) {
-    constexpr int NF = XMarchLayout<PHYS>::NF, NS = XMarchLayout<PHYS>::NS;
+    constexpr int NF = XMarchLayout::NF, NS = XMarchLayout::NS;
     extern __shared__ double xsm[];
     const int t = threadIdx.y * 32 + threadIdx.x;
     double* ring = xsm + t;                // [NS][NF][128]
     double* fprev = ring + NS * NF * 128;  // [5][128]
-    double* opnd = fprev + 5 * 128;        // [10][128]: U0 and U of the cell
+    double* opnd = fprev + 5 * 128;        // [5][128]: U0 of the cell
     int j, k;
     const bool live = row_tile(b, j, k);
     // threads outside the grid march no cells but join the block reduction of LAST
@@ -144,33 +148,69 @@ __global__ void __launch_bounds__(128, kXMarchBlocks)
         if (c.dim == 3) mk = images(k, b.nz, c.periodic[2]);
     }
     const bool first = U == U0;  // the first stage's input is the step's start
-    auto load_plane = [&](int p) {  // plane p of W into slot (p - x0 + 3) % NS
-        const double* w = W + b.at(p + NG, j + NG, k + NG);
-        double* d = ring + ((p - x0 + 3) % NS) * NF * 128;
+    auto slot_of = [&](int p) { return ring + ((p - x0 + 3) % NS) * NF * 128; };
+    auto load_plane = [&](int p) {
+        const double* u = U + b.at(fold_x(p, b.nx, c) + NG, j + NG, k + NG);
+        double* d = slot_of(p);
 #pragma unroll
-        for (int q = 0; q < NF; q++) cp_async8(d + q * 128, w + (q < 5 ? q : 6) * b.fstride);
+        for (int q = 0; q < 5; q++) cp_async8(d + q * 128, u + q * b.fstride);
+    };
+    double win[6] = {0, 0, 0, 0, 0, 0};  // |u| + c of planes i-2 .. i+3 (physical semantics)
+    auto arrived = [&](int p) {  // p, 1/rho and |u| + c of a plane
+        double* d = slot_of(p);
+        double u[5], w[5];
+#pragma unroll
+        for (int q = 0; q < 5; q++) u[q] = d[q * 128];
+        prim_from_cons(u, c.gm1, w);
+        d[5 * 128] = w[1];
+        d[6 * 128] = 1.0 / u[0];
+        if constexpr (PHYS) {
+#pragma unroll
+            for (int s = 0; s < 5; s++) win[s] = win[s + 1];
+            win[5] = fabs(w[2]) + sound_speed(w, c.gamma);
+        }
     };
     if (live)
         for (int p = x0 - 3; p < x0 + 3; p++) load_plane(p);
     cp_async_commit();
+    cp_async_wait_all();
+    if (live)
+        for (int p = x0 - 3; p < x0 + 2; p++) arrived(p);
     for (int i = x0 - 1; i < x1; i++) {
         const long long o = b.at(i + NG, j + NG, k + NG);
         if (i + 4 <= x1 + 2) load_plane(i + 4);
-        if (i >= x0) {
+        if (i >= x0 && !first) {
 #pragma unroll
-            for (int q = 0; q < 5; q++) {
-                cp_async8(opnd + q * 128, U0 + q * b.fstride + o);
-                if (!first) cp_async8(opnd + (5 + q) * 128, U + q * b.fstride + o);
-            }
+            for (int q = 0; q < 5; q++) cp_async8(opnd + q * 128, U0 + q * b.fstride + o);
         }
         cp_async_commit();
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // plane i + 3 has landed
+        arrived(i + 3);
         const double* P[6];
 #pragma unroll
-        for (int s = 0; s < 6; s++) P[s] = ring + ((i - x0 + 1 + s) % NS) * NF * 128;
-        auto at = [&](int q, int s) { return P[s][(q < 5 ? q : 5) * 128]; };
+        for (int s = 0; s < 6; s++) P[s] = slot_of(i - 2 + s);
+        auto cell = [&](int s, double u[5], double g[5]) {
+            const double* d = P[s];
+#pragma unroll
+            for (int q = 0; q < 5; q++) u[q] = d[q * 128];
+            const double pr = d[5 * 128], vel = u[2] * d[6 * 128];
+            g[0] = u[2];
+            g[1] = (u[1] + pr) * vel;
+            g[2] = fma(u[2], vel, pr);
+            g[3] = u[3] * vel;
+            g[4] = u[4] * vel;
+        };
+        auto prim = [&](int s, double w[5]) {
+            const double* d = P[s];
+            const double ir = d[6 * 128];
+            w[0] = d[0];
+            w[1] = d[5 * 128];
+#pragma unroll
+            for (int a = 0; a < 3; a++) w[2 + a] = d[(2 + a) * 128] * ir;
+        };
+        auto lam = [&](int s) { return win[s]; };
         double f[5];
-        face_flux64_w<0, CHAR, BORGES, PHYS>(at, c, f);
+        face_flux64<0, CHAR, BORGES, PHYS>(cell, prim, lam, c, f);
         if (i < x0) {
 #pragma unroll
             for (int q = 0; q < 5; q++) fprev[q * 128] = f[q];
@@ -190,7 +230,7 @@ __global__ void __launch_bounds__(128, kXMarchBlocks)
             r += (py[q * fy.fstride + b.nz] - py[q * fy.fstride]) * c.half_inv[1];
             if (Fz) r += (pz[q * fz.fstride + 1] - pz[q * fz.fstride]) * c.half_inv[2];
             if (q && V) r += pv[(q - 1) * vs];
-            const double u0 = opnd[q * 128], u = first ? u0 : opnd[(5 + q) * 128];
+            const double u = P[2][q * 128], u0 = first ? u : opnd[q * 128];
             un[q] = (u0 * m1) + (u * m2) + (r * m3);
             Uout[q * b.fstride + o] = un[q];
         }
@@ -286,7 +326,7 @@ void launch_step_faces(int dir, bool chr, bool borges, bool phys, const double* 
 
 template <bool CHAR, bool BORGES, bool PHYS, bool LAST, bool IMAGES>
 static void xmarch_one(const XMarchArgs& a, cudaStream_t s, Planes pl) {
-    constexpr size_t bytes = XMarchLayout<PHYS>::bytes;
+    constexpr size_t bytes = XMarchLayout::bytes;
     auto kern = k_xmarch<CHAR, BORGES, PHYS, LAST, IMAGES>;
     // the attribute is per device; a refusal surfaces as the launch's error
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -295,7 +335,7 @@ static void xmarch_one(const XMarchArgs& a, cudaStream_t s, Planes pl) {
     // a segment costs its cells, its first face and the latency of its first planes
     const int lx = march_length(np, blocks, a.sms * kXMarchBlocks, 2.0, 64);
     kern<<<dim3((unsigned)blocks, (np + lx - 1) / lx), dim3(32, 4), bytes, s>>>(
-        a.W, a.U, a.U0, a.Uout, a.Wnext, a.Fy, a.Fz, a.V, a.vs, a.b, a.fy, a.fz, a.c, a.slot,
+        a.U, a.U0, a.Uout, a.Wnext, a.Fy, a.Fz, a.V, a.vs, a.b, a.fy, a.fz, a.c, a.slot,
         LAST ? a.slot_next : nullptr, a.m1, a.m2, a.mc, a.clock, a.slot_reset, x0, x0 + np, lx);
 }
 
