@@ -871,8 +871,10 @@ static ns_status device_status(ns_ctx* ctx);
 #define NS_STEP_PIPELINE 1  // ns_time_step overlaps its host transfers with the stages
 #endif
 
-// x-planes per chunk of ns_time_step's transfer pipeline
-static int pipe_chunk() { return 64; }
+// x-planes per chunk of ns_time_step's transfer pipeline: what the last chunk up and the
+// first one down add to the transfers falls with the chunk (256^3 step: 31.2 ms with 64
+// planes, 30.6 with 32), and launches and segments' first faces rise.
+static int pipe_chunk() { return 32; }
 
 static bool pinned(const void* p) {
     cudaPointerAttributes a;
@@ -884,12 +886,12 @@ static bool pinned(const void* p) {
 }
 
 // whether ns_time_step runs time_step_pipelined: an FP64 step of do_step's
-// x-march form, on a single domain, at least two chunks long, from and to pinned
+// x-march form, on a single domain, at least 128 planes long, from and to pinned
 // host memory (to pageable memory a copy blocks the calling thread and
 // serialises the chunks)
 static bool pipelined(const ns_ctx* ctx, const double* W, const double* U) {
     const ns_params& p = ctx->p;
-    if (!NS_STEP_PIPELINE || !ctx->xfused || slab(ctx) || p.sensor || p.nx < 2 * pipe_chunk()) return false;
+    if (!NS_STEP_PIPELINE || !ctx->xfused || slab(ctx) || p.sensor || p.nx < 128) return false;
     return pinned(W) && (!U || pinned(U));
 }
 

@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(128, kXMarchBlocks)
 int march_length(int n, long long blocks, int resident, double extra, int longest) {
     int best = n;
     double cost = 1e300;
-    for (int seg = (n + longest - 1) / longest; seg <= (n + 3) / 4; seg++) {
+    for (int seg = (n + longest - 1) / longest; seg <= n; seg++) {
         const int len = (n + seg - 1) / seg;
         const long long waves = (blocks * ((n + len - 1) / len) + resident - 1) / resident;
         const double w = waves > 8 ? (double)blocks * seg / resident : (double)waves;
