@@ -61,7 +61,7 @@ struct ns_ctx {
     double* U = nullptr;   // conservative, halo'd SoA
     double* U0 = nullptr;  // RK stage base (interior used)
     double* U2 = nullptr;  // second stage buffer of the fused paths
-    bool xfused = false;   // FP64 steps: x-faces and update in one kernel (k_xface_update)
+    bool xfused = false;   // FP64 steps: x-faces and update in one kernel (k_xmarch)
     double* W2 = nullptr;  // its second W buffer (the next stage's W)
     bool w_next_ready = false;  // with fused_ready: W holds prim(U0) for the next step's first stage
     double* R = nullptr;   // residual for the operator entry points (lazy)

@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(MarchTile<T, H>::FT, MarchTile<T, H>::MINB)
 // component-wise one where those fill the GPU once (shorter ones that would even out the
 // last wave cost 1-2%: the blocks of a thin wave run faster), shorter marches on
 // smaller grids (ms per step at the longest throughout -> now: Taylor-Green 64^3 1.56 ->
-// 0.21, 32^3 0.81 -> 0.15, 200x130x70 2.60 -> 1.81; sensor-gated Sod 256x64x64 0.78 -> 0.64).
+// 0.21, 32^3 0.81 -> 0.077, 200x130x70 2.60 -> 1.81; sensor-gated Sod 256x64x64 0.78 -> 0.64).
 constexpr double kMarchExtra = 3.0;
 template <bool CHAR>
 struct MarchLongest {

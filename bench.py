@@ -275,50 +275,50 @@ def job_rate(world, cells, steps, ms_max):
 # vortex.  The x-update and fused stage rows average the three stages (the
 # third also forms the next step's start).
 COMPUTE_PER_UNIT = {
-    ("reference", "fp64_char", "face_y"): (1408, 996, "fp64", "face"),
-    ("reference", "fp64_char", "face_z"): (1406, 994, "fp64", "face"),
-    ("reference", "fp64_comp", "face_y"): (995, 748, "fp64", "face"),
-    ("reference", "fp64_comp", "face_z"): (995, 748, "fp64", "face"),
-    ("reference", "fp64_char", "xface_update"): (1533, 1079, "fp64", "cell"),
-    ("reference", "fp64_comp", "xface_update"): (1134, 841, "fp64", "cell"),
-    ("reference", "fp64_char", "viscous"): (221, 135, "fp64", "cell"),
-    ("reference", "fp64_comp", "viscous"): (221, 135, "fp64", "cell"),
+    ("reference", "fp64_char", "face_y"): (976, 639, "fp64", "face"),
+    ("reference", "fp64_char", "face_z"): (970, 635, "fp64", "face"),
+    ("reference", "fp64_comp", "face_y"): (756, 514, "fp64", "face"),
+    ("reference", "fp64_comp", "face_z"): (756, 514, "fp64", "face"),
+    ("reference", "fp64_char", "xface_update"): (1073, 703, "fp64", "cell"),
+    ("reference", "fp64_comp", "xface_update"): (850, 578, "fp64", "cell"),
+    ("reference", "fp64_char", "viscous"): (126, 95, "fp64", "cell"),
+    ("reference", "fp64_comp", "viscous"): (126, 95, "fp64", "cell"),
     ("reference", "fp32_char", "stage_fused"): (4216, 2885, "fp32", "cell"),
     ("reference", "fp32_comp", "stage_fused"): (3211, 2244, "fp32", "cell"),
-    ("physical", "fp64_char", "face_y"): (1438, 1022, "fp64", "face"),
-    ("physical", "fp64_char", "face_z"): (1438, 1022, "fp64", "face"),
-    ("physical", "fp64_comp", "face_y"): (1091, 815, "fp64", "face"),
-    ("physical", "fp64_comp", "face_z"): (1091, 815, "fp64", "face"),
-    ("physical", "fp64_char", "xface_update"): (1590, 1123, "fp64", "cell"),
-    ("physical", "fp64_comp", "xface_update"): (1233, 909, "fp64", "cell"),
-    ("physical", "fp64_char", "viscous"): (378, 218, "fp64", "cell"),
-    ("physical", "fp64_comp", "viscous"): (378, 218, "fp64", "cell"),
+    ("physical", "fp64_char", "face_y"): (976, 646, "fp64", "face"),
+    ("physical", "fp64_char", "face_z"): (976, 646, "fp64", "face"),
+    ("physical", "fp64_comp", "face_y"): (762, 525, "fp64", "face"),
+    ("physical", "fp64_comp", "face_z"): (762, 525, "fp64", "face"),
+    ("physical", "fp64_char", "xface_update"): (1109, 732, "fp64", "cell"),
+    ("physical", "fp64_comp", "xface_update"): (886, 606, "fp64", "cell"),
+    ("physical", "fp64_char", "viscous"): (139, 103, "fp64", "cell"),
+    ("physical", "fp64_comp", "viscous"): (139, 103, "fp64", "cell"),
     ("physical", "fp32_char", "stage_fused"): (4440, 3037, "fp32", "cell"),
     ("physical", "fp32_comp", "stage_fused"): (3521, 2448, "fp32", "cell"),
 }
 # DRAM bytes (read + write) per unit from the same captures at 128^3 (inputs
 # larger than L2; the kernels stream their inputs once at 128^3 and above, so
 # traffic scales with the units), averaged over the three stages of a step
-# like the counts above; "fill" is the steady-state k_fill_halo.
+# like the counts above; "fill" is the steady-state k_fill_w of the ghost cells.
 TRAFFIC_PER_UNIT = {
-    ("reference", "fp64_char", "face_y"): 69.6, ("reference", "fp64_char", "face_z"): 63.5,
-    ("reference", "fp64_comp", "face_y"): 66.3, ("reference", "fp64_comp", "face_z"): 63.4,
-    ("reference", "fp64_char", "xface_update"): 319.9, ("reference", "fp64_comp", "xface_update"): 317.7,
-    ("reference", "fp64_char", "viscous"): 61.6, ("reference", "fp64_comp", "viscous"): 61.7,
-    ("reference", "fp64_char", "fill_prim"): 21.8, ("reference", "fp64_comp", "fill_prim"): 21.7,
+    ("reference", "fp64_char", "face_y"): 67.5, ("reference", "fp64_char", "face_z"): 61.8,
+    ("reference", "fp64_comp", "face_y"): 68.0, ("reference", "fp64_comp", "face_z"): 61.7,
+    ("reference", "fp64_char", "xface_update"): 275.9, ("reference", "fp64_comp", "xface_update"): 275.4,
+    ("reference", "fp64_char", "viscous"): 47.7, ("reference", "fp64_comp", "viscous"): 47.8,
+    ("reference", "fp64_char", "fill_prim"): 12.0, ("reference", "fp64_comp", "fill_prim"): 12.0,
     ("reference", "fp32_char", "stage_fused"): 119.2, ("reference", "fp32_comp", "stage_fused"): 119.4,
-    ("physical", "fp64_char", "face_y"): 66.3, ("physical", "fp64_char", "face_z"): 62.9,
-    ("physical", "fp64_comp", "face_y"): 65.9, ("physical", "fp64_comp", "face_z"): 62.7,
-    ("physical", "fp64_char", "xface_update"): 319.6, ("physical", "fp64_comp", "xface_update"): 317.9,
-    ("physical", "fp64_char", "viscous"): 61.9, ("physical", "fp64_comp", "viscous"): 61.9,
-    ("physical", "fp64_char", "fill_prim"): 21.6, ("physical", "fp64_comp", "fill_prim"): 21.9,
+    ("physical", "fp64_char", "face_y"): 78.7, ("physical", "fp64_char", "face_z"): 73.8,
+    ("physical", "fp64_comp", "face_y"): 78.6, ("physical", "fp64_comp", "face_z"): 73.3,
+    ("physical", "fp64_char", "xface_update"): 291.3, ("physical", "fp64_comp", "xface_update"): 291.4,
+    ("physical", "fp64_char", "viscous"): 48.0, ("physical", "fp64_comp", "viscous"): 48.3,
+    ("physical", "fp64_char", "fill_prim"): 13.9, ("physical", "fp64_comp", "fill_prim"): 13.9,
     ("physical", "fp32_char", "stage_fused"): 118.9, ("physical", "fp32_comp", "stage_fused"): 119.0,
 }
 KERNEL_NAMES = {"stage_fused": "k_stage_march", "update": "k_update",
                 "sensor": "k_sensor_prims + k_sensor_mask_tc + k_gate_delta/k_gate_apply",
-                "xface_update": "k_xface_update_tma", "viscous": "k_viscous", "fill_prim": "k_fill_prim/k_fill_halo",
-                "step_begin": "k_step_begin", "face_x": "k_face_flux<x>", "face_y": "k_face_flux<y>",
-                "face_z": "k_face_flux<z>"}
+                "xface_update": "k_xmarch", "viscous": "k_viscous", "fill_prim": "k_fill_w",
+                "step_begin": "k_step_begin", "face_x": "k_face_flux<x>", "face_y": "k_faces_y",
+                "face_z": "k_faces_z"}
 
 
 def profile(s, reps=3):
@@ -360,10 +360,9 @@ def rooflines(form, prof, n, ms_per_step, peaks, fma, semantics):
             continue
         step_traffic += t * (faces if cls.startswith("face") else cells) * (1 if cls == "step_begin" else 3)
     kname = KERNEL_NAMES.get(dom, dom)
-    if sem == "physical" and dom in ("face_y", "face_z"):
-        kname = kname.replace("k_face_flux", "k_face_flux_tma")
     if dom == "viscous":
-        kname = "k_viscous_tma<%d>" % (FORMS[form].get("order", 2) // 2)
+        half = FORMS[form].get("order", 2) // 2
+        kname = "k_viscous_cd2_tma" if half == 1 else "k_viscous<%d>" % half
     kname += f" ({form})"
     hbm = {"bound": "hbm", "kernel": kname, "achieved": round(achieved, 1), "peak": hbm_peak, "unit": "GB/s",
            "frac": round(achieved / hbm_peak, 4), "traffic": traffic,

@@ -185,8 +185,8 @@ NS_API ns_status ns_advance(ns_ctx* ctx, int nsteps);
 NS_API ns_status ns_get_dt(ns_ctx* ctx, double* dt, double* time);
 /* Blocks until the context's stream is idle.  NS_ERR_TIMEOUT if a bounded
  * device wait ran out since the context was created (a tensor-core wait of the
- * sensor's flag kernel, or a TMA tile wait of the FP64 face or viscous
- * kernels; the kernel then ended without its results).  With
+ * sensor's flag kernel, or a TMA tile wait of the FP64 CD-2 viscous kernel;
+ * the kernel then ended without its results).  With
  * params.check_finite set it then checks the current state: NS_ERR_NONFINITE if
  * an interior cell holds NaN/Inf or a non-positive density or pressure (the
  * message gives the number of such cells).  ns_time_step runs the same check
