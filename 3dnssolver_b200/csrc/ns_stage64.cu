@@ -6,10 +6,12 @@
 // in L1.  Threads are numbered through rows and planes, so warps are full at any
 // extent and no axis needs a launch for its last face plane.
 //
-// Bound: the FP64 pipe.  One face per thread, nothing carried: 16 warps per SM
-// (128 registers) hide the stencil's latency and each other's dependent chains.
-// Tried and slower on B200 (Taylor-Green 384^3, ms per step, y/z 7.94/7.58 as it
-// is): 12 warps per SM 8.27/7.77; the sound speeds formed per face 9.47/9.50; tiles
+// Bound: the FP64 pipe, 75% (y) and 81% (z) busy.  One face per thread, nothing carried:
+// 16 warps per SM (128 registers) hide the stencil's latency and each other's dependent
+// chains.  ms per step, y/z: Taylor-Green 384^3 12.4/12.5 -> 8.1/7.5, shear layer 256^3
+// 3.10/3.04 -> 2.18/2.09 (fluxes on differences, the sound speed's plane, no tiles).
+// Tried and slower on B200 (Taylor-Green 384^3, ms per step, y/z 7.94/7.58 in the same
+// runs): 12 warps per SM 8.27/7.77; the sound speeds formed per face 9.47/9.50; tiles
 // of W staged by TMA 8.90/9.01; flux differences instead of fluxes, y marched per
 // thread and z through shared memory 9.50/8.74.
 #include <cuda_runtime.h>
@@ -84,8 +86,8 @@ __global__ void __launch_bounds__(128, kFaceBlocks)
 // and U0 are one buffer, only read, and only once; U0 is written in the third stage
 // only, where it is not U (so the restrict qualifiers hold).
 //
-// Bound: memory first (about 280 bytes a cell, 9 ms a step at 384^3 at the copy rate
-// with the third stage's extra write), the FP64 pipe next (61% busy).  Three blocks per SM hold
+// Bound: memory (291 bytes a cell measured, 7.6 ms a step at 384^3 at the copy rate:
+// 66% of it) and the FP64 pipe (61% busy) together, at 12 warps per SM.  Three blocks per SM hold
 // the ring without spills.  ms per step (Taylor-Green 384^3 / shear layer 256^3 / Sod
 // 512x128x128 component-wise): this 11.4 / 3.25 / 1.53; a ring of W and U read besides
 // 12.0 / 3.31 / 1.58; planes of W through TMA on mbarriers with a block barrier per cell
@@ -276,9 +278,9 @@ __global__ void __launch_bounds__(128, kXMarchBlocks)
 int march_length(int n, long long blocks, int resident, double extra, int longest) {
     int best = n;
     double cost = 1e300;
-    for (int seg = (n + longest - 1) / longest; seg <= n; seg++) {
-        const int len = (n + seg - 1) / seg;
-        const long long waves = (blocks * ((n + len - 1) / len) + resident - 1) / resident;
+    for (int most = std::min(n, longest); most >= 1; most--) {
+        const int seg = (n + most - 1) / most, len = (n + seg - 1) / seg;
+        const long long waves = (blocks * seg + resident - 1) / resident;
         const double w = waves > 8 ? (double)blocks * seg / resident : (double)waves;
         if (w * (len + extra) < cost * (1 - 1e-9)) {
             cost = w * (len + extra);

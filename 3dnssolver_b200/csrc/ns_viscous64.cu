@@ -18,7 +18,7 @@
 // (k_viscous_cd2).  ms per step before -> now (both with TMA tiles / without):
 //   CD-2, physical, 384^3: 3.73 -> 2.50 / 4.67      256x256x17: 0.123 / 0.134, x8: 0.123 / 0.074
 //   CD-2, reference, 256^3: 1.00 -> 0.58 / 0.79     256x256x8: 0.094 / 0.044, 512x512x1: 0.301 / 0.086
-//   CD-6, physical, 101x75x130: 0.80 -> 0.31 (cells near an edge had read 250 neighbours each)
+//   CD-6, physical, 101x75x130: 0.80 -> 0.25 (cells near an edge had read 250 neighbours each)
 // Marching along y instead of x, or loading the next plane's rows ahead into registers,
 // measured the same or slower.
 #include <cuda.h>
@@ -43,6 +43,10 @@ struct ViscRing {
     static constexpr int NR = PHYS ? 7 : 8, NS = 2 * H + 1;
     static constexpr size_t bytes = (size_t)NS * NR * 128 * 8;
     static constexpr int MINB = H == 2 ? 4 : 3;
+    // a warp's dv/dy and dw/dy of one plane, each of its at most two runs of columns with
+    // H columns on both sides
+    static constexpr int RUN = 32 + 4 * H;
+    static constexpr size_t shared_bytes = (size_t)4 * 2 * RUN * 8;
 };
 
 // centered first and second difference of f(-H) .. f(H), undivided
@@ -88,7 +92,15 @@ __device__ __forceinline__ void viscous_physical_terms(const double gu[3][3], co
     for (int a = 0; a < 3; a++) v[(1 + a) * vs] = -mom[a];
 }
 
-template <int H, bool PHYS>
+// SHARE (physical semantics, 3D, nz >= 32): the lanes of a warp run along z, at most once
+// around the end of their rows, so d2/dydz of v and w is taken from the lanes' own d/dy of
+// the plane (shared memory) and 4H columns of it at the runs' ends, which the lanes form
+// besides: 12 reads of shared memory and 6 loads instead of 72 loads for CD-6, half of a
+// cell's, and loads are what bounds this kernel.  ms per step without -> with: CD-6
+// 101x75x130 0.301 -> 0.246, 128x128x40 0.192 -> 0.164, 384^3 12.2 -> 10.3; CD-4 0.195 ->
+// 0.182, 384^3 7.78 -> 7.19.  In rows of less than 32 cells a warp has more ends than its
+// lanes can serve, and each lane takes the products.
+template <int H, bool PHYS, bool SHARE>
 __global__ void __launch_bounds__(128, ViscRing<H, PHYS>::MINB)
     k_viscous(const double* __restrict__ W, Box b, Consts c, double* __restrict__ V, long long vs, int xlo, int xhi,
               int lx) {
@@ -96,10 +108,29 @@ __global__ void __launch_bounds__(128, ViscRing<H, PHYS>::MINB)
     extern __shared__ double vsm[];
     const int t = threadIdx.y * 32 + threadIdx.x;
     int j, k;
-    if (!row_tile(b, j, k)) return;
+    const bool mine = row_tile(b, j, k);
+    if (SHARE ? !__any_sync(~0u, mine) : !mine) return;  // a lane without a column goes along in row 0
     const int x0 = xlo + blockIdx.y * lx, x1 = min(x0 + lx, xhi);
     double* ring = vsm + t;  // [NS][NR][128]
     const long long xs = (long long)b.NY * b.NZp;
+    // SHARE: where this lane's d/dy goes, and the column at an end that it forms besides
+    double* run = nullptr;
+    double* end = nullptr;
+    const double* we = nullptr;
+    if constexpr (SHARE) {
+        double* warp = vsm + VR::NS * VR::NR * 128 + threadIdx.y * 2 * VR::RUN;
+        const int l = threadIdx.x, k0 = __shfl_sync(~0u, k, 0), j0 = __shfl_sync(~0u, j, 0);
+        const int m = min(32, b.nz - k0);  // lanes of the first run
+        run = warp + H + l + (l < m ? 0 : 2 * H);
+        const int f = l / (4 * H), e = l % (4 * H), side = e / H, h = e % H;  // v or w; the runs' ends in turn
+        // (the first lane's column exists where any does: rows rise with the lanes)
+        const int je = side < 2 ? j0 : j0 + 4;
+        const int ke = side == 0 ? k0 - H + h : side == 1 ? k0 + m + h : side == 2 ? h - H : 32 - m + h;
+        if (f < 2 && (side < 2 || (m < 32 && je < b.ny))) {
+            end = warp + f * VR::RUN + (side == 0 ? h : side == 1 ? H + m + h : side == 2 ? 2 * H + m + h : 3 * H + 32 + h);
+            we = W + (3 + f) * b.fstride + b.at(x0 + NG, je + NG, ke + NG);
+        }
+    }
     const double* w = W + b.at(x0 - H + NG, j + NG, k + NG);
     double* v = V + ((long long)x0 * b.ny + j) * b.nz + k;
     const bool three = c.dim == 3;
@@ -167,8 +198,9 @@ __global__ void __launch_bounds__(128, ViscRing<H, PHYS>::MINB)
             gu[1][0] = dx(2);
             gu[2][0] = dx(3);
             gu[0][1] = X(5, 0);
-            gu[1][1] = diff1<H>([&](int h) { return Y(3, h); }, c) * c.inv_dy;
-            gu[2][1] = diff1<H>([&](int h) { return Y(4, h); }, c) * c.inv_dy;
+            const double v_y = diff1<H>([&](int h) { return Y(3, h); }, c), w_y = diff1<H>([&](int h) { return Y(4, h); }, c);
+            gu[1][1] = v_y * c.inv_dy;
+            gu[2][1] = w_y * c.inv_dy;
             gu[0][2] = gu[1][2] = gu[2][2] = 0.0;
             lap[0] = uxx + dyy(2);
             lap[1] = dxx(2) + vyy;
@@ -184,11 +216,23 @@ __global__ void __launch_bounds__(128, ViscRing<H, PHYS>::MINB)
                 lap[0] += dzz(2);
                 lap[1] += dzz(3);
                 lap[2] += wzz;
-                gdiv[1] += dyz(4);
-                gdiv[2] = wzz + dx(6) + dyz(3);
+                if constexpr (SHARE) {
+                    run[0] = v_y;
+                    run[VR::RUN] = w_y;
+                    if (end) *end = diff1<H>([&](int h) { return we[h * b.NZp]; }, c);
+                    __syncwarp();
+                    const double s = c.inv_dy * c.inv_dz;
+                    gdiv[1] += diff1<H>([&](int h) { return run[VR::RUN + h]; }, c) * s;
+                    gdiv[2] = wzz + dx(6) + diff1<H>([&](int h) { return run[h]; }, c) * s;
+                    __syncwarp();
+                    if (end) we += xs;
+                } else {
+                    gdiv[1] += dyz(4);
+                    gdiv[2] = wzz + dx(6) + dyz(3);
+                }
             }
             const double vel[3] = {X(1, 0), X(2, 0), X(3, 0)};
-            viscous_physical_terms(gu, lap, gdiv, lapT, vel, c, v, vs);
+            if (!SHARE || mine) viscous_physical_terms(gu, lap, gdiv, lapT, vel, c, v, vs);
         } else {
             double Dx[4], Dy[4], Dxx[4], Dyy[4], Dxy[2], Dyx[2], r[5] = {0, 0, 0, 0, 0};
             const double ix2 = c.inv_dx * c.inv_dx, iy2 = c.inv_dy * c.inv_dy;
@@ -512,18 +556,19 @@ static void viscous_cd2(const VTmaMap* m, const double* W, const Box& b, const C
                                                                                              lx);
 }
 
-template <int H, bool PHYS>
+template <int H, bool PHYS, bool SHARE>
 static void viscous_one(const double* W, const Box& b, const Consts& c, double* V, long long vs, int sms,
                         cudaStream_t s, Planes pl) {
     using VR = ViscRing<H, PHYS>;
     // the attribute is per device; a refusal surfaces as the launch's error
-    cudaFuncSetAttribute(k_viscous<H, PHYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VR::bytes);
+    constexpr size_t bytes = VR::bytes + (SHARE ? VR::shared_bytes : 0);
+    cudaFuncSetAttribute(k_viscous<H, PHYS, SHARE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     const int x0 = pl.n < 0 ? 0 : pl.lo, np = pl.n < 0 ? b.nx : pl.n;
     const long long blocks = row_tiles(b);
     // a segment costs its cells and 2H planes of the ring, about half a cell's work each
     const int lx = march_length(np, blocks, sms * VR::MINB, 1.0 + H, 32);
-    k_viscous<H, PHYS><<<dim3((unsigned)blocks, (np + lx - 1) / lx), dim3(32, 4), VR::bytes, s>>>(W, b, c, V, vs, x0, x0 + np,
-                                                                                            lx);
+    k_viscous<H, PHYS, SHARE><<<dim3((unsigned)blocks, (np + lx - 1) / lx), dim3(32, 4), bytes, s>>>(
+        W, b, c, V, vs, x0, x0 + np, lx);
 }
 
 void launch_viscous(int h, bool phys, const VTmaMap* m, const double* W, const Box& b, const Consts& c, double* V,
@@ -532,11 +577,14 @@ void launch_viscous(int h, bool phys, const VTmaMap* m, const double* W, const B
         if (phys) viscous_cd2<true>(m, W, b, c, V, vs, err, sms, s, pl);
         else viscous_cd2<false>(m, W, b, c, V, vs, err, sms, s, pl);
     } else if (phys) {
-        if (h == 2) viscous_one<2, true>(W, b, c, V, vs, sms, s, pl);
-        else viscous_one<3, true>(W, b, c, V, vs, sms, s, pl);
+        const bool share = c.dim == 3 && b.nz >= 32;
+        if (h == 2 && share) viscous_one<2, true, true>(W, b, c, V, vs, sms, s, pl);
+        else if (h == 2) viscous_one<2, true, false>(W, b, c, V, vs, sms, s, pl);
+        else if (share) viscous_one<3, true, true>(W, b, c, V, vs, sms, s, pl);
+        else viscous_one<3, true, false>(W, b, c, V, vs, sms, s, pl);
     } else {
-        if (h == 2) viscous_one<2, false>(W, b, c, V, vs, sms, s, pl);
-        else viscous_one<3, false>(W, b, c, V, vs, sms, s, pl);
+        if (h == 2) viscous_one<2, false, false>(W, b, c, V, vs, sms, s, pl);
+        else viscous_one<3, false, false>(W, b, c, V, vs, sms, s, pl);
     }
 }
 

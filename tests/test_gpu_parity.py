@@ -421,3 +421,20 @@ def test_ghost_cells_from_the_march_and_from_the_fill_agree(bc, order, sem):
         Ua, Ub = interior(a.download_conservative()), interior(b.download_conservative())
     # (the last case's state turns non-finite in the oracle's second step too)
     assert np.array_equal(Ua, Ub[:, :128], equal_nan=True) and np.array_equal(Ua, Ub[:, 128:], equal_nan=True)
+
+
+# The mixed y-z derivatives of the CD-4 and CD-6 terms come from neighbouring lanes where
+# rows have 32 cells or more: rows that end within a warp at its first and last lanes,
+# rows that a group of four does not fill.  The sums are the products' in another order,
+# so the bound is that of the stage terms above.
+@pytest.mark.parametrize("order", [4, 6])
+@pytest.mark.parametrize("ny,nz", [(7, 31), (3, 32), (5, 33), (9, 34), (4, 61), (6, 63), (3, 95)])
+def test_viscous_mixed_derivatives_across_warps(oracle, order, ny, nz):
+    p = pkg.make_params(6, ny, nz, convection=1, diffusion_order=order, bc=(N, P, N), mu=0.05, cfl=0.1, semantics=1)
+    W0 = wl.random_field(p, seed=59, smooth=True)
+    Wo, Uo, dto = oracle.run(p, W0, 2)
+    with pkg.Solver(p) as s:
+        s.upload_primitive(W0)
+        s.advance(2)
+        Ug = s.download_conservative()
+    assert (rel_l2(interior(Ug), interior(Uo)) <= TOL).all()
