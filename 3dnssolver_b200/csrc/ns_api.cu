@@ -62,7 +62,6 @@ struct ns_ctx {
     double* U0 = nullptr;  // RK stage base (interior used)
     double* U2 = nullptr;  // second stage buffer of the fused paths
     bool xfused = false;   // FP64 steps: x-faces and update in one kernel (k_xmarch)
-    double* W2 = nullptr;  // its second W buffer (the next stage's W)
     bool w_next_ready = false;  // with fused_ready: W holds prim(U0) for the next step's first stage
     double* R = nullptr;   // residual for the operator entry points (lazy)
     void* F[3] = {nullptr, nullptr, nullptr};
@@ -87,7 +86,7 @@ struct ns_ctx {
     unsigned long long* xslot = nullptr;     // the CFL minimum reduced over the slabs
     bool flags_valid = false;                // the sensor's flags belong to the current state's run
     int sms = 148;                           // multiprocessors of the context's device
-    nsb::VTmaMap vmap[2];                    // FP64 steps: tensor maps of W and W2 for the CD-2 viscous march
+    nsb::VTmaMap vmap;                       // FP64 steps: tensor map of W for the CD-2 viscous march
     // ns_time_step's transfer pipeline: the copy stream and its events (lazy)
     cudaStream_t copy = nullptr;
     std::vector<cudaEvent_t> ev;
@@ -275,13 +274,6 @@ static void prof_mark(ns_ctx* ctx, int cls) {
     g_prof->cls[g_prof->n++] = cls;
 }
 
-// the tensor map of the context's current W for the CD-2 viscous march, or null
-static const nsb::VTmaMap* visc_map(const ns_ctx* ctx) {
-    for (const nsb::VTmaMap& m : ctx->vmap)
-        if (m.W == ctx->W) return &m;
-    return nullptr;
-}
-
 // face fluxes of the current (W, U) along every convected axis (operator calls)
 static ns_status faces(ns_ctx* ctx) {
     const ns_params& p = ctx->p;
@@ -422,26 +414,30 @@ static const double kRkM1[3] = {1.0, 3.0 / 4.0, 1. / 3.};
 static const double kRkM2[3] = {0.0, 1.0 / 4.0, 2. / 3.};
 static const double kRkMc[3] = {-1.0, -(1. / 4.), -(2. / 3.)};
 
-// FP64 stage st after its fill, on the x-planes pl: the y- and z-faces (with
-// with_faces), the viscous terms, then the x-faces marched together with the cell
-// update from Uin into Uout (and the next stage's W into W2, with images its ghost
-// cells too)
+// the viscous terms of an FP64 stage on the x-planes pl, into the x-face array, which a
+// step leaves unused otherwise
+static ns_status step_viscous(ns_ctx* ctx, Planes pl) {
+    if (ctx->p.diffusion != NS_DIFF_CENTERED) return NS_OK;
+    launch_viscous(ctx->c.order / 2, phys(ctx), ctx->vmap.W ? &ctx->vmap : nullptr, ctx->W, ctx->box, ctx->c,
+                   (double*)ctx->F[0], ctx->fb[0].fstride, ctx->slot + 4, ctx->sms, ctx->stream, pl);
+    NS_TRY(check_launch(ctx, 1));
+    prof_mark(ctx, NS_PROF_VISCOUS);
+    return NS_OK;
+}
+
+// FP64 stage st on the x-planes pl, after its fill, y- and z-faces and viscous terms: the
+// x-faces marched together with the cell update from Uin into Uout.  The next stage's W
+// takes the place of this one's, which the march does not read (with images, its ghost
+// cells too): other planes' viscous terms must have been formed before.
 static ns_status xstage(ns_ctx* ctx, int st, double* Uin, double* Uout, unsigned long long* cur,
-                        unsigned long long* nxt, bool with_faces, bool images, Planes pl) {
+                        unsigned long long* nxt, bool images, Planes pl) {
     cudaStream_t s = ctx->stream;
-    if (with_faces) NS_TRY(step_faces(ctx, pl));
     const bool visc = ctx->p.diffusion == NS_DIFF_CENTERED;
-    if (visc) {  // into the x-face array, which a step leaves unused otherwise
-        launch_viscous(ctx->c.order / 2, phys(ctx), visc_map(ctx), ctx->W, ctx->box, ctx->c, (double*)ctx->F[0],
-                       ctx->fb[0].fstride, ctx->slot + 4, ctx->sms, s, pl);
-        NS_TRY(check_launch(ctx, 1));
-        prof_mark(ctx, NS_PROF_VISCOUS);
-    }
     XMarchArgs a;
     a.U = Uin;
     a.U0 = ctx->U0;
     a.Uout = Uout;
-    a.Wnext = ctx->W2;
+    a.Wnext = ctx->W;
     a.Fy = (const double*)ctx->F[1];
     a.Fz = (const double*)ctx->F[2];
     a.V = visc ? (const double*)ctx->F[0] : nullptr;
@@ -474,7 +470,7 @@ static bool march_images(const ns_ctx* ctx) {
 }
 
 // the state after an FP64 step of do_step: U holds it, U0 and the other parity
-// slot the next step's start, W (after the last swap) the next stage's W
+// slot the next step's start, W the next stage's W
 static void end_xstep(ns_ctx* ctx) {
     ctx->parity ^= 1;
     ctx->fused_ready = true;
@@ -532,8 +528,8 @@ static ns_status do_step(ns_ctx* ctx) {
     }
     double* in[3] = {ctx->U0, ctx->U, ctx->U2};
     double* out[3] = {ctx->U, ctx->U2, ctx->U};
-    // W for a stage, its ghost cells included, is the previous x-march's output (W and
-    // W2 swap each stage), or its ghost cells are filled (on a slab after the exchange).  A
+    // W for a stage, its ghost cells included, is the previous x-march's output, or its
+    // ghost cells are filled (on a slab after the exchange).  A
     // first stage without that output (after a state change or a download of W) fills all
     // cells.
     const bool w_ready = ctx->fused_ready && ctx->w_next_ready, img = march_images(ctx);
@@ -546,8 +542,9 @@ static ns_status do_step(ns_ctx* ctx) {
             NS_TRY(check_launch(ctx, 1));
             prof_mark(ctx, NS_PROF_FILL);
         }
-        NS_TRY(xstage(ctx, st, in[st], out[st], cur, nxt, true, img, Planes()));
-        std::swap(ctx->W, ctx->W2);
+        NS_TRY(step_faces(ctx, Planes()));
+        NS_TRY(step_viscous(ctx, Planes()));
+        NS_TRY(xstage(ctx, st, in[st], out[st], cur, nxt, img, Planes()));
     }
     end_xstep(ctx);
     return NS_OK;
@@ -654,7 +651,6 @@ void ns_destroy(ns_ctx* ctx) {
     cudaFree(ctx->U);
     cudaFree(ctx->U0);
     cudaFree(ctx->U2);
-    cudaFree(ctx->W2);
     cudaFree(ctx->R);
     for (int d = 0; d < 3; d++) cudaFree(ctx->F[d]);
     cudaFree(ctx->stage);
@@ -723,13 +719,9 @@ ns_status ns_create(const ns_params* p, ns_ctx** out) {
     ctx->fused = p->precision == NS_PREC_FP32;
     ctx->xfused = !ctx->fused && p->precision == NS_PREC_FP64 && p->convection != NS_CONV_NONE;
     if (ctx->fused || ctx->xfused) A((void**)&ctx->U2, soa_bytes(ctx->box));
-    if (ctx->xfused) A((void**)&ctx->W2, wbytes);
     // the CD-2 viscous march reads tiles 32 cells wide through TMA where at least half of
     // them is filled (measured: ns_viscous64.cu)
-    if (st == NS_OK && ctx->xfused && p->nz >= 16) {
-        nsb::visc_tma_encode(&ctx->vmap[0], ctx->W, ctx->box, wplanes);
-        nsb::visc_tma_encode(&ctx->vmap[1], ctx->W2, ctx->box, wplanes);
-    }
+    if (st == NS_OK && ctx->xfused && p->nz >= 16) nsb::visc_tma_encode(&ctx->vmap, ctx->W, ctx->box, wplanes);
     A((void**)&ctx->diag, 8 * sizeof(double));
     A((void**)&ctx->clock, 2 * sizeof(double));
     if (st == NS_OK) {
@@ -977,27 +969,37 @@ static ns_status time_step_pipelined_run(ns_ctx* ctx, const double* Wh, double* 
     launch_fill_w(phys(ctx), ctx->W, ctx->U0, ctx->box, ctx->c, s, ghost_lo);
     launch_fill_w(phys(ctx), ctx->W, ctx->U0, ctx->box, ctx->c, s, ghost_hi);
     NS_TRY(check_launch(ctx, 2));
-    NS_TRY(xstage(ctx, 0, ctx->U0, ctx->U, cur, nxt, false, false, Planes()));
-    std::swap(ctx->W, ctx->W2);
+    NS_TRY(step_viscous(ctx, Planes()));
+    NS_TRY(xstage(ctx, 0, ctx->U0, ctx->U, cur, nxt, false, Planes()));
 
     // stage 2 (U -> U2)
     launch_fill_shell(phys(ctx), ctx->W, ctx->U, ctx->box, ctx->c, s);
     NS_TRY(check_launch(ctx, 1));
-    NS_TRY(xstage(ctx, 1, ctx->U, ctx->U2, cur, nxt, true, false, Planes()));
-    std::swap(ctx->W, ctx->W2);
+    NS_TRY(step_faces(ctx, Planes()));
+    NS_TRY(step_viscous(ctx, Planes()));
+    NS_TRY(xstage(ctx, 1, ctx->U, ctx->U2, cur, nxt, false, Planes()));
 
-    // stage 3 (U2 -> U) chunk by chunk into W2, which then holds prim(U) on every
-    // cell (finalize_w); U's ghost cells are final after the fill
+    // stage 3 (U2 -> U) chunk by chunk; W then holds prim(U) on every cell (finalize_w), which
+    // takes the place of the stage's W: the viscous terms, which read the neighbouring
+    // chunks' W, are formed a chunk ahead, and the x ghost planes follow the first and the
+    // last chunk's.  U's ghost cells are final after the fill
     launch_fill_shell(phys(ctx), ctx->W, ctx->U2, ctx->box, ctx->c, s);
     launch_fill_uhalo(ctx->U, ctx->U2, ctx->box, ctx->c, s);
-    launch_prim_all(ctx->W2, ctx->U, ctx->box, ctx->c, s, ghost_lo);
-    launch_prim_all(ctx->W2, ctx->U, ctx->box, ctx->c, s, ghost_hi);
-    NS_TRY(check_launch(ctx, 4));
+    NS_TRY(check_launch(ctx, 2));
+    NS_TRY(step_viscous(ctx, interior(0)));
+    launch_prim_all(ctx->W, ctx->U, ctx->box, ctx->c, s, ghost_lo);
+    NS_TRY(check_launch(ctx, 1));
     for (int c = 0; c < K; c++) {
-        NS_TRY(xstage(ctx, 2, ctx->U2, ctx->U, cur, nxt, true, false, interior(c)));
+        if (c + 1 < K) NS_TRY(step_viscous(ctx, interior(c + 1)));
+        if (c == std::max(K - 2, 0)) {
+            launch_prim_all(ctx->W, ctx->U, ctx->box, ctx->c, s, ghost_hi);
+            NS_TRY(check_launch(ctx, 1));
+        }
+        NS_TRY(step_faces(ctx, interior(c)));
+        NS_TRY(xstage(ctx, 2, ctx->U2, ctx->U, cur, nxt, false, interior(c)));
         const Planes sp = span(c);
-        launch_prim_all(ctx->W2, ctx->U, ctx->box, ctx->c, s, halo_interior(c));
-        launch_soa_to_aos(ctx->W2, ctx->stage, ctx->box, s, sp);
+        launch_prim_all(ctx->W, ctx->U, ctx->box, ctx->c, s, halo_interior(c));
+        launch_soa_to_aos(ctx->W, ctx->stage, ctx->box, s, sp);
         NS_TRY(check_launch(ctx, 2));
         NS_CUDA(cudaEventRecord(ev[K + c], s));
         NS_CUDA(cudaStreamWaitEvent(cs, ev[K + c], 0));
@@ -1007,7 +1009,6 @@ static ns_status time_step_pipelined_run(ns_ctx* ctx, const double* Wh, double* 
     // the compute stream's next use of the staging buffer follows the downloads
     NS_CUDA(cudaEventRecord(ev[2 * K + 1], cs));
     NS_CUDA(cudaStreamWaitEvent(s, ev[2 * K + 1], 0));
-    std::swap(ctx->W, ctx->W2);
     end_xstep(ctx);
     ctx->w_next_ready = false;  // W holds prim(U) (finalize_w)
     ctx->w_valid = true;
