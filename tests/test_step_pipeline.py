@@ -121,3 +121,22 @@ def test_registered_host_arrays_take_the_pipeline():
             assert b.launches > a.launches
         finally:
             pkg.host_unregister(Wb)
+
+
+# The third stage forms the viscous terms a chunk ahead of the march that replaces W: chunks
+# narrower than the CD-6 stencil at the end, and along it both boundary kinds.
+@pytest.mark.parametrize("nx,order,bc,sem", [
+    (129, 6, (P, N, P), pkg.SEM_PHYSICAL), (162, 6, (N, P, N), pkg.SEM_PHYSICAL),
+    (129, 4, (N, N, P), pkg.SEM_REFERENCE), (161, 2, (P, P, P), pkg.SEM_PHYSICAL)])
+def test_pipelined_step_with_narrow_last_chunk(nx, order, bc, sem):
+    p = pkg.make_params(nx, 6, 33, convection=1, diffusion_order=order, bc=bc, mu=0.02, cfl=0.1, semantics=sem)
+    W0 = wl.random_field(p, seed=31, smooth=True)
+    with pkg.Solver(p) as a, pkg.Solver(p) as b:
+        Wa, Ua = W0.copy(), a.new_array()
+        tW, Wb = _pinned_like(W0)
+        tU, Ub = _pinned_like(b.new_array())
+        for _ in range(2):
+            assert a.time_step(Wa, Ua) == b.time_step(Wb, Ub)
+            assert _same(Wa, Wb) and _same(Ua, Ub)
+        del Wb, Ub
+        del tW, tU
