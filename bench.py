@@ -12,12 +12,14 @@ Headline workload (one "step" = one TimeScheme::step, i.e. three RK stages):
   sensor form are timed beside it and compared with it field by field.
   Synthetic input: no dataset is involved.  The device state (22 GB at 512^3)
   is larger than L2, so no flush is needed between timed steps.
-Also in the line: the Sod shock tube 512x128x128 run to t = 0.2 by every form
+Also measured: the Sod shock tube 512x128x128 run to t = 0.2 by every form
 (per-field L2/Linf against FP64 characteristic-wise), the sensor's training
 recipe with held-out precision/recall, the HBM roofline in algorithmic bytes
 (120 B per cell-stage: read U_stage and U0, write U_next), the compute
 roofline, the end-to-end rate through ns_time_step with host buffers, and the
-reference's own CPU TimeScheme::step timed on the host cores.
+reference's own CPU TimeScheme::step timed on the host cores.  The printed line
+holds the rates, errors and rooflines in short (result_line); --detail FILE keeps
+the full record.
 
 Arms:
   default            our CUDA path (libns_b200.so through its C ABI)
@@ -100,6 +102,8 @@ def parse():
     ap.add_argument("--no-sod", action="store_true", help="skip the 512x128x128 Sod comparison")
     ap.add_argument("--cpu-sample-n", type=int, default=256,
                     help="grid of the reference CPU sample (the same workload's IC)")
+    ap.add_argument("--detail", default="", metavar="FILE",
+                    help="also write the full record there (histories, each form's kernels, rooflines and errors)")
     return ap.parse_args()
 
 
@@ -119,6 +123,82 @@ def workload_name(wk, n, form):
 
 def initial_state(wl, wk, p, seed):
     return getattr(wl, WORKLOADS[wk]["ic"])(p, seed=seed)
+
+
+# ---------------------------------------------------------------------------
+# the printed line
+
+MAX_LINE = 4000  # characters: a log's tail holds the whole line
+
+
+def _sig(x, digits):
+    if isinstance(x, float) and math.isfinite(x):
+        return float(f"{x:.{digits}g}")
+    if isinstance(x, dict):
+        return {k: _sig(v, digits) for k, v in x.items()}
+    if isinstance(x, (list, tuple)):
+        return [_sig(v, digits) for v in x]
+    return x
+
+
+def _errors(e):
+    """Relative L2 per field (in the order of FIELDS) of a field_errors record."""
+    return [_sig(e["rel_l2"][f], 3) for f in FIELDS]
+
+
+def result_line(out):
+    """The one JSON line of a full record: every key of the record's top level, with the
+    per-form, Sod and training records cut down to their rates and errors."""
+    line = dict(out)
+    for k in ("roofline", "compute_roofline"):
+        if line.get(k):
+            line[k] = {a: b for a, b in line[k].items()
+                       if a not in ("traffic_source", "counts_source", "algorithmic_unit", "note")}
+    forms = {}
+    for name, f in (out.get("forms") or {}).items():
+        if name == out["config"].get("form"):
+            continue  # the line's own value
+        c = {k: _sig(f[k], 5) for k in ("value", "sensor_fraction", "error") if k in f}
+        for k, v in f.items():
+            if k.startswith("errors_vs_"):
+                c["rel_l2"] = _errors(v)
+        forms[name] = c
+    if forms:
+        line["fields"], line["forms"] = FIELDS, forms
+    if "forms" in out and not forms:
+        del line["forms"]
+    train = out.get("sensor_training")
+    if train:
+        line["sensor_training"] = {k: _sig({"faces": v["faces"], "seconds": v["seconds"],
+                                            "precision": v["held_out"]["precision"],
+                                            "recall": v["held_out"]["recall"]}, 4) for k, v in train.items()}
+    sod = out.get("sod_512x128x128")
+    if sod and "forms" in sod:
+        line["sod_512x128x128"] = {
+            "t_end": sod["t_end"], "steps": sod["steps"], "fp64_char_nonfinite": sod["fp64_char_nonfinite"],
+            "forms": {k: {"value": _sig(v["cell_updates_per_s"], 5), "rel_l2": _errors(v)}
+                      for k, v in sod["forms"].items()}}
+    for k in ("cpu_baseline", "sod_512x128x128"):
+        if isinstance(line.get(k), dict):
+            line[k] = {a: b[:160] if isinstance(b, str) else b for a, b in line[k].items()}
+    for c in forms.values():
+        if "error" in c:
+            c["error"] = str(c["error"])[:80]
+    text = json.dumps(line)
+    # what the contract does not name goes first if it is too long all the same
+    for k in ("sod_512x128x128", "sensor_training", "forms", "kernel_ms_per_step", "compute_roofline"):
+        if len(text) <= MAX_LINE:
+            break
+        line.pop(k, None)
+        text = json.dumps(line)
+    return text
+
+
+def report(out, detail):
+    if detail:
+        with open(detail, "w") as fh:
+            json.dump(out, fh)
+    print(result_line(out))
 
 
 # ---------------------------------------------------------------------------
@@ -586,7 +666,7 @@ def slab_bench(args, dist, rank, world, local):
                     "steps": args.e2e_steps, "api": "ns_time_step on every rank's slab, pinned host W"},
             "diagnostics": {"nonfinite": diag["nonfinite"], "dt": diag["dt"]},
         }
-        print(json.dumps(out))
+        report(out, args.detail)
     return 0
 
 
@@ -708,8 +788,7 @@ def main():
     e2e = {"value": job_rate(world, cells, args.e2e_steps, e2e_ms), "unit": UNIT,
            "h2d_bytes_per_step": int(Wh.nbytes), "d2h_bytes_per_step": int(Wh.nbytes),
            "steps": args.e2e_steps,
-           "api": "ns_time_step (TimeScheme::step drop-in), pinned host W; the library overlaps the chunked "
-                  "upload with the first stage and the chunked download with the third"}
+           "api": "ns_time_step (TimeScheme::step drop-in), pinned host W, transfers overlapped with the stages"}
     s.close()
     del Wh, Wh_t
 
@@ -780,7 +859,7 @@ def main():
             "sensor_training": {("physical" if k else "reference"): v for k, v in sensor_info.items()},
             "sod_512x128x128": sod,
         }
-        print(json.dumps(out))
+        report(out, args.detail)
     if dist is not None:
         dist.destroy_process_group()
     return 0
