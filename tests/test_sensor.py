@@ -258,3 +258,45 @@ def test_step_flags_agree_with_the_predict_path():
     frac_pred = float((lg > 0).float().mean().item())
     assert frac_pred > 0.01
     assert abs(frac_step - frac_pred) <= 0.005 + 0.02 * frac_pred, (frac_step, frac_pred)
+
+
+# Training takes a tile of 16 samples a warp, and several in turn where a batch has more
+# than its 296 warps hold at once (4736 samples), the gradients summed over them in the
+# tensor core's accumulators: a count that fills neither the last tile nor all warps' last
+# turn.  Tolerances as for the single tiles above; a run repeats bit for bit.
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [4737, 10007, 30011])
+def test_gradients_over_several_tiles_match_numpy(n):
+    rng = np.random.default_rng(n)
+    X = (rng.standard_normal((n, SM.NF)) * 0.7).astype(np.float32)
+    y = (rng.random(n) < 0.25).astype(np.float32)
+    w = pkg.sensor_init(3)
+    w[SM.OFF_B1:SM.OFF_W2] = 0.1 * rng.standard_normal(32)
+    w[SM.OFF_B3] = -0.3
+    dX, dy = _dev(X), _dev(y)
+    g, loss = pkg.sensor_gradients(dX.data_ptr(), dy.data_ptr(), n, w, pos_weight=3.0)
+    loss_ref, g_ref = SM.loss_and_grad(X, y, w, 3.0)
+    assert abs(loss - loss_ref) <= 1e-2 * loss_ref
+    rel = np.linalg.norm(g - g_ref) / np.linalg.norm(g_ref)
+    cos = g @ g_ref / (np.linalg.norm(g) * np.linalg.norm(g_ref))
+    assert rel < 3e-2 and cos > 0.999, (rel, cos)
+    for name, a, b in [("W1", 0, 1024), ("b1", 1024, 1056), ("W2", 1056, 2080), ("b2", 2080, 2112),
+                       ("w3", 2112, 2144), ("b3", 2144, 2145)]:
+        e = np.linalg.norm(g[a:b] - g_ref[a:b]) / (np.linalg.norm(g_ref[a:b]) + 1e-12)
+        assert e < 5e-2, (name, e)
+    g2, loss2 = pkg.sensor_gradients(dX.data_ptr(), dy.data_ptr(), n, w, pos_weight=3.0)
+    assert np.array_equal(g, g2) and loss == loss2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch", [777, 6000])
+def test_training_repeats_bit_for_bit(batch):
+    rng = np.random.default_rng(5)
+    n = 12345
+    dX = _dev(rng.standard_normal((n, SM.NF)) * 0.7)
+    dy = _dev(rng.random(n) < 0.25)
+    w0 = pkg.sensor_init(3)
+    runs = [pkg.sensor_train(dX.data_ptr(), dy.data_ptr(), n, w0, epochs=2, batch=batch, lr=3e-3, pos_weight=3.0,
+                             seed=9) for _ in range(2)]
+    assert np.isfinite(runs[0][0]).all() and not np.array_equal(runs[0][0], w0)
+    assert np.array_equal(runs[0][0], runs[1][0]) and np.array_equal(runs[0][1], runs[1][1])
