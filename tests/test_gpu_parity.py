@@ -462,3 +462,69 @@ def test_fluxes_of_any_magnitude_match_oracle(oracle, conv, weights, rho, pr):
     assert (err <= TOL).all(), err
     _, Uo, _ = oracle.run(p, W, 1)
     _assert_close(Ug, Uo, what="U after a step")
+
+
+# The ghost cells again, on states that stay finite throughout (the boundaries of every
+# kind, periodic along all axes among them), so that each of them counts.
+@pytest.mark.parametrize("bc,order,sem", [((N, P, P), 2, 1), ((P, P, N), 4, 1), ((N, P, N), 2, 0), ((P, P, P), 6, 0),
+                                          ((P, P, P), 6, 1)])
+def test_ghost_cells_from_the_march_and_from_the_fill_agree_on_finite_states(bc, order, sem):
+    kw = dict(convection=2, diffusion_order=order, bc=bc, mu=0.002, cfl=0.05, semantics=sem)
+    small = pkg.make_params(64, 128, 128, L=(1.0, 1.0, 1.0), **kw)
+    large = pkg.make_params(64, 256, 128, L=(1.0, 2.0, 1.0), **kw)
+    W0 = wl.random_field(small, seed=61, smooth=True)
+    W1 = wl.random_field(large, seed=61, smooth=True)
+    interior(W1)[:, :128] = interior(W0)
+    interior(W1)[:, 128:] = interior(W0)
+    with pkg.Solver(small) as a, pkg.Solver(large) as b:
+        a.upload_primitive(W0)
+        b.upload_primitive(W1)
+        a.advance(3)
+        b.advance(3)
+        Ua, Ub = interior(a.download_conservative()), interior(b.download_conservative())
+    assert np.isfinite(Ua).all() and np.isfinite(Ub).all()
+    assert np.array_equal(Ua, Ub[:, :128]) and np.array_equal(Ua, Ub[:, 128:])
+
+
+# The mixed y-z derivatives from neighbouring lanes on periodic rows, where the columns at
+# a row's ends are the other end's cells (bound as for the Neumann rows above).
+@pytest.mark.parametrize("order", [4, 6])
+@pytest.mark.parametrize("bc", [(P, N, P), (P, P, P)])
+@pytest.mark.parametrize("ny,nz", [(3, 32), (5, 33), (4, 61), (6, 63), (3, 95)])
+def test_viscous_mixed_derivatives_on_periodic_rows(oracle, ny, nz, bc, order):
+    p = pkg.make_params(6, ny, nz, convection=1, diffusion_order=order, bc=bc, mu=0.05, cfl=0.1, semantics=1)
+    W0 = wl.random_field(p, seed=59, smooth=True)
+    Wo, Uo, dto = oracle.run(p, W0, 2)
+    with pkg.Solver(p) as s:
+        s.upload_primitive(W0)
+        s.advance(2)
+        Ug = s.download_conservative()
+    assert np.isfinite(interior(Ug)).all() and (rel_l2(interior(Ug), interior(Uo)) <= TOL).all()
+
+
+# The y-faces number their columns (i, k) through blocks of 32 over the grid's second and
+# third dimension; the third is used beyond 65535 x 32 columns.  Two copies of a grid
+# along a periodic x give the same state in both halves and in the grid alone.
+def test_y_faces_of_more_columns_than_one_grid_dimension():
+    kw = dict(convection=1, diffusion=pkg.DIFF_NONE, bc=(P, P, P), mu=0.0, cfl=0.2, semantics=1)
+    nx, ny, nz = 1049, 3, 1000
+    assert nx * nz <= 65535 * 32 < 2 * nx * nz
+    one = pkg.make_params(nx, ny, nz, L=(1.0, 1.0, 1.0), **kw)
+    two = pkg.make_params(2 * nx, ny, nz, L=(2.0, 1.0, 1.0), **kw)
+    rng = np.random.default_rng(67)
+    W0 = np.ones(pkg.halo_shape(one))
+    W0[3:-3, 3:-3, 3:-3] += 0.1 * rng.standard_normal((nx, 1, nz, 5)) + 0.1 * rng.standard_normal((1, ny, 1, 5))
+    W0 = np.clip(W0, 0.5, 1.5)
+    W1 = np.ones(pkg.halo_shape(two))
+    interior(W1)[:nx] = interior(W0)
+    interior(W1)[nx:] = interior(W0)
+    with pkg.Solver(one) as a:
+        a.upload_primitive(W0)
+        a.advance(1)
+        Ua = a.download_conservative()
+    with pkg.Solver(two) as b:
+        b.upload_primitive(W1)
+        b.advance(1)
+        Ub = interior(b.download_conservative())
+    assert np.isfinite(interior(Ua)).all()
+    assert np.array_equal(interior(Ua), Ub[:nx]) and np.array_equal(interior(Ua), Ub[nx:])
