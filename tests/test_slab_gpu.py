@@ -129,3 +129,12 @@ def test_device_transport_one_periodic_rank_over_nccl(tmp_path):
                        join=True, start_method="spawn")
     err = rel_l2(np.load(tmp_path / "U.npy"), Ug)
     assert (err <= 1e-13).all(), err
+
+
+# The CD-4 and CD-6 terms of rows of 32 cells or more take their mixed y-z derivatives from
+# neighbouring lanes: the same on slabs, whose ghost planes are a neighbour's cells.
+@pytest.mark.parametrize("shape,world,bc,order", [((20, 5, 33), 2, (P, N, P), 6), ((22, 6, 41), 2, (N, P, P), 4),
+                                                  ((27, 4, 35), 3, (P, P, N), 6)])
+def test_gpu_slabs_with_long_rows_and_wide_stencils(oracle, tmp_path, shape, world, bc, order):
+    test_gpu_slabs_equal_the_single_domain(oracle, tmp_path, shape, world, bc, 2, order, pkg.PREC_FP64,
+                                           pkg.SEM_PHYSICAL)
