@@ -486,7 +486,7 @@ static ns_status do_step(ns_ctx* ctx) {
     if (ctx->fused) return do_step_fused(ctx);
     cudaStream_t s = ctx->stream;
     unsigned long long* cur = ctx->slot + ctx->parity;
-    if (!ctx->xfused) {
+    if (!ctx->xfused) {  // FP64 without convection
         NS_CUDA(cudaMemsetAsync(cur, 0xFF, sizeof(unsigned long long), s));
         launch_step_begin(!ctx->w_valid, phys(ctx), ctx->W, ctx->U, ctx->U0, ctx->box, ctx->c, cur, s);
         NS_TRY(check_launch(ctx, 1));
@@ -497,8 +497,7 @@ static ns_status do_step(ns_ctx* ctx) {
             launch_fill_prim(ctx->W, ctx->U, ctx->box, ctx->c, s);
             NS_TRY(check_launch(ctx, 1));
             prof_mark(ctx, NS_PROF_FILL);
-            NS_TRY(faces(ctx));
-            UpdateArgs a = update_args(ctx, MODE_STAGE, true, true);
+            UpdateArgs a = update_args(ctx, MODE_STAGE, false, true);
             a.slot = cur;
             a.m1 = kRkM1[st];
             a.m2 = kRkM2[st];
@@ -991,7 +990,7 @@ static ns_status time_step_pipelined_run(ns_ctx* ctx, const double* Wh, double* 
     NS_TRY(check_launch(ctx, 1));
     for (int c = 0; c < K; c++) {
         if (c + 1 < K) NS_TRY(step_viscous(ctx, interior(c + 1)));
-        if (c == std::max(K - 2, 0)) {
+        if (c == K - 2) {  // K >= 4 here
             launch_prim_all(ctx->W, ctx->U, ctx->box, ctx->c, s, ghost_hi);
             NS_TRY(check_launch(ctx, 1));
         }

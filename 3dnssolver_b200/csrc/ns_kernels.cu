@@ -875,21 +875,17 @@ static void update_h(int h, const UpdateArgs& a, cudaStream_t s) {
     }
 }
 
-template <int MODE>
+template <int MODE, typename T>
 static void update_mode(const UpdateArgs& a, cudaStream_t s) {
     int h = a.viscous ? a.c.order / 2 : 0;
-    if (a.fp32) {
-        if (a.phys) update_h<MODE, true, float, float>(h, a, s);
-        else update_h<MODE, false, float, float>(h, a, s);
-    } else {
-        if (a.phys) update_h<MODE, true, double, double>(h, a, s);
-        else update_h<MODE, false, double, double>(h, a, s);
-    }
+    if (a.phys) update_h<MODE, true, T, T>(h, a, s);
+    else update_h<MODE, false, T, T>(h, a, s);
 }
 
 void launch_update(const UpdateArgs& a, cudaStream_t s) {
-    if (a.mode == MODE_STAGE) update_mode<MODE_STAGE>(a, s);
-    else update_mode<MODE_RHS>(a, s);
+    if (a.mode == MODE_STAGE) update_mode<MODE_STAGE, double>(a, s);  // FP32 steps are fused (ns_fused.cuh)
+    else if (a.fp32) update_mode<MODE_RHS, float>(a, s);
+    else update_mode<MODE_RHS, double>(a, s);
 }
 
 void launch_check_state(const double* A, bool prim, const Box& b, const Consts& c,

@@ -97,16 +97,15 @@ __device__ __forceinline__ float gelu_grad(float x) {
 struct alignas(16) MlpSmem {
     __nv_bfloat16 W1[SH * XS];
     __nv_bfloat16 W2[SH * XS];
-    __nv_bfloat16 W2T[SH * XS];  // backward only
+    __nv_bfloat16 W2T[SH * XS];  // training only
     float b1[SH], b2[SH], w3[SH], b3;
 };
 
-__device__ void mlp_load(MlpSmem& m, const float* __restrict__ w, bool transpose) {
+__device__ void mlp_load(MlpSmem& m, const float* __restrict__ w) {
     for (int e = threadIdx.x + threadIdx.y * blockDim.x; e < SH * XS; e += blockDim.x * blockDim.y) {
         int r = e / XS, col = e % XS;
         m.W1[e] = __float2bfloat16(col < SF ? w[OFF_W1 + r * 32 + col] : 0.f);
         m.W2[e] = __float2bfloat16(col < SH ? w[OFF_W2 + r * 32 + col] : 0.f);
-        if (transpose) m.W2T[e] = __float2bfloat16(col < SH ? w[OFF_W2 + col * 32 + r] : 0.f);
     }
     for (int e = threadIdx.x + threadIdx.y * blockDim.x; e < SH; e += blockDim.x * blockDim.y) {
         m.b1[e] = w[OFF_B1 + e];
@@ -634,7 +633,7 @@ __global__ void __launch_bounds__(128) k_mlp_predict(const float* __restrict__ f
     __shared__ __align__(16) MlpSmem m;
     __shared__ __align__(16) __nv_bfloat16 Xs[4][32 * XS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
-    mlp_load(m, w, false);
+    mlp_load(m, w);
     long long r = (long long)blockIdx.x * 128 + warp * 32 + lane;
     __nv_bfloat16* X = Xs[warp];
     for (int e = 0; e < XS; e++) X[lane * XS + e] = __float2bfloat16(r < n && e < SF ? feat[r * SF + e] : 0.f);
@@ -670,7 +669,7 @@ __global__ void __launch_bounds__(128) k_face_gated(const double* __restrict__ W
     __shared__ int nlist;
     const int tid = threadIdx.x + 32 * threadIdx.y, warp = threadIdx.y, lane = threadIdx.x;
     const int g = lane >> 2, q = lane & 3;
-    mlp_load(m, w, false);
+    mlp_load(m, w);
     if (tid == 0) nlist = 0;
     int kk = blockIdx.x * 32 + threadIdx.x;
     int bb = blockIdx.y * 4 + threadIdx.y;
