@@ -462,9 +462,13 @@ static ns_status xstage(ns_ctx* ctx, int st, double* Uin, double* Uout, unsigned
 }
 
 // Whether the x-march writes the ghost cells of the next stage's W itself.  That takes a
-// launch less per stage, and costs the warps at the boundary more than k_fill_w does:
-// ms per step with / without on B200: 96x64 0.124 / 0.138, 64^3 0.221 / 0.241, 101x75x130
-// 0.969 / 0.981, Sod 512x128x128 3.82 / 3.79, shear layer 256^3 8.39 / 8.30.
+// launch less per stage, and costs the warps at the boundary more than k_fill_w does: it
+// gains where launches count and costs up to 2% beyond.  ms per step with / without on
+// B200: 96x64 0.068 / 0.075, 64^3 0.189 / 0.199, 100^3 0.698 / 0.692, 101x75x130 CD-6
+// 0.878 / 0.870, 512x64x64 1.09 / 1.08, 160^3 2.43 / 2.40, 512x128x128 3.85 / 3.80, 256^3
+// 8.65 / 8.62.  In 3D the line lies above where the two cross, by 1%; in 2D, where k_fill_w
+// fills 6 ghost cells along z for each cell, the march is the faster one at every size
+// measured (1200x1200 2.31 / 3.18, 2048x2048 6.55 / 9.10), also beyond the line.
 static bool march_images(const ns_ctx* ctx) {
     return !slab(ctx) && (long long)ctx->p.nx * ctx->p.ny * ctx->p.nz <= (1 << 20);
 }
@@ -877,9 +881,11 @@ static bool pinned(const void* p) {
 }
 
 // whether ns_time_step runs time_step_pipelined: an FP64 step of do_step's
-// x-march form, on a single domain, at least 128 planes long, from and to pinned
-// host memory (to pageable memory a copy blocks the calling thread and
-// serialises the chunks)
+// x-march form, on a single domain, at least 128 planes long (four chunks), from and
+// to pinned host memory (to pageable memory a copy blocks the calling thread and
+// serialises the chunks).  From 64 to 127 planes it depends on the planes' size, ms of
+// a step without / with: 127x32x32 0.54 / 0.59, 64x32x32 0.35 / 0.37, 64^3 0.83 / 0.82,
+// 64x128x128 2.71 / 2.56, 96x256x256 14.2 / 13.0; those grids go without.
 static bool pipelined(const ns_ctx* ctx, const double* W, const double* U) {
     const ns_params& p = ctx->p;
     if (!NS_STEP_PIPELINE || !ctx->xfused || slab(ctx) || p.sensor || p.nx < 128) return false;

@@ -59,12 +59,12 @@ namespace nsb {
 // next plane's conversion overwrites plane i-2, whose last reader (the x-faces)
 // finished before this plane's second barrier.
 //
-// The FP32 form runs here; the FP64 form runs the face kernels and the x-face
-// march of ns_kernels.cu.  An FP64 variant of this kernel on an 8 x 16 column
+// The FP32 form runs here; the FP64 form runs the face kernels and the x-march
+// of ns_stage64.cu.  An FP64 variant of this kernel on an 8 x 16 column
 // (128 threads, 109 KB, two blocks of 252 registers per SM) reproduced the FP64
 // path's results exactly but ran 1.25-1.56x slower on B200 (Taylor-Green and
 // shear layer at 256^3): with 8 warps per SM and the plane barriers, the FP64
-// pipe idles; the separate face kernels keep it 62-67% busy at 12 warps.
+// pipe idles; the separate face kernels keep it 75-81% busy at 16 warps.
 template <typename T, int H = 1>
 struct MarchTile {
     static_assert(sizeof(T) == 4, "the fused stage serves the FP32 form");

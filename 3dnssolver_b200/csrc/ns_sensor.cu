@@ -330,6 +330,7 @@ __global__ void __launch_bounds__(128) k_sensor_harvest(const double* __restrict
 // the second.)
 
 constexpr int SPR = (SP + 1 + 3) / 4 * 4;  // floats per row of partial sums: the parameters', then the loss
+// at most one block per multiprocessor of a B200; larger batches take several tiles a warp
 constexpr int kTrainWarps = 2, kTrainBlocks = 148;
 
 struct TrainSmem {

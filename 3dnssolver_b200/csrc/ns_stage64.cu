@@ -8,8 +8,8 @@
 //
 // Bound: the FP64 pipe, 75% (y) and 81% (z) busy.  One face per thread, nothing carried:
 // 16 warps per SM (128 registers) hide the stencil's latency and each other's dependent
-// chains.  ms per step, y/z: Taylor-Green 384^3 12.4/12.5 -> 8.1/7.5, shear layer 256^3
-// 3.10/3.04 -> 2.18/2.09 (fluxes on differences, the sound speed's plane, no tiles).
+// chains.  ms per step, y/z: Taylor-Green 384^3 12.4/12.5 -> 8.1/7.6, shear layer 256^3
+// 3.10/3.04 -> 2.22/2.12 (fluxes on differences, the sound speed's plane, no tiles).
 // Tried and slower on B200 (Taylor-Green 384^3, ms per step, y/z 7.94/7.58 in the same
 // runs): 12 warps per SM 8.27/7.77; the sound speeds formed per face 9.47/9.50; tiles
 // of W staged by TMA 8.90/9.01; flux differences instead of fluxes, y marched per
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(128, kFaceBlocks)
 // Bound: memory (291 bytes a cell measured, 7.6 ms a step at 384^3 at the copy rate:
 // 66% of it) and the FP64 pipe (61% busy) together, at 12 warps per SM.  Three blocks per SM hold
 // the ring without spills.  ms per step (Taylor-Green 384^3 / shear layer 256^3 / Sod
-// 512x128x128 component-wise): this 11.4 / 3.25 / 1.53; a ring of W and U read besides
+// 512x128x128 component-wise): this 11.3 / 3.28 / 1.54; a ring of W and U read besides
 // 12.0 / 3.31 / 1.58; planes of W through TMA on mbarriers with a block barrier per cell
 // 12.3 / 3.51 / 1.69; with the faces' operands staged too 13.2 / 3.65 / 1.75; U0 not staged
 // 15.3 / 4.53 / 2.18; four blocks of 128 registers 15.7 / 3.61 / 1.60.  |u| + c in the ring
@@ -186,7 +186,9 @@ __global__ void __launch_bounds__(128, kXMarchBlocks)
             for (int q = 0; q < 5; q++) cp_async8(opnd + q * 128, U0 + q * b.fstride + o);
         }
         cp_async_commit();
-        asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // plane i + 3 has landed
+        // plane i + 3 has landed (beyond the first cell by the update's wait, which drains
+        // plane i + 4 with U0: the next plane's latency is covered by one face, not two)
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         arrived(i + 3);
         const double* P[6];
 #pragma unroll

@@ -355,22 +355,22 @@ def job_rate(world, cells, steps, ms_max):
 # vortex.  The x-update and fused stage rows average the three stages (the
 # third also forms the next step's start).
 COMPUTE_PER_UNIT = {
-    ("reference", "fp64_char", "face_y"): (976, 639, "fp64", "face"),
-    ("reference", "fp64_char", "face_z"): (970, 635, "fp64", "face"),
-    ("reference", "fp64_comp", "face_y"): (756, 514, "fp64", "face"),
-    ("reference", "fp64_comp", "face_z"): (756, 514, "fp64", "face"),
-    ("reference", "fp64_char", "xface_update"): (1073, 703, "fp64", "cell"),
-    ("reference", "fp64_comp", "xface_update"): (850, 578, "fp64", "cell"),
+    ("reference", "fp64_char", "face_y"): (981, 644, "fp64", "face"),
+    ("reference", "fp64_char", "face_z"): (975, 640, "fp64", "face"),
+    ("reference", "fp64_comp", "face_y"): (761, 519, "fp64", "face"),
+    ("reference", "fp64_comp", "face_z"): (761, 519, "fp64", "face"),
+    ("reference", "fp64_char", "xface_update"): (1078, 709, "fp64", "cell"),
+    ("reference", "fp64_comp", "xface_update"): (855, 583, "fp64", "cell"),
     ("reference", "fp64_char", "viscous"): (126, 95, "fp64", "cell"),
     ("reference", "fp64_comp", "viscous"): (126, 95, "fp64", "cell"),
     ("reference", "fp32_char", "stage_fused"): (4216, 2885, "fp32", "cell"),
     ("reference", "fp32_comp", "stage_fused"): (3211, 2244, "fp32", "cell"),
-    ("physical", "fp64_char", "face_y"): (976, 646, "fp64", "face"),
-    ("physical", "fp64_char", "face_z"): (976, 646, "fp64", "face"),
-    ("physical", "fp64_comp", "face_y"): (762, 525, "fp64", "face"),
-    ("physical", "fp64_comp", "face_z"): (762, 525, "fp64", "face"),
-    ("physical", "fp64_char", "xface_update"): (1109, 732, "fp64", "cell"),
-    ("physical", "fp64_comp", "xface_update"): (886, 606, "fp64", "cell"),
+    ("physical", "fp64_char", "face_y"): (981, 651, "fp64", "face"),
+    ("physical", "fp64_char", "face_z"): (981, 651, "fp64", "face"),
+    ("physical", "fp64_comp", "face_y"): (767, 530, "fp64", "face"),
+    ("physical", "fp64_comp", "face_z"): (767, 530, "fp64", "face"),
+    ("physical", "fp64_char", "xface_update"): (1114, 737, "fp64", "cell"),
+    ("physical", "fp64_comp", "xface_update"): (891, 611, "fp64", "cell"),
     ("physical", "fp64_char", "viscous"): (139, 103, "fp64", "cell"),
     ("physical", "fp64_comp", "viscous"): (139, 103, "fp64", "cell"),
     ("physical", "fp32_char", "stage_fused"): (4440, 3037, "fp32", "cell"),

@@ -5,8 +5,8 @@ next computes).  The same call with pageable arrays runs the unpipelined step.
 Both run the same kernels on the same cells, so the results must agree bit for
 bit; the pipelined step is also held to the oracle like every other step.
 
-The chunks are 64 x-planes, so the grids here have 2-3 chunks, including a
-last chunk of 2 planes and one of 32.
+The chunks are 32 x-planes, so the grids here have 4-6 chunks, including a
+last chunk of 1 plane and one of 32.
 """
 import importlib
 
