@@ -92,9 +92,11 @@ __device__ __forceinline__ void weno5_diff(double d0, double d1, double d2, doub
 // acoustic fields (2c times as large), a small fraction of what the literal form bears.
 // Both terms therefore take dL at the exponent of [2, 4), and dR times the same power of two
 // f; being a power of two it changes no bit of the quotient, and differences up to 1e33
-// pass.  One multiplication a field, 0.6 to 1.1% of a step (Taylor-Green 384^3 168.6 ->
-// 170.4 ms a pass of 4 steps).  (f is 0 for a dL that is not finite, which makes the
-// denominator and so the result NaN.)
+// pass.  One multiplication a field, 0.6 to 1.4% of a step (Taylor-Green 384^3 168.6 ->
+// 170.4 ms a pass of 4 steps, shear layer 256^3 8.23 -> 8.34 ms a step).  A check of the
+// exponents that forms a face again where it fails cost nearly as much, 8.31, for twice
+// the code.  (f is 0 for a dL that is not finite, which makes the denominator and so the
+// result NaN.)
 template <bool BORGES>
 __device__ __forceinline__ double weno5_pair_diff(const double l[4], const double r[4], double eps) {
     double nL, dL, nR, dR;
